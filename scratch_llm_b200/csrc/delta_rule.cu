@@ -14,7 +14,7 @@
 //
 // Columns of S are independent of each other: u_j and o_j need column j of S only.  A warp
 // owns one column (its 32 lanes hold D / 32 elements each, in quads), a CTA of 16 warps takes
-// 16 columns of one (row, head).  Tokens are taken in chunks of TC = 16, and inside a chunk the
+// 16 columns of one (row, head).  Tokens are taken in chunks of CT = 16, and inside a chunk the
 // recurrence is unrolled so that only a small triangular system is sequential.  With S0 the
 // state at the chunk's start, L_t the sum of log g up to token t of the chunk, per column:
 //
@@ -47,11 +47,13 @@
 // pair of tokens, shared by the CTA's 16 columns.  The step size then comes from column b_col +
 // head of `ab`, and A_log / dt_bias are the caller's business (they are inside log_decay).
 //
+// Rows of at least min_chunked tokens go to the kernels of delta_chunks.cuh where the key size fits them.
+//
 // The weights depend on keys, queries and decays alone: delta_weights_kernel forms the tables of
 // ALL chunks of a step in parallel before the scan starts, which then reads its chunk's table.
 //
 // Compiled once per key size: -DSLLM_HEAD_DIM=<D>.
-#include "common.cuh"
+#include "delta_chunks.cuh"
 
 #ifndef SLLM_HEAD_DIM
 #error "compile with -DSLLM_HEAD_DIM=<key size>"
@@ -64,7 +66,7 @@ static_assert(D >= 1 && D <= 256, "key size: 1 to 256 (a chunk of keys and queri
 constexpr int QUADS = (D + 3) / 4;                  // groups of 4 elements of a column
 constexpr int QPL = (QUADS + 31) / 32;              // quads per lane
 constexpr int LDK = 4 * QUADS + 4;                  // row stride of the staged keys / queries
-constexpr int TC = 16;                              // tokens per chunk
+constexpr int CT = 16;                              // tokens per chunk
 constexpr int COLS = 16;                            // columns (warps) per CTA
 constexpr int THREADS = 32 * COLS;
 
@@ -81,10 +83,11 @@ struct DeltaArgs {
     int b_col;                           // the step input of head h is ab[b_col + h]
     // with a decay per channel: the chunks' tables of weights, made by delta_weights_kernel before
     // this launch (null: every CTA forms its chunk's table itself).  The chunk that starts at
-    // token t of row r has slot t / TC + r; a slot holds [H][2 TC][TC] floats.
+    // token t of row r has slot t / CT + r; a slot holds [H][2 CT][CT] floats.
     const float* tables;
+    int min_chunked;                     // rows of at least so many tokens are the chunk kernels'
 };
-// the kernel for a decay per channel stages a third [TC][D] table in (static) shared memory
+// the kernel for a decay per channel stages a third [CT][D] table in (static) shared memory
 constexpr bool CHANNEL_FITS = D <= 192;
 
 // One token of one column by one warp: the rule as it stands.  Every warp norms the key and
@@ -194,28 +197,28 @@ template <typename T, bool VECTOR, bool CHANNEL>
 __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) {
     constexpr int VEC = VECTOR ? 16 / (int)sizeof(T) : 1;
     constexpr int PER_ROW = D / VEC;                               // pieces of a key or query
-    constexpr int QK_PIECES = 2 * TC * PER_ROW;                    // of a chunk
+    constexpr int QK_PIECES = 2 * CT * PER_ROW;                    // of a chunk
     constexpr int QK_ITEMS = (QK_PIECES + THREADS - 1) / THREADS;  // per thread
     struct alignas(16) Piece { T e[VEC]; };
     // keys and queries of the chunk as unit vectors (the query scaled), padded with zeros to
     // whole quads; lane l of a warp owns the quads l, l + 32, ... of its column
-    __shared__ __align__(16) float ks[TC][LDK];
-    __shared__ __align__(16) float qs[TC][LDK];
-    __shared__ float vs[TC][COLS];
+    __shared__ __align__(16) float ks[CT][LDK];
+    __shared__ __align__(16) float qs[CT][LDK];
+    __shared__ float vs[CT][COLS];
     // row t < 16: -e^{L_t - L_s} (k_s . k_t) for s < t; row 16 + t: e^{L_t - L_s} (k_s . q_t) for
     // s <= t; zero elsewhere
-    __shared__ float weight[2 * TC][TC + 1];
-    __shared__ float log_g[TC], cum_s[TC], beta_s[TC], grow_s[TC], rest_s[TC];
+    __shared__ float weight[2 * CT][CT + 1];
+    __shared__ float log_g[CT], cum_s[CT], beta_s[CT], grow_s[CT], rest_s[CT];
     // a decay per channel: the channels' log decays of the chunk's tokens, then their running
     // sums L_t, and at last e^{L_t} * k_t (the keys that meet S0); last_s: L of the chunk's last token
-    __shared__ __align__(16) float lam[CHANNEL ? TC : 1][CHANNEL ? LDK : 4];
+    __shared__ __align__(16) float lam[CHANNEL ? CT : 1][CHANNEL ? LDK : 4];
     __shared__ float last_s[CHANNEL ? LDK : 4];
 
     pdl_wait();
     pdl_trigger();
     const int r = blockIdx.z, head = blockIdx.y;
     const int t0 = a.row_start[r], n_new = a.row_start[r + 1] - t0;
-    if (n_new <= 0) return;
+    if (n_new <= 0 || n_new >= a.min_chunked) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = head / (a.H / a.G);
     const int col0 = blockIdx.x * COLS;
@@ -242,7 +245,7 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
         return;
     }
     // columns beyond D (where D is no multiple of 4) stay zero for good
-    for (int idx = tid; idx < TC * LDK; idx += THREADS) {
+    for (int idx = tid; idx < CT * LDK; idx += THREADS) {
         (&ks[0][0])[idx] = 0.f;
         (&qs[0][0])[idx] = 0.f;
         if (CHANNEL) (&lam[0][0])[idx] = 0.f;
@@ -253,24 +256,24 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
     float raw_a = 0.f, raw_b = 0.f;
     // a decay per channel: the chunk's log decays and this thread's entry of its table of weights
     // travel with the same request
-    constexpr int L_ITEMS = CHANNEL ? (TC * D + THREADS - 1) / THREADS : 1;
+    constexpr int L_ITEMS = CHANNEL ? (CT * D + THREADS - 1) / THREADS : 1;
     float raw_l[L_ITEMS], raw_w = 0.f;
     auto fetch = [&](int c0) {     // requests the chunk at c0 (tokens beyond the row: nothing)
-        const int nt = min(TC, n_new - c0);
+        const int nt = min(CT, n_new - c0);
         if (CHANNEL) {
             const float* lg = a.log_decay + (int64_t)(t0 + c0) * a.ld_decay + (int64_t)head * D;
 #pragma unroll
             for (int i = 0; i < L_ITEMS; ++i) {
                 const int idx = tid + i * THREADS, t = idx / D, e = idx - t * D;
-                raw_l[i] = (idx < TC * D && t < nt) ? lg[(int64_t)t * a.ld_decay + e] : 0.f;
+                raw_l[i] = (idx < CT * D && t < nt) ? lg[(int64_t)t * a.ld_decay + e] : 0.f;
             }
             if (a.tables != nullptr)
-                raw_w = a.tables[(((int64_t)(t0 + c0) / TC + r) * a.H + head) * 2 * TC * TC + tid];
+                raw_w = a.tables[(((int64_t)(t0 + c0) / CT + r) * a.H + head) * 2 * CT * CT + tid];
         }
 #pragma unroll
         for (int i = 0; i < QK_ITEMS; ++i) {
             const int item = tid + i * THREADS;
-            const int which = item / (TC * PER_ROW), rem = item - which * (TC * PER_ROW);
+            const int which = item / (CT * PER_ROW), rem = item - which * (CT * PER_ROW);
             const int t = rem / PER_ROW, c = rem - t * PER_ROW;
             if (item < QK_PIECES && t < nt) {
                 const T* src = act + (int64_t)(t0 + c0 + t) * a.ld_act + (int64_t)g * D +
@@ -279,7 +282,7 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
                 else raw[i].e[0] = src[0];
             }
         }
-        if (tid < TC * COLS) {
+        if (tid < CT * COLS) {
             const int t = tid / COLS, j = tid - t * COLS;
             if (t < nt && col0 + j < a.V)
                 raw_v = act[(int64_t)(t0 + c0 + t) * a.ld_act + v_col0 + (int64_t)head * a.V +
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
 #pragma unroll
         for (int i = 0; i < QK_ITEMS; ++i) {
             const int item = tid + i * THREADS;
-            const int which = item / (TC * PER_ROW), rem = item - which * (TC * PER_ROW);
+            const int which = item / (CT * PER_ROW), rem = item - which * (CT * PER_ROW);
             const int t = rem / PER_ROW, c = rem - t * PER_ROW;
             if (item < QK_PIECES) {
                 float* dst = (which ? &ks[t][0] : &qs[t][0]) + c * VEC;
@@ -303,11 +306,11 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
                 for (int w = 0; w < VEC; ++w) dst[w] = t < nt ? to_float(raw[i].e[w]) : 0.f;
             }
         }
-        if (tid < TC * COLS) {
+        if (tid < CT * COLS) {
             const int t = tid / COLS, j = tid - t * COLS;
             vs[t][j] = (t < nt && col0 + j < a.V) ? to_float(raw_v) : 0.f;
         }
-        if (tid < TC) {
+        if (tid < CT) {
             float lg = 0.f, beta = 0.f;
             if (tid < nt) {
                 const float x = raw_a + dt_bias;
@@ -322,8 +325,8 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
     __syncthreads();
     fetch(0);
 
-    for (int c0 = 0; c0 < n_new; c0 += TC) {
-        const int nt = min(TC, n_new - c0);
+    for (int c0 = 0; c0 < n_new; c0 += CT) {
+        const int nt = min(CT, n_new - c0);
         __syncthreads();   // the previous chunk's staging is no longer read
         commit(nt);
         float table_entry = 0.f;
@@ -331,11 +334,11 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
 #pragma unroll
             for (int i = 0; i < L_ITEMS; ++i) {
                 const int idx = tid + i * THREADS, t = idx / D, e = idx - t * D;
-                if (idx < TC * D) lam[t][e] = raw_l[i];
+                if (idx < CT * D) lam[t][e] = raw_l[i];
             }
             table_entry = raw_w;
         }
-        if (c0 + TC < n_new) fetch(c0 + TC);   // in flight while this chunk is worked on
+        if (c0 + CT < n_new) fetch(c0 + CT);   // in flight while this chunk is worked on
         __syncthreads();
         // unit vectors and the query's scale: one warp per token
         if (warp < nt) {
@@ -358,16 +361,16 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
             for (int e = tid; e < D; e += THREADS) {
                 float c = 0.f;
 #pragma unroll
-                for (int t = 0; t < TC; ++t) {
+                for (int t = 0; t < CT; ++t) {
                     c += lam[t][e];
                     lam[t][e] = c;
                 }
                 last_s[e] = lam[nt - 1][e];
             }
-        } else if (tid >= THREADS - TC) {   // (the last warp: it has no token to norm unless nt is 16)
-            const int t = tid - (THREADS - TC);
+        } else if (tid >= THREADS - CT) {   // (the last warp: it has no token to norm unless nt is 16)
+            const int t = tid - (THREADS - CT);
             float c = 0.f, last = 0.f;
-            for (int i = 0; i < TC; ++i) {
+            for (int i = 0; i < CT; ++i) {
                 if (i <= t) c += log_g[i];
                 if (i < nt) last += log_g[i];
             }
@@ -380,11 +383,11 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
         // with queries
         {
             const int row = tid >> 4, s = tid & 15, t = row & 15;
-            const bool with_q = row >= TC;
+            const bool with_q = row >= CT;
             float dot = 0.f;
             const bool used = t < nt && s < nt && (with_q ? s <= t : s < t);
             if (CHANNEL && a.tables != nullptr) {
-                dot = table_entry;       // (entry [row][s] = [tid / TC][tid % TC], as requested)
+                dot = table_entry;       // (entry [row][s] = [tid / CT][tid % CT], as requested)
             } else if (used && CHANNEL) {
                 const float* x = with_q ? &qs[t][0] : &ks[t][0];
                 for (int e = 0; e < D; ++e)
@@ -405,7 +408,7 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
         if (CHANNEL) {
             // what the rest of the chunk needs: e^{L_t} * k_t (in lam's place) and e^{L_t} * q_t for
             // the products with S0, and e^{L_last - L_t} * k_t for the state's update
-            for (int idx = tid; idx < TC * D; idx += THREADS) {
+            for (int idx = tid; idx < CT * D; idx += THREADS) {
                 const int t = idx / D, e = idx - t * D;
                 const float L = lam[t][e], grow = expf(L), k = ks[t][e];
                 lam[t][e] = grow * k;
@@ -416,9 +419,9 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
         }
 
         // ---- this lane's share of S0^T k_t (v[t]) and S0^T q_t (v[16 + t])
-        float v[2 * TC];
+        float v[2 * CT];
 #pragma unroll
-        for (int t = 0; t < TC; ++t) {
+        for (int t = 0; t < CT; ++t) {
             float pk = 0.f, pq = 0.f;
 #pragma unroll
             for (int i = 0; i < QPL; ++i) {
@@ -434,7 +437,7 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
                 }
             }
             v[t] = pk;
-            v[TC + t] = pq;
+            v[CT + t] = pq;
         }
         // ---- sum over the lanes, so that lane i ends with the total of v[i]: in the round
         // with offset o a lane keeps the half of its values whose index has bit o as its own
@@ -452,15 +455,15 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
         // lane t < 16: the sum that becomes u_t; lane 16 + t: the sum that becomes o_t
         const int t_mine = lane & 15;
         const float grow_mine = CHANNEL ? 1.f : grow_s[t_mine];   // (per channel: inside v[0])
-        float acc = lane < TC ? vs[t_mine][warp] - grow_mine * v[0] : grow_mine * v[0];
-        const float beta_mine = lane < TC ? beta_s[t_mine] : 0.f;
-        float u[TC];
+        float acc = lane < CT ? vs[t_mine][warp] - grow_mine * v[0] : grow_mine * v[0];
+        const float beta_mine = lane < CT ? beta_s[t_mine] : 0.f;
+        float u[CT];
 #pragma unroll
-        for (int s = 0; s < TC; ++s) {
+        for (int s = 0; s < CT; ++s) {
             u[s] = __shfl_sync(0xffffffffu, beta_mine * acc, s);   // lane s has all of its sum
             acc = fmaf(weight[lane][s], u[s], acc);                 // (weight[s][s] is 0)
         }
-        if (lane >= TC && t_mine < nt && live)
+        if (lane >= CT && t_mine < nt && live)
             a.out[(int64_t)(t0 + c0 + t_mine) * a.H * a.V + (int64_t)head * a.V + col] = acc;
         // ---- the state after the chunk
         if (CHANNEL) {
@@ -477,7 +480,7 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
             for (int i = 0; i < 4 * QPL; ++i) S[i] *= keep_all;
         }
 #pragma unroll
-        for (int t = 0; t < TC; ++t) {
+        for (int t = 0; t < CT; ++t) {
             // (u is zero beyond the chunk's tokens; per channel the keys carry their factors)
             const float f = CHANNEL ? u[t] : rest_s[t] * u[t];
 #pragma unroll
@@ -508,25 +511,25 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
 // the top): they depend on the keys, queries and decays alone, not on the state, so the chunks of
 // a row need not wait for each other.  grid (chunks of the longest row, H, rows), 256 threads: a
 // thread per pair of tokens that the table uses (120 pairs of keys with earlier keys, 136 of
-// queries with keys up to their own).  tables: [slots][H][2 TC][TC] as DeltaArgs says; entries
+// queries with keys up to their own).  tables: [slots][H][2 CT][CT] as DeltaArgs says; entries
 // that no pair uses are zero.
 constexpr int TABLE_THREADS = 256;
 template <typename T>
 __global__ void __launch_bounds__(TABLE_THREADS) delta_weights_kernel(const DeltaArgs a, float* tables) {
-    __shared__ __align__(16) float ks[TC][LDK];
-    __shared__ __align__(16) float qs[TC][LDK];
-    __shared__ __align__(16) float lam[TC][LDK];
+    __shared__ __align__(16) float ks[CT][LDK];
+    __shared__ __align__(16) float qs[CT][LDK];
+    __shared__ __align__(16) float lam[CT][LDK];
     pdl_wait();
     pdl_trigger();
-    const int r = blockIdx.z, head = blockIdx.y, c0 = blockIdx.x * TC;
+    const int r = blockIdx.z, head = blockIdx.y, c0 = blockIdx.x * CT;
     const int t0 = a.row_start[r], n_new = a.row_start[r + 1] - t0;
-    if (c0 >= n_new || n_new <= 1) return;     // (rows of one token take the kernel's plain path)
-    const int nt = min(TC, n_new - c0);
+    if (c0 >= n_new || n_new <= 1 || n_new >= a.min_chunked) return;     // (rows of one token take the kernel's plain path)
+    const int nt = min(CT, n_new - c0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = head / (a.H / a.G);
     const T* act = reinterpret_cast<const T*>(a.act);
     const int64_t k_col0 = (int64_t)a.G * D;
-    for (int idx = tid; idx < TC * D; idx += TABLE_THREADS) {
+    for (int idx = tid; idx < CT * D; idx += TABLE_THREADS) {
         const int t = idx / D, e = idx - t * D;
         float k = 0.f, q = 0.f, l = 0.f;
         if (t < nt) {
@@ -556,17 +559,17 @@ __global__ void __launch_bounds__(TABLE_THREADS) delta_weights_kernel(const Delt
     for (int e = tid; e < D; e += TABLE_THREADS) {
         float c = 0.f;
 #pragma unroll
-        for (int t = 0; t < TC; ++t) {
+        for (int t = 0; t < CT; ++t) {
             c += lam[t][e];
             lam[t][e] = c;
         }
     }
     __syncthreads();
-    float* table = tables + (((int64_t)(t0 + c0) / TC + r) * a.H + head) * 2 * TC * TC;
+    float* table = tables + (((int64_t)(t0 + c0) / CT + r) * a.H + head) * 2 * CT * CT;
     // thread -> pair: the first 120 threads take (t, s < t) of keys with keys, the other 136 take
     // (t, s <= t) of queries with keys; both triangles are walked row by row
-    const bool with_q = tid >= TC * (TC - 1) / 2;
-    int p = with_q ? tid - TC * (TC - 1) / 2 : tid, t = 0;
+    const bool with_q = tid >= CT * (CT - 1) / 2;
+    int p = with_q ? tid - CT * (CT - 1) / 2 : tid, t = 0;
     if (with_q) { while (p > t) { p -= t + 1; ++t; } }        // row t has t + 1 pairs
     else { t = 1; while (p >= t) { p -= t; ++t; } }           // row t has t pairs
     const int sidx = p;
@@ -577,11 +580,11 @@ __global__ void __launch_bounds__(TABLE_THREADS) delta_weights_kernel(const Delt
         for (int e = 0; e < D; ++e)
             dot = fmaf(x[e] * ks[sidx][e], __expf(lam[t][e] - lam[sidx][e]), dot);
     }
-    table[((with_q ? TC : 0) + t) * TC + sidx] = dot;
+    table[((with_q ? CT : 0) + t) * CT + sidx] = dot;
     // the entries that no pair uses
-    for (int idx = tid; idx < 2 * TC * TC; idx += TABLE_THREADS) {
-        const int row = idx / TC, s2 = idx - row * TC, t2 = row & (TC - 1);
-        if (row >= TC ? s2 > t2 : s2 >= t2) table[idx] = 0.f;
+    for (int idx = tid; idx < 2 * CT * CT; idx += TABLE_THREADS) {
+        const int row = idx / CT, s2 = idx - row * CT, t2 = row & (CT - 1);
+        if (row >= CT ? s2 > t2 : s2 >= t2) table[idx] = 0.f;
     }
 }
 
@@ -591,14 +594,44 @@ using namespace sllm;
 
 SLLM_EXPORT int sllm_delta_rule_head_dim() { return D; }
 
+// The chunk kernels' lanes share out channels in sixteenths and quads that have to fill warps evenly, and a
+// chunk's keys, queries and sums of decays fit shared memory together: these key sizes.
+constexpr bool CHUNKS = D == 32 || D == 64 || D == 128;
+
+// Floats of scratch the chunk kernels take per chunk slot and head; 0: this key size has none.
+SLLM_EXPORT int64_t sllm_delta_rule_chunk_floats(int V) {
+    return CHUNKS ? chunks::scratch_floats(D, V) : 0;
+}
+
+template <typename T, bool CHANNEL>
+static int launch_chunks(const DeltaArgs& a, float* scratch, int n_tokens, int n_rows, cudaStream_t stream) {
+    if constexpr (CHUNKS) {
+        const int slots = n_tokens / sllm::TC + n_rows + 1;
+        if (slots > 65535) return (int)cudaErrorInvalidValue;
+        const chunks::Scratch z = chunks::scratch_at(scratch, (int64_t)slots * a.H, D, a.V);
+        chunks::PrepArgs p = {};
+        p.x = a.act; p.ld = a.ld_act; p.k0 = a.G * D; p.v0 = 2 * a.G * D; p.per = a.H / a.G;
+        p.log_decay = a.log_decay; p.ldl = a.ld_decay; p.ab = a.ab; p.ldab = a.ld_ab; p.b_col = a.b_col;
+        p.A_log = a.A_log; p.dt_bias = a.dt_bias; p.row_start = a.row_start; p.n_rows = n_rows;
+        p.min_chunked = a.min_chunked; p.H = a.H; p.V = a.V;
+        p.vec4 = a.ld_act % 4 == 0 && ((uintptr_t)a.act & 15) == 0 &&
+                 (!CHANNEL || (a.ld_decay % 4 == 0 && ((uintptr_t)a.log_decay & 15) == 0));
+        return chunks::launch<D, T, CHANNEL>(p, z, a.state, a.row_slot, a.out, slots, stream);
+    }
+    return (int)cudaErrorInvalidValue;
+}
+
 // dtype: 0 = float32, 1 = bfloat16 (of act).  n_rows rows of the packed batch (row_start has
 // n_rows + 1 entries); state slots are indexed by row_slot.  max_new: the most tokens any row
-// brings (1 selects the kernel for decode steps).
+// brings (1 selects the kernel for decode steps).  chunk_scratch (or null): room for (n_tokens / 64 + n_rows
+// + 1) x H x sllm_delta_rule_chunk_floats floats on a 16-byte boundary; rows of at least min_chunked tokens
+// then run in chunks.  shortest: no row brings fewer tokens (rows without tokens apart).
 SLLM_EXPORT int sllm_delta_rule(const void* act, int64_t ld_act, const float* ab, int64_t ld_ab,
                                 const float* A_log, const float* dt_bias, float* state,
                                 const int* row_start, const int* row_slot, float* out, int n_rows,
                                 int max_new, int H, int G, int V, const float* log_decay,
                                 int64_t ld_decay, int b_col, float* tables, int longest,
+                                float* chunk_scratch, int n_tokens, int min_chunked, int shortest,
                                 int dtype, cudaStream_t stream) {
     if (n_rows <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G != 0 || V <= 0 || n_rows > 65535 || H > 65535 ||
@@ -609,6 +642,7 @@ SLLM_EXPORT int sllm_delta_rule(const void* act, int64_t ld_act, const float* ab
     DeltaArgs a;
     a.log_decay = log_decay; a.ld_decay = ld_decay; a.b_col = b_col;
     a.tables = nullptr;
+    a.min_chunked = chunk_scratch ? min_chunked : 0x7fffffff;
     a.act = act; a.ld_act = ld_act; a.ab = ab; a.ld_ab = ld_ab; a.A_log = A_log;
     a.dt_bias = dt_bias; a.state = state; a.row_start = row_start; a.row_slot = row_slot;
     a.out = out; a.H = H; a.G = G; a.V = V;
@@ -632,12 +666,22 @@ SLLM_EXPORT int sllm_delta_rule(const void* act, int64_t ld_act, const float* ab
     const bool vector = D % vec == 0 && ld_act % vec == 0 && ((uintptr_t)act & 15) == 0 &&
                         ((int64_t)G * D) % vec == 0;
     if (dtype != 0 && dtype != 1) return (int)cudaErrorInvalidValue;
+    if (chunk_scratch) {
+        if (min_chunked < 2 || n_tokens < 0 || ((uintptr_t)chunk_scratch & 15) || ((uintptr_t)state & 15))
+            return (int)cudaErrorInvalidValue;
+        const int code = log_decay
+            ? (dtype == 0 ? launch_chunks<float, true>(a, chunk_scratch, n_tokens, n_rows, stream)
+                          : launch_chunks<__nv_bfloat16, true>(a, chunk_scratch, n_tokens, n_rows, stream))
+            : (dtype == 0 ? launch_chunks<float, false>(a, chunk_scratch, n_tokens, n_rows, stream)
+                          : launch_chunks<__nv_bfloat16, false>(a, chunk_scratch, n_tokens, n_rows, stream));
+        if (code || shortest >= min_chunked) return code;
+    }
     if (log_decay) {
         if constexpr (CHANNEL_FITS) {
             if (tables != nullptr && longest > 1) {
-                // all chunks' tables at once; `tables` holds (tokens / TC + n_rows + 1) slots of
-                // H * 2 TC * TC floats, `longest` is the most tokens any row brings
-                dim3 tgrid((longest + TC - 1) / TC, H, n_rows);
+                // all chunks' tables at once; `tables` holds (tokens / CT + n_rows + 1) slots of
+                // H * 2 CT * CT floats, `longest` is the most tokens any row brings
+                dim3 tgrid((longest + CT - 1) / CT, H, n_rows);
                 if (tgrid.x > 65535u * 32u) return (int)cudaErrorInvalidValue;
                 if (dtype == 0) delta_weights_kernel<float><<<tgrid, TABLE_THREADS, 0, stream>>>(a, tables);
                 else delta_weights_kernel<__nv_bfloat16><<<tgrid, TABLE_THREADS, 0, stream>>>(a, tables);

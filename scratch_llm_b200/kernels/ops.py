@@ -1583,11 +1583,36 @@ def moe_combine(y: torch.Tensor, x: torch.Tensor, shared: torch.Tensor | None, i
     return out
 
 
+#: rows of at least so many tokens run in chunks in the delta rule.  In order against in chunks, one
+#: decay per head / per channel: 1 row of 96 tokens, 16 heads of 128 x 128: 39 / 41 and 44 / 53 us;
+#: of 128 tokens: 50 / 41 and 54 / 53 us, with 32 heads 97 / 49 and 95 / 55 us; of 2,048: 733 / 246 and
+#: 666 / 343 us.  (With more heads and rows shorter ones gain too, but a row takes one path
+#: whatever else is in the step.)
+DELTA_MIN_CHUNKED = 128
+
+
+def _delta_chunks(lib, n: int, n_rows: int, n_heads: int, value_dim: int, longest: int,
+                  min_chunked: int | None, state: torch.Tensor) -> tuple[torch.Tensor | None, int]:
+    """(scratch of the delta rule's chunk kernels or None, from how many tokens on a row takes them)."""
+    if min_chunked is None:
+        min_chunked = DELTA_MIN_CHUNKED
+    slots = n // 64 + n_rows + 1
+    if not min_chunked or longest < max(2, min_chunked) or slots > 65535 or state.data_ptr() % 16:
+        return None, 0
+    lib.sllm_delta_rule_chunk_floats.restype = c_int64
+    floats = lib.sllm_delta_rule_chunk_floats(c_int(value_dim))
+    if floats == 0:
+        return None, 0
+    return torch.empty(slots * n_heads * floats, dtype=torch.float32, device=state.device), \
+        max(2, min_chunked)
+
+
 def delta_rule(act: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
                state: torch.Tensor, row_start: torch.Tensor, row_slot: torch.Tensor,
                out: torch.Tensor, n_rows: int, n_heads: int, n_kv_heads: int, key_dim: int,
                value_dim: int, max_new: int = 0, log_decay: torch.Tensor | None = None,
-               b_col: int | None = None, longest: int = 0) -> torch.Tensor:
+               b_col: int | None = None, longest: int = 0, shortest: int = 1,
+               min_chunked: int | None = None) -> torch.Tensor:
     """The gated delta rule over the packed batch (csrc/delta_rule.cu): ``act`` [N, 2 G D + H V]
     holds query heads, key heads and value heads after the convolution; ``ab`` float32
     [N, 2 H] the decay and step inputs; ``state`` float32 [slots, H, V, D] is read and written
@@ -1604,7 +1629,8 @@ def delta_rule(act: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias
     if log_decay is not None:
         return _delta_rule_channels(act, ab, state, row_start, row_slot, out, n_rows, n_heads,
                                     n_kv_heads, key_dim, value_dim, max_new, log_decay,
-                                    n_heads if b_col is None else b_col, longest)
+                                    n_heads if b_col is None else b_col, longest, shortest,
+                                    min_chunked)
     _need(a_log, torch.float32, "A_log")
     _need(dt_bias, torch.float32, "dt_bias")
     _need(state, torch.float32, "state")
@@ -1620,11 +1646,15 @@ def delta_rule(act: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias
         raise KernelError("delta_rule shapes")
     if not 1 <= key_dim <= DELTA_MAX_KEY_DIM:
         raise KernelError(f"delta_rule takes key sizes up to {DELTA_MAX_KEY_DIM}, got {key_dim}")
-    _check(_load(*delta_rule_library(key_dim)).sllm_delta_rule(
+    lib = _load(*delta_rule_library(key_dim))
+    scratch, min_chunked = _delta_chunks(lib, n, n_rows, n_heads, value_dim,
+                                         0 if max_new == 1 else longest, min_chunked, state)
+    _check(lib.sllm_delta_rule(
         _ptr(act), c_int64(act.stride(0)), _ptr(ab), c_int64(ab.stride(0)), _ptr(a_log),
         _ptr(dt_bias), _ptr(state), _ptr(row_start), _ptr(row_slot), _ptr(out), c_int(n_rows),
         c_int(max_new), c_int(n_heads), c_int(n_kv_heads), c_int(value_dim), c_void_p(0),
-        c_int64(0), c_int(n_heads), c_void_p(0), c_int(0), c_int(_code(act.dtype)), _stream()),
+        c_int64(0), c_int(n_heads), c_void_p(0), c_int(0), _ptr(scratch), c_int(n),
+        c_int(min_chunked), c_int(shortest), c_int(_code(act.dtype)), _stream()),
         "delta_rule")
     return out
 
@@ -1638,7 +1668,8 @@ DELTA_CHUNK = 16
 
 
 def _delta_rule_channels(act, ab, state, row_start, row_slot, out, n_rows, n_heads, n_kv_heads,
-                         key_dim, value_dim, max_new, log_decay, b_col, longest) -> torch.Tensor:
+                         key_dim, value_dim, max_new, log_decay, b_col, longest, shortest,
+                         min_chunked) -> torch.Tensor:
     _need(log_decay, torch.float32, "log_decay", contiguous=False)
     _need(state, torch.float32, "state")
     _need(row_start, torch.int32, "row_start")
@@ -1655,17 +1686,20 @@ def _delta_rule_channels(act, ab, state, row_start, row_slot, out, n_rows, n_hea
     if not 1 <= key_dim <= DELTA_CHANNEL_MAX_KEY_DIM:
         raise KernelError(f"delta_rule with a decay per channel takes key sizes up to "
                           f"{DELTA_CHANNEL_MAX_KEY_DIM}, got {key_dim}")
+    lib = _load(*delta_rule_library(key_dim))
+    scratch, min_chunked = _delta_chunks(lib, n, n_rows, n_heads, value_dim,
+                                         0 if max_new == 1 else longest, min_chunked, state)
     tables = None
-    if longest > 1 and max_new != 1:
+    if longest > 1 and max_new != 1 and (scratch is None or shortest < min_chunked):
         slots = n // DELTA_CHUNK + n_rows + 1
         tables = torch.empty((slots, n_heads, 2 * DELTA_CHUNK, DELTA_CHUNK), dtype=torch.float32,
                              device=act.device)
-    _check(_load(*delta_rule_library(key_dim)).sllm_delta_rule(
+    _check(lib.sllm_delta_rule(
         _ptr(act), c_int64(act.stride(0)), _ptr(ab), c_int64(ab.stride(0)), c_void_p(0),
         c_void_p(0), _ptr(state), _ptr(row_start), _ptr(row_slot), _ptr(out), c_int(n_rows),
         c_int(max_new), c_int(n_heads), c_int(n_kv_heads), c_int(value_dim), _ptr(log_decay),
-        c_int64(log_decay.stride(0)), c_int(b_col), _ptr(tables), c_int(longest),
-        c_int(_code(act.dtype)), _stream()),
+        c_int64(log_decay.stride(0)), c_int(b_col), _ptr(tables), c_int(longest), _ptr(scratch),
+        c_int(n), c_int(min_chunked), c_int(shortest), c_int(_code(act.dtype)), _stream()),
         "delta_rule")
     return out
 

@@ -1,0 +1,80 @@
+"""The delta rule's chunk kernels (long portions) against the rule written out in 64 bits, token by
+token, and beside the kernel that walks the tokens in order."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def ops():
+    from scratch_llm_b200.kernels import ops as o
+    return o
+
+
+def rand(*shape, seed=0, scale=1.0):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * scale
+
+
+def unit(x):
+    return x / torch.sqrt(x.square().sum(-1, keepdim=True) + 1e-6)
+
+
+def i32(v):
+    return torch.tensor(v, dtype=torch.int32, device=DEV)
+
+
+def close(got, want, what):
+    # 32-bit sums of up to 64 + D products, and as many roundings from chunk to chunk: a few hundred
+    # roundings of 2^-24 that add up like a walk, and a triangular system of unit keys that may grow
+    # them a little: 2^-24 * sqrt(512) * 8 = 1.1e-5
+    err = ((got.double().cpu() - want).norm() / want.norm()).item()
+    assert err < 2e-5, f"{what}: {err}"
+
+
+# edges of chunks and blocks, rows below the limit beside rows above it, rows without tokens
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("channels", [False, True])
+@pytest.mark.parametrize("D,V,H,G,odd", [(128, 128, 2, 1, 0), (64, 72, 3, 3, 0), (32, 37, 2, 2, 1)])
+@pytest.mark.parametrize("lengths", [[128], [129, 3, 0, 191, 1], [193, 127, 64], [255, 256]])
+def test_delta_rule_in_chunks(dtype, channels, D, V, H, G, odd, lengths):
+    n, rows = sum(lengths), len(lengths)
+    # (an odd row stride: no reads of several elements)
+    act = rand(n, 2 * G * D + H * V + odd, seed=1).to(dtype).to(DEV)
+    ab = rand(n, 2 * H, seed=2).to(DEV)
+    A_log, dt_bias = rand(H, seed=3), rand(H, seed=4)
+    # decays from nearly none to ones that leave nothing
+    log_decay = -torch.exp(rand(n, H * D, seed=5, scale=2.0) - 2.0)
+    log_decay[:, ::7] = -torch.exp(rand(n, log_decay[:, ::7].shape[1], seed=6) + 3.0)
+    start = rand(rows + 1, H, V, D, seed=7)
+    slots = list(range(rows, 0, -1))
+    q, k, v = act.double().cpu()[:, :2 * G * D + H * V].split([G * D, G * D, H * V], 1)
+    q = unit(q.view(n, G, D)).repeat_interleave(H // G, 1) * D ** -0.5
+    k = unit(k.view(n, G, D)).repeat_interleave(H // G, 1)
+    v = v.view(n, H, V)
+    x = ab.double().cpu()
+    beta = torch.sigmoid(x[:, H:])
+    g = torch.exp(log_decay.double()).view(n, H, D) if channels else torch.exp(
+        -torch.exp(A_log.double()) * torch.nn.functional.softplus(x[:, :H] + dt_bias.double()))[..., None]
+    want, want_S, t = [], [], 0
+    for r, length in enumerate(lengths):
+        S = start[slots[r]].double()
+        for _ in range(length):
+            S = S * g[t][:, None]
+            u = beta[t][:, None] * (v[t] - (S @ k[t][..., None])[..., 0])
+            S = S + u[..., None] * k[t][:, None]
+            want.append((S @ q[t][..., None])[..., 0])
+            t += 1
+        want_S.append(S)
+    want, want_S = torch.stack(want), torch.stack(want_S)
+    row_start = i32([sum(lengths[:i]) for i in range(rows + 1)])
+    for min_chunked in (None, 0):
+        S = start.to(DEV).clone()
+        out = torch.full((n, H * V), float("nan"), device=DEV)
+        ops().delta_rule(act, ab, None if channels else A_log.to(DEV), None if channels else dt_bias.to(DEV), S,
+                         row_start, i32(slots), out, rows, H, G, D, V, longest=max(lengths), shortest=min(lengths),
+                         log_decay=log_decay.to(DEV) if channels else None, min_chunked=min_chunked)
+        close(out.view(n, H, V), want, f"out, min_chunked {min_chunked}")
+        close(S[slots], want_S, f"state, min_chunked {min_chunked}")
+        assert torch.equal(S[0].cpu(), start[0])
