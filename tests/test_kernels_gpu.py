@@ -697,3 +697,22 @@ def test_sampling_distribution_and_draws(ops, V):
     assert freq[want == 0].sum() <= 1.0 / n_draws * 2
     top = want.argsort(descending=True)[:5]
     torch.testing.assert_close(freq[top], want[top], rtol=0.3, atol=0.01)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 3, 4), (16, 16, 64), (17, 130, 60), (16, 33, 68), (33, 32, 32), (65, 95, 100),
+                                   (130, 20480, 20), (1030, 1090, 36)])
+def test_gemm_simt_tiles(m, n, k):
+    """The 32-bit product's kernels at the edges of their tiles: one chain of multiply-adds over k per
+    output whichever kernel takes the size, so all of them give the same bits as the plainest one (which
+    serves rows that allow no 16-byte requests), and a row does not depend on the rows beside it."""
+    from scratch_llm_b200.kernels import ops
+    g = torch.Generator().manual_seed(m * n + k)
+    x = torch.randn(m, k, generator=g).cuda()
+    w = torch.randn(n, k, generator=g).cuda()
+    got = ops.gemm_simt(x, w, torch.full((m, n), float("nan"), device="cuda"))
+    odd = torch.empty(m, k + 1, device="cuda")[:, :k].copy_(x)      # (rows of another alignment)
+    assert torch.equal(got, ops.gemm_simt(odd, w, torch.empty(m, n, device="cuda")))
+    assert torch.equal(got[:1], ops.gemm_simt(x[:1], w, torch.empty(1, n, device="cuda")))
+    want = x.double() @ w.double().t()
+    # k products of about 1, each rounded to 2^-24 and as many sums
+    assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -24 * k ** 0.5 * 4
