@@ -22,34 +22,51 @@ namespace sllm {
 
 constexpr int HD = SLLM_HEAD_DIM;
 static_assert(HD >= 1 && HD <= 640, "head size: 1 to 640");
-constexpr int BQ = 16, BKV = 32, THREADS = 128, ROWS_PER_WARP = 4;
+constexpr int BKV = 32, THREADS = 128, WARPS = THREADS / 32;
 constexpr int DPL = (HD + 31) / 32;  // head dims per lane
-constexpr int KS_LD = HD + 1;
+constexpr bool QUADS = HD % 4 == 0;  // rows of whole 16-byte words
+constexpr int KS_LD = QUADS ? HD + 4 : HD + 1;     // (neighbouring keys start on other banks)
+constexpr bool PAIRS = HD % 64 == 0; // a lane's dims are pairs of neighbours
+// Queries of a warp: a read of a key or a value in shared memory serves all of them, and a tile of keys
+// that a CTA fetches serves WARPS times as many.  Eight for long portions, where registers and shared
+// memory hold them; one for steps of a few tokens, whose other queries would be worked on for nothing.
+// 777 tokens, 32 heads of 64: 317 us with four queries a warp and a read per operand, 220 with eight.
+constexpr int LONG_QUERIES = HD <= 128 ? 8 : 4;
 
-constexpr size_t smem_floats() {
-    return (size_t)BQ * HD + (size_t)BKV * KS_LD + (size_t)BKV * HD + (size_t)BQ * BKV;
+constexpr size_t smem_floats(int rpw) {
+    return (size_t)WARPS * rpw * HD + (size_t)BKV * KS_LD + (size_t)BKV * HD + (size_t)WARPS * rpw * BKV;
 }
 
-template <typename T>
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+    const uint2 r = *reinterpret_cast<const uint2*>(p);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
+    return make_float4(__low2float(h[0]), __high2float(h[0]), __low2float(h[1]), __high2float(h[1]));
+}
+
+// RPW queries a warp.  vec: pages allow reads of four elements.  Every query is one chain over the dims per
+// score and over the keys per output, whatever RPW is.
+template <typename T, int RPW>
 __global__ void __launch_bounds__(THREADS)
 attn_simt_kernel(const T* __restrict__ q, int64_t q_stride, const T* __restrict__ pages,
                  const int* __restrict__ block_table, int table_stride, int page_size,
                  const int* __restrict__ row_start, const int* __restrict__ row_pos0,
                  T* __restrict__ out, int64_t out_stride, int H, int G, float scale, int window,
                  const float* __restrict__ slopes, const float* __restrict__ sinks, int planes,
-                 float softcap, int chunk) {
-    extern __shared__ float smem[];
+                 float softcap, int chunk, int vec) {
+    constexpr int BQ = WARPS * RPW;
+    extern __shared__ __align__(16) float smem[];
     __shared__ long long key_base[BKV];  // element offset of each key's K row, -1 if absent
-    float* Qs = smem;
-    float* Ks = Qs + BQ * HD;
-    float* Vs = Ks + BKV * KS_LD;
-    float* Ss = Vs + BKV * HD;
+    float* Qs = smem;                    // [BQ][HD]
+    float* Ks = Qs + BQ * HD;            // [BKV][KS_LD]
+    float* Vs = Ks + BKV * KS_LD;        // [BKV][HD]
+    float* Ss = Vs + BKV * HD;           // [WARPS][BKV][RPW]: probabilities
 
     const int r = blockIdx.y, h = blockIdx.z;
     const int g = h / (H / G);
     const int t0 = row_start[r];
     const int n_new = row_start[r + 1] - t0;
-    const int q0 = blockIdx.x * BQ;
+    const int q0 = (gridDim.x - 1 - blockIdx.x) * BQ;    // the queries with the most keys first
     if (q0 >= n_new) return;
     const int nq = min(BQ, n_new - q0);
     const int first_pos = row_pos0[r] + q0;
@@ -67,9 +84,9 @@ attn_simt_kernel(const T* __restrict__ q, int64_t q_stride, const T* __restrict_
                          : 0.f;
     }
 
-    float m[ROWS_PER_WARP], l[ROWS_PER_WARP], acc[ROWS_PER_WARP][DPL];
+    float m[RPW], l[RPW], acc[RPW][DPL];
 #pragma unroll
-    for (int a = 0; a < ROWS_PER_WARP; ++a) {
+    for (int a = 0; a < RPW; ++a) {
         m[a] = -INFINITY;
         l[a] = 0.f;
 #pragma unroll
@@ -77,6 +94,9 @@ attn_simt_kernel(const T* __restrict__ q, int64_t q_stride, const T* __restrict_
     }
     // (one plane: the values are the leading entries of the keys themselves)
     const int64_t v_offset = (int64_t)(planes - 1) * G * page_size * HD;
+    const float* qs = Qs + warp * HD;              // query a of this warp: row warp + WARPS * a
+    const float* kj = Ks + lane * KS_LD;
+    float* ps = Ss + warp * BKV * RPW;
 
     for (int kt = k_lo; kt <= last_pos; kt += BKV) {
         __syncthreads();  // the previous tile's Ks / Vs / key_base are no longer read
@@ -91,32 +111,63 @@ attn_simt_kernel(const T* __restrict__ q, int64_t q_stride, const T* __restrict_
             key_base[tid] = base;
         }
         __syncthreads();
-        for (int idx = tid; idx < BKV * HD; idx += THREADS) {
-            const int j = idx / HD, d = idx - j * HD;
-            const long long base = key_base[j];
-            float kv = 0.f, vv = 0.f;
-            if (base >= 0) {
-                kv = to_float(pages[base + d]);
-                vv = to_float(pages[base + v_offset + d]);
+        if (QUADS && vec) {
+#pragma unroll 4
+            for (int idx = tid; idx < BKV * HD / 4; idx += THREADS) {
+                const int j = idx / (HD / 4), d = (idx - j * (HD / 4)) * 4;
+                const long long base = key_base[j];
+                float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
+                if (base >= 0) {
+                    kv = load4(pages + base + d);
+                    vv = load4(pages + base + v_offset + d);
+                }
+                *reinterpret_cast<float4*>(Ks + j * KS_LD + d) = kv;
+                *reinterpret_cast<float4*>(Vs + j * HD + d) = vv;
             }
-            Ks[j * KS_LD + d] = kv;
-            Vs[j * HD + d] = vv;
+        } else {
+            for (int idx = tid; idx < BKV * HD; idx += THREADS) {
+                const int j = idx / HD, d = idx - j * HD;
+                const long long base = key_base[j];
+                float kv = 0.f, vv = 0.f;
+                if (base >= 0) {
+                    kv = to_float(pages[base + d]);
+                    vv = to_float(pages[base + v_offset + d]);
+                }
+                Ks[j * KS_LD + d] = kv;
+                Vs[j * HD + d] = vv;
+            }
         }
         __syncthreads();
 
         const int kpos = kt + lane;
+        float dot[RPW];
 #pragma unroll
-        for (int a = 0; a < ROWS_PER_WARP; ++a) {
-            const int i = warp + 4 * a;
-            const float* qi = Qs + i * HD;
-            const float* kj = Ks + lane * KS_LD;
-            float dot = 0.f;
-#pragma unroll 8
-            for (int d = 0; d < HD; ++d) dot = fmaf(qi[d], kj[d], dot);
-            const int qpos = first_pos + i;
+        for (int a = 0; a < RPW; ++a) dot[a] = 0.f;
+        if (QUADS) {
+#pragma unroll 4
+            for (int d = 0; d < HD; d += 4) {
+                const float4 k = load4(kj + d);
+#pragma unroll
+                for (int a = 0; a < RPW; ++a) {
+                    const float4 x = load4(qs + a * WARPS * HD + d);
+                    dot[a] = fmaf(x.w, k.w, fmaf(x.z, k.z, fmaf(x.y, k.y, fmaf(x.x, k.x, dot[a]))));
+                }
+            }
+        } else {
+#pragma unroll 4
+            for (int d = 0; d < HD; ++d) {
+                const float k = kj[d];
+#pragma unroll
+                for (int a = 0; a < RPW; ++a) dot[a] = fmaf(qs[a * WARPS * HD + d], k, dot[a]);
+            }
+        }
+        const bool there = key_base[lane] >= 0;
+#pragma unroll
+        for (int a = 0; a < RPW; ++a) {
+            const int i = warp + WARPS * a, qpos = first_pos + i;
             const bool valid = i < nq && kpos <= qpos && (window <= 0 || kpos > qpos - window) &&
-                               (chunk <= 0 || kpos >= qpos / chunk * chunk) && key_base[lane] >= 0;
-            float sc = dot * scale;
+                               (chunk <= 0 || kpos >= qpos / chunk * chunk) && there;
+            float sc = dot[a] * scale;
             if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
             const float s = valid ? sc - slope * (float)(qpos - kpos) : -INFINITY;
             const float m_new = fmaxf(m[a], warp_max(s));
@@ -129,25 +180,46 @@ attn_simt_kernel(const T* __restrict__ q, int64_t q_stride, const T* __restrict_
             m[a] = m_new;
 #pragma unroll
             for (int c = 0; c < DPL; ++c) acc[a][c] *= corr;
-            Ss[i * BKV + lane] = p;
+            ps[lane * RPW + a] = p;
         }
-        __syncwarp();  // each warp reads back only the rows of Ss it wrote
+        __syncwarp();  // each warp reads back only what it wrote
+#pragma unroll 4
+        for (int j = 0; j < BKV; ++j) {
+            float p[RPW];
+            if (RPW % 4 == 0) {
 #pragma unroll
-        for (int a = 0; a < ROWS_PER_WARP; ++a) {
-            const float* pi = Ss + (warp + 4 * a) * BKV;
-            for (int j = 0; j < BKV; ++j) {
-                const float p = pi[j];
+                for (int a = 0; a < RPW; a += 4) {
+                    const float4 x = load4(ps + j * RPW + a);
+                    p[a] = x.x; p[a + 1] = x.y; p[a + 2] = x.z; p[a + 3] = x.w;
+                }
+            } else {
 #pragma unroll
-                for (int c = 0; c < DPL; ++c) {
+                for (int a = 0; a < RPW; ++a) p[a] = ps[j * RPW + a];
+            }
+#pragma unroll
+            for (int c = 0; c < DPL; ++c) {
+                if (PAIRS) {          // dims 32 c + 2 lane and the next, in the entries c and c + 1
+                    if (c % 2) continue;
+                    const float2 v = *reinterpret_cast<const float2*>(Vs + j * HD + 32 * c + 2 * lane);
+#pragma unroll
+                    for (int a = 0; a < RPW; ++a) {
+                        acc[a][c] = fmaf(p[a], v.x, acc[a][c]);
+                        acc[a][c + 1] = fmaf(p[a], v.y, acc[a][c + 1]);
+                    }
+                } else {
                     const int d = lane + 32 * c;
-                    if (d < HD) acc[a][c] = fmaf(p, Vs[j * HD + d], acc[a][c]);
+                    if (d < HD) {
+                        const float v = Vs[j * HD + d];
+#pragma unroll
+                        for (int a = 0; a < RPW; ++a) acc[a][c] = fmaf(p[a], v, acc[a][c]);
+                    }
                 }
             }
         }
     }
 #pragma unroll
-    for (int a = 0; a < ROWS_PER_WARP; ++a) {
-        const int i = warp + 4 * a;
+    for (int a = 0; a < RPW; ++a) {
+        const int i = warp + WARPS * a;
         if (i >= nq) continue;
         float total = l[a], keep = 1.f;
         if (sinks && m[a] != -INFINITY) {
@@ -160,10 +232,35 @@ attn_simt_kernel(const T* __restrict__ q, int64_t q_stride, const T* __restrict_
         T* o = out + (int64_t)(t0 + q0 + i) * out_stride + (int64_t)h * HD;
 #pragma unroll
         for (int c = 0; c < DPL; ++c) {
-            const int d = lane + 32 * c;
+            const int d = PAIRS ? 32 * (c & ~1) + 2 * lane + (c & 1) : lane + 32 * c;
             if (d < HD) o[d] = from_float<T>(acc[a][c] * inv);
         }
     }
+}
+
+template <typename T, int RPW>
+static int launch(const void* q, int64_t q_stride, const void* pages, const int* block_table, int table_stride,
+                  int page_size, const int* row_start, const int* row_pos0, void* out, int64_t out_stride,
+                  int n_rows, int max_new, int H, int G, float scale, int window, const float* slopes,
+                  const float* sinks, int planes, float softcap, int chunk, cudaStream_t stream) {
+    const size_t smem = smem_floats(RPW) * sizeof(float);
+    const cudaError_t e = cudaFuncSetAttribute(attn_simt_kernel<T, RPW>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    constexpr int BQ = WARPS * RPW;
+    const int vec = ((uintptr_t)pages & 15) == 0;
+    attn_simt_kernel<T, RPW><<<dim3((max_new + BQ - 1) / BQ, n_rows, H), THREADS, smem, stream>>>(
+        (const T*)q, q_stride, (const T*)pages, block_table, table_stride, page_size, row_start, row_pos0,
+        (T*)out, out_stride, H, G, scale, window, slopes, sinks, planes, softcap, chunk, vec);
+    SLLM_LAUNCH_CHECK();
+    return 0;
+}
+
+template <typename T, typename... Args>
+static int launch_for(int max_new, Args... args) {
+    if (max_new <= WARPS) return launch<T, 1>(args...);
+    if (max_new <= 4 * WARPS) return launch<T, 4>(args...);
+    return launch<T, LONG_QUERIES>(args...);
 }
 
 }  // namespace sllm
@@ -193,28 +290,13 @@ SLLM_EXPORT int sllm_attn_simt(const void* q, int64_t q_stride, const void* page
     if (H <= 0 || G <= 0 || H % G != 0 || page_size <= 0 || window < 0 || chunk < 0 || planes < 1 || planes > 2)
         return (int)cudaErrorInvalidValue;
     if (n_rows > 65535 || H > 65535) return (int)cudaErrorInvalidValue;
-    const size_t smem = smem_floats() * sizeof(float);
-    dim3 grid((max_new + BQ - 1) / BQ, n_rows, H);
-    cudaError_t e;
-    if (dtype == 0) {
-        e = cudaFuncSetAttribute(attn_simt_kernel<float>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        attn_simt_kernel<float><<<grid, THREADS, smem, stream>>>(
-            (const float*)q, q_stride, (const float*)pages, block_table, table_stride, page_size,
-            row_start, row_pos0, (float*)out, out_stride, H, G, scale, window, slopes, sinks,
-            planes, softcap, chunk);
-    } else if (dtype == 1) {
-        e = cudaFuncSetAttribute(attn_simt_kernel<__nv_bfloat16>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        attn_simt_kernel<__nv_bfloat16><<<grid, THREADS, smem, stream>>>(
-            (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)pages, block_table,
-            table_stride, page_size, row_start, row_pos0, (__nv_bfloat16*)out, out_stride, H, G,
-            scale, window, slopes, sinks, planes, softcap, chunk);
-    } else {
-        return (int)cudaErrorInvalidValue;
-    }
-    SLLM_LAUNCH_CHECK();
-    return 0;
+    if (dtype == 0)
+        return launch_for<float>(max_new, q, q_stride, pages, block_table, table_stride, page_size, row_start,
+                                 row_pos0, out, out_stride, n_rows, max_new, H, G, scale, window, slopes, sinks,
+                                 planes, softcap, chunk, stream);
+    if (dtype == 1)
+        return launch_for<__nv_bfloat16>(max_new, q, q_stride, pages, block_table, table_stride, page_size,
+                                         row_start, row_pos0, out, out_stride, n_rows, max_new, H, G, scale,
+                                         window, slopes, sinks, planes, softcap, chunk, stream);
+    return (int)cudaErrorInvalidValue;
 }
