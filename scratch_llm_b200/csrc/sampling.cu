@@ -208,16 +208,17 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, int V,
 // barrier, and each adds the eight slots in rank order, so that all hold the same bits and take
 // the same branches.  (Two sets of slots take turns: a CTA can be one round ahead of another,
 // never two.)  The bisection stops as soon as no probability lies strictly between its bounds:
-// the threshold can then only be the upper one (22 rounds instead of 31 for 128,256 random
-// logits; eight ways per round instead of two took 8 rounds but as long, a round's arithmetic
-// growing as its number fell).  Arithmetic and rules are those of
+// the threshold can then only be the upper one (22 steps instead of 31 for 128,256 random
+// logits).  A round takes two steps, with the sums that either outcome of the first would ask for: the
+// same decisions from the same sums, half the meetings (64 rows: 211 us with one step a round, 172
+// with two; three took 8 rounds but as long, a round's arithmetic growing as its number fell).  Arithmetic and rules are those of
 // sample_kernel; only the order of the sums differs.
 constexpr int SC_RANKS = 8;
 constexpr int SC_MAX_SLICE = 24576;     // values a CTA keeps in shared memory (two CTAs share an SM)
 constexpr int SC_MIN_VOCAB = 8192;      // below, one CTA per row has the row in L1 anyway
 
 struct ScSlots {
-    float f[2][SC_RANKS][2];
+    float f[2][SC_RANKS][4];
     ArgMax a[2][SC_RANKS];
     int i[2][SC_RANKS];
 };
@@ -246,21 +247,22 @@ __device__ __forceinline__ float2 sc_all_sum(cg::cluster_group& cluster, ScSlots
 
 
 // N values per CTA summed over the block and then over the cluster (in v, the same bits in every
-// thread of every CTA).  scratch: [32][N] floats.
+// thread of every CTA).  scratch: [2][32][N] floats.
 template <int N>
 __device__ __forceinline__ void sc_all_sum_n(cg::cluster_group& cluster, ScSlots* slots, int& round,
                                              float (&v)[N], float* scratch) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < N; ++k) v[k] = warp_sum(v[k]);
-    __syncthreads();        // scratch may still be read from the round before
+    // (two halves of scratch take turns as the slots do: the cluster's barrier lies between)
+    const int set = round & 1;
+    ++round;
+    scratch += set * (SAMPLE_THREADS / 32) * N;
     if (lane == 0) {
 #pragma unroll
         for (int k = 0; k < N; ++k) scratch[warp * N + k] = v[k];
     }
     __syncthreads();
-    const int set = round & 1;
-    ++round;
     if (threadIdx.x < SC_RANKS * N) {
         // thread (peer, k): the block's sum of value k, in warp order, into the peer's slot
         const int peer = threadIdx.x / N, k = threadIdx.x % N;
@@ -291,7 +293,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t ld, int V, int s
     __shared__ float fscratch[33];
     __shared__ ArgMax ascratch[33];
     __shared__ float chunk_sum[32];
-    __shared__ float nscratch[NUCLEUS ? 32 * 2 : 1];
+    __shared__ float nscratch[NUCLEUS ? 2 * 32 * 4 : 1];
     __shared__ int chosen;
     __shared__ ScSlots slots;
     cg::cluster_group cluster = cg::this_cluster();
@@ -342,20 +344,29 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t ld, int V, int s
             // f(t) = sum of p_i > t.  lo: f(lo) > tp.  hi: f(hi) <= tp.  p_max = 1 / Z.
             unsigned lo = 0u, hi = __float_as_uint(inv_z);
             while (hi - lo > 1u) {
+                // two steps of the bisection in one round: the middle, and the middles of the
+                // two halves of which one is asked next
                 const unsigned mid = lo + (hi - lo) / 2u;
-                const float t = __uint_as_float(mid);
-                float v[2] = {0.f, 0.f};       // f(mid); how many probabilities lie inside
+                const unsigned left = lo + (mid - lo) / 2u, right = mid + (hi - mid) / 2u;
+                const float t = __uint_as_float(mid), tl = __uint_as_float(left), tr = __uint_as_float(right);
+                // f of the three; how many probabilities lie inside
+                float v[4] = {0.f, 0.f, 0.f, 0.f};
                 for (int i = tid; i < n; i += SAMPLE_THREADS) {
                     const float p = ps[i];
                     v[0] += p > t ? p : 0.f;
+                    v[1] += p > tl ? p : 0.f;
+                    v[2] += p > tr ? p : 0.f;
                     const unsigned bits = __float_as_uint(p);
-                    v[1] += (bits > lo && bits < hi && bits != mid) ? 1.f : 0.f;
+                    v[3] += (bits > lo && bits < hi && bits != mid) ? 1.f : 0.f;
                 }
-                sc_all_sum_n<2>(cluster, &slots, round, v, nscratch);
-                if (v[0] <= tp) hi = mid; else lo = mid;
+                sc_all_sum_n<4>(cluster, &slots, round, v, nscratch);
+                const bool down = v[0] <= tp;
+                if (down) hi = mid; else lo = mid;
                 // no probability strictly inside the bounds (mid has just become one of them):
                 // f is constant on [lo, hi), so the search can only end at this hi
-                if (v[1] == 0.f) break;
+                if (v[3] == 0.f || hi - lo <= 1u) break;
+                if ((down ? v[1] : v[2]) <= tp) hi = down ? left : right;
+                else lo = down ? left : right;
             }
             thresh = __uint_as_float(hi);
         }
