@@ -151,24 +151,34 @@ __device__ __forceinline__ void tile16(const float* x, const float* y, const flo
     Two acc[4][2];
 #pragma unroll
     for (int a = 0; a < 4; ++a) acc[a][0] = acc[a][1] = two(0.f, 0.f);
+    for (int d0 = 0; d0 < D; d0 += 32) {
+        Two part[4][2];              // (sums of 32 channels each: chains over all of them round more)
+#pragma unroll
+        for (int a = 0; a < 4; ++a) part[a][0] = part[a][1] = two(0.f, 0.f);
 #pragma unroll 4
-    for (int d = 0; d < D; d += 4) {
-        Four yv[2];
+        for (int d = d0; d < d0 + 32; d += 4) {
+            Four yv[2];
 #pragma unroll
-        for (int b = 0; b < 2; ++b) yv[b] = load22(y + (sg + 8 * b) * LD + d);
-        if (mid) {
-            const Four m = load22(mid + d);
-            const Two zero = two(0.f, 0.f);
+            for (int b = 0; b < 2; ++b) yv[b] = load22(y + (sg + 8 * b) * LD + d);
+            if (mid) {
+                const Four m = load22(mid + d);
+                const Two zero = two(0.f, 0.f);
 #pragma unroll
-            for (int b = 0; b < 2; ++b) yv[b] = {fma2(yv[b].a, m.a, zero), fma2(yv[b].b, m.b, zero)};
+                for (int b = 0; b < 2; ++b) yv[b] = {fma2(yv[b].a, m.a, zero), fma2(yv[b].b, m.b, zero)};
+            }
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                const Four xv = load22(x + (tg + 4 * a) * LD + d);
+#pragma unroll
+                for (int b = 0; b < 2; ++b)
+                    part[a][b] = fma2(xv.b, yv[b].b, fma2(xv.a, yv[b].a, part[a][b]));
+            }
         }
+        const Two one = two(1.f, 1.f);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const Four xv = load22(x + (tg + 4 * a) * LD + d);
+        for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int b = 0; b < 2; ++b)
-                acc[a][b] = fma2(xv.b, yv[b].b, fma2(xv.a, yv[b].a, acc[a][b]));
-        }
+            for (int b = 0; b < 2; ++b) acc[a][b] = fma2(part[a][b], one, acc[a][b]);
     }
 #pragma unroll
     for (int a = 0; a < 4; ++a)
@@ -363,8 +373,13 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prep_head_kernel(const PrepAr
                 if (j <= i) {
                     uint32_t b[4];
                     ldsm4(b, right + (BT * j * LD + 16 * kk) * 2);
-                    mma_bf16(acc[j][0], f, b);
-                    mma_bf16(acc[j][1], f, b + 2);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float part[4] = {0.f, 0.f, 0.f, 0.f};
+                        mma_bf16(part, f, b + 2 * h);
+#pragma unroll
+                        for (int w = 0; w < 4; ++w) acc[j][h][w] += part[w];
+                    }
                 }
         }
 #pragma unroll
@@ -615,7 +630,10 @@ __global__ void __launch_bounds__(PREP_THREADS, 1) prep_channels_kernel(const Pr
 // ------------------------------------------------------------------------------------- pass
 
 // c += a b of 32-bit operands as bfloat16 parts (PARTS each, which hold all of their 24 bits): the six
-// products of parts that reach above 2^-24, small ones first.
+// products of parts that reach above 2^-24, small ones first.  mma.sync cuts its sums off instead of
+// rounding them: longer sums are therefore added up outside, from a fresh accumulator per 16 products.
+// (600 tokens, weak decays, 128 x 128, error of the read-outs against 64 bits: 1.3e-6 with one accumulator
+// over all 192 products, 2.2e-7 now, 3.2e-7 token by token in fmaf; 2,048 tokens, 16 heads: 245 -> 252 us.)
 __device__ __forceinline__ void mma_parts(float* c, const uint32_t (*a)[4], const uint32_t (*b)[2]) {
     mma_bf16(c, a[1], b[1]);
     mma_bf16(c, a[0], b[2]);
@@ -623,6 +641,12 @@ __device__ __forceinline__ void mma_parts(float* c, const uint32_t (*a)[4], cons
     mma_bf16(c, a[0], b[1]);
     mma_bf16(c, a[1], b[0]);
     mma_bf16(c, a[0], b[0]);
+}
+__device__ __forceinline__ void add_parts(float* c, const uint32_t (*a)[4], const uint32_t (*b)[2]) {
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+    mma_parts(sum, a, b);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] += sum[i];
 }
 __device__ __forceinline__ void split_b(float4 v, uint32_t (*b)[2]) {
     uint32_t p[PARTS];
@@ -760,7 +784,7 @@ pass_kernel(const Scratch z, float* __restrict__ state, const int* __restrict__ 
             for (int n = 0; n < 2; ++n) {
                 uint32_t right[PARTS][2];
                 split_b(y[2 * k + n], right);
-                mma_parts(acc[n], left, right);
+                add_parts(acc[n], left, right);
             }
         }
 #pragma unroll
@@ -849,7 +873,7 @@ out_kernel(const Scratch z, const int* __restrict__ row_start, float* __restrict
                 const float2 y = *reinterpret_cast<const float2*>(q + 8 * n * ld + k + 8);
                 uint32_t b[PARTS][2];
                 split_b(make_float4(x.x, x.y, y.x, y.y), b);
-                mma_parts(acc[n], a, b);
+                add_parts(acc[n], a, b);
             }
         }
     };
