@@ -27,6 +27,8 @@
 // heads of 128 x 128, bfloat16: one decay per head 733 -> 246 us, per channel 666 -> 343 us.
 #pragma once
 
+#include <algorithm>
+
 #include "scan_chunks.cuh"
 
 namespace sllm {
@@ -37,7 +39,7 @@ constexpr int LDT = TC + 4;              // row stride of A in shared memory
 constexpr int PREP_THREADS = 256, OUT_THREADS = 256, OUT_COLS = 64;
 constexpr int NC = 16;                   // columns of the state per CTA of the pass
 
-struct Scratch {                         // per (slot of a chunk, head), 32-bit
+struct Scratch {                         // per (slot, head), 32-bit
     float *W, *Y;                        // [TC][D] in the order in which the pass's threads take them
     float* Q;                            // [TC][D]
     float* X;                            // [V][TC]: X0, after the pass X
@@ -60,6 +62,53 @@ static inline Scratch scratch_at(float* at, int64_t n, int D, int64_t V) {
     s.decay = at; at += n * D;
     s.X = at;
     return s;
+}
+
+// The chunks of a step are numbered over the rows that have any (at least min_chunked tokens), row after
+// row.  They are worked on in groups of as many as the scratch has slots: chunk `first` + i has slot i.
+struct Group { int first, count; };
+struct RowAt { int row, t0, n_new, first; };     // first: the number of the row's first chunk
+// BY_CHUNK: the row of the group's chunk number `which`; else the row number `which` of those that have chunks
+// in the group or after it.
+template <bool BY_CHUNK>
+__device__ __forceinline__ bool find_row(const int* row_start, int n_rows, int min_chunked, const Group& group,
+                                         int which, RowAt& at) {
+    const int lane = threadIdx.x & 31;
+    int chunks_before = 0, rows_before = 0;
+    for (int r0 = 0; r0 < n_rows; r0 += 32) {
+        const int r = r0 + lane;
+        int start = 0, count = 0;
+        if (r < n_rows) {
+            start = row_start[r];
+            count = row_start[r + 1] - start;
+        }
+        const bool has = r < n_rows && count >= min_chunked;
+        if (!__any_sync(0xffffffffu, has)) continue;
+        const int chunks = has ? (count + TC - 1) / TC : 0;
+        int end = chunks;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int more = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += more;
+        }
+        end += chunks_before;
+        const int first = end - chunks;
+        const unsigned open = __ballot_sync(0xffffffffu, has && end > group.first);
+        const bool mine = BY_CHUNK ? group.first + which >= first && group.first + which < end
+                                   : (open >> lane & 1) && rows_before + __popc(open & ((1u << lane) - 1)) == which;
+        const unsigned hit = __ballot_sync(0xffffffffu, mine);
+        if (hit) {
+            const int who = __ffs(hit) - 1;
+            at.row = r0 + who;
+            at.t0 = __shfl_sync(0xffffffffu, start, who);
+            at.n_new = __shfl_sync(0xffffffffu, count, who);
+            at.first = __shfl_sync(0xffffffffu, first, who);
+            return true;
+        }
+        chunks_before = __shfl_sync(0xffffffffu, end, 31);
+        rows_before += __popc(open);
+    }
+    return false;
 }
 
 // Two multiply-adds in one instruction, each rounded as fmaf rounds.
@@ -274,7 +323,7 @@ template <int D, typename T> constexpr size_t prep_head_smem() {
 // tokens.  52 us at 2,048 tokens and 16 heads of 128 x 128; bound by the substitution's shared-memory reads
 // (544 of 16 bytes a warp) and, with two CTAs of eight warps an SM, by latencies.
 template <int D, typename T>
-__global__ void __launch_bounds__(PREP_THREADS, 2) prep_head_kernel(const PrepArgs a, const Scratch z) {
+__global__ void __launch_bounds__(PREP_THREADS, 2) prep_head_kernel(const PrepArgs a, const Scratch z, const Group group) {
     constexpr int LD = HEAD_LD<D, T>;
     extern __shared__ __align__(16) float sm[];
     float* At = sm;
@@ -284,11 +333,11 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prep_head_kernel(const PrepAr
     pdl_wait();
     pdl_trigger();
     const int slot = blockIdx.x, head = blockIdx.y;
-    int row, t0, c0, n_new;
-    if (!find_chunk(a.row_start, a.n_rows, a.min_chunked, slot, row, t0, c0, n_new)) return;
-    const int nt = min(TC, n_new - c0);
+    RowAt row;
+    if (!find_row<true>(a.row_start, a.n_rows, a.min_chunked, group, slot, row)) return;
+    const int c0 = (group.first + slot - row.first) * TC, nt = min(TC, row.n_new - c0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t tok = t0 + c0, at = (int64_t)slot * a.H + head;
+    const int64_t tok = row.t0 + c0, at = (int64_t)slot * a.H + head;
     const T* x = reinterpret_cast<const T*>(a.x) + tok * a.ld;
     const int g = head / a.per;
     {
@@ -497,7 +546,7 @@ __device__ __forceinline__ void block_pairs(const float* x, const float* y, cons
 // k e^{l}; L = the decays, then k e^{border - l} (l: sums of logarithms from the block's border on).  One
 // CTA an SM (127 KB at D = 128); 256 us at 3,001 tokens in four rows and 16 heads of 128 x 128.
 template <int D, typename T>
-__global__ void __launch_bounds__(PREP_THREADS, 1) prep_channels_kernel(const PrepArgs a, const Scratch z) {
+__global__ void __launch_bounds__(PREP_THREADS, 1) prep_channels_kernel(const PrepArgs a, const Scratch z, const Group group) {
     constexpr int LD = D + 4;
     extern __shared__ __align__(16) float sm[];
     float* R = sm;
@@ -512,11 +561,11 @@ __global__ void __launch_bounds__(PREP_THREADS, 1) prep_channels_kernel(const Pr
     pdl_wait();
     pdl_trigger();
     const int slot = blockIdx.x, head = blockIdx.y;
-    int row, t0, c0, n_new;
-    if (!find_chunk(a.row_start, a.n_rows, a.min_chunked, slot, row, t0, c0, n_new)) return;
-    const int nt = min(TC, n_new - c0);
+    RowAt row;
+    if (!find_row<true>(a.row_start, a.n_rows, a.min_chunked, group, slot, row)) return;
+    const int c0 = (group.first + slot - row.first) * TC, nt = min(TC, row.n_new - c0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t tok = t0 + c0, at = (int64_t)slot * a.H + head;
+    const int64_t tok = row.t0 + c0, at = (int64_t)slot * a.H + head;
     const T* x = reinterpret_cast<const T*>(a.x) + tok * a.ld;
     const float* lg = a.log_decay + tok * a.ldl + (int64_t)head * D;
     const int g = head / a.per;
@@ -671,24 +720,27 @@ constexpr int LDP = TC + 8;              // row stride of what the pass's warps 
 // from shared memory a chunk took 4,700 cycles (shared-memory reads).
 template <int D>
 __global__ void __launch_bounds__(2 * D)
-pass_kernel(const Scratch z, float* __restrict__ state, const int* __restrict__ row_start,
-            const int* __restrict__ row_slot, int min_chunked, int H, int V) {
+pass_kernel(const Scratch z, const Group group, float* __restrict__ state, const int* __restrict__ row_start,
+            const int* __restrict__ row_slot, int n_rows, int min_chunked, int H, int V) {
     constexpr int WARPS = D / 16, THREADS = 32 * WARPS, QUADS = NC * TC / 4 / THREADS;
     __shared__ __align__(16) float sums[WARPS][NC][LDP];
     __shared__ __align__(16) bf16 parts[PARTS][NC][LDP];
     pdl_wait();
     pdl_trigger();
-    const int r = blockIdx.z, head = blockIdx.y, col0 = blockIdx.x * NC;
-    const int t0 = row_start[r], n_new = row_start[r + 1] - t0;
-    if (n_new < min_chunked) return;
+    const int head = blockIdx.y, col0 = blockIdx.x * NC;
+    RowAt row;
+    if (!find_row<false>(row_start, n_rows, min_chunked, group, blockIdx.z, row)) return;
+    // the row's chunks of this group: the state goes through memory between groups
+    const int slot0 = max(row.first - group.first, 0);
+    const int n_chunks = min(row.first + (row.n_new + TC - 1) / TC - group.first, group.count) - slot0;
+    if (n_chunks <= 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t chunk0 = (int64_t)(t0 / TC + r) * H + head;
-    const int n_chunks = (n_new + TC - 1) / TC;
+    const int64_t chunk0 = (int64_t)slot0 * H + head;
     // S[n][i]: column lane / 4 + 8 (i / 2), channel 16 warp + 8 n + 2 (lane % 4) + i % 2
     const int column = lane >> 2, channel = 16 * warp + (lane & 3) * 2;
     const bool live[2] = {col0 + column < V, col0 + column + 8 < V};
     float S[2][4];
-    float* st = state + (((int64_t)row_slot[r] * H + head) * V + col0 + column) * D + channel;
+    float* st = state + (((int64_t)row_slot[row.row] * H + head) * V + col0 + column) * D + channel;
 #pragma unroll
     for (int n = 0; n < 2; ++n)
 #pragma unroll
@@ -815,8 +867,8 @@ template <int D> constexpr size_t out_smem() { return (size_t)(TC + OUT_COLS) * 
 // of the SM covers.  (As fused multiply-adds it was bound by shared-memory reads.)
 template <int D>
 __global__ void __launch_bounds__(OUT_THREADS, 2)
-out_kernel(const Scratch z, const int* __restrict__ row_start, float* __restrict__ out, int n_rows,
-           int min_chunked, int H, int V) {
+out_kernel(const Scratch z, const Group group, const int* __restrict__ row_start, float* __restrict__ out,
+           int n_rows, int min_chunked, int H, int V) {
     constexpr int LD = D + 8;
     extern __shared__ __align__(16) float sm[];
     float* Qs = sm;                       // [TC][LD]
@@ -826,9 +878,9 @@ out_kernel(const Scratch z, const int* __restrict__ row_start, float* __restrict
     pdl_wait();
     pdl_trigger();
     const int slot = blockIdx.z, head = blockIdx.y, col0 = blockIdx.x * OUT_COLS;
-    int row, t0, c0, n_new;
-    if (!find_chunk(row_start, n_rows, min_chunked, slot, row, t0, c0, n_new)) return;
-    const int nt = min(TC, n_new - c0);
+    RowAt row;
+    if (!find_row<true>(row_start, n_rows, min_chunked, group, slot, row)) return;
+    const int c0 = (group.first + slot - row.first) * TC, nt = min(TC, row.n_new - c0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t at = (int64_t)slot * H + head;
     const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -884,16 +936,18 @@ out_kernel(const Scratch z, const int* __restrict__ row_start, float* __restrict
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int t = r0 + place + (i >> 1) * 8, c = col0 + n0 + 8 * n + pair + (i & 1);
-            if (t < nt && c < V) out[((int64_t)(t0 + c0 + t) * H + head) * V + c] = acc[n][i];
+            if (t < nt && c < V) out[((int64_t)(row.t0 + c0 + t) * H + head) * V + c] = acc[n][i];
         }
 }
 
 // --------------------------------------------------------------------------------- launches
 
+// `slots`: room of the scratch.  Launches for every chunk that a step of n_tokens tokens can have: a row with
+// chunks ends at most one short of a whole one more than its tokens fill.
 template <int D, typename T, bool CHANNEL>
 static inline int launch(const PrepArgs& a, const Scratch& z, float* state, const int* row_slot, float* out,
-                         int slots, cudaStream_t stream) {
-    void (*prep)(PrepArgs, Scratch);
+                         int n_tokens, int slots, cudaStream_t stream) {
+    void (*prep)(PrepArgs, Scratch, Group);
     if constexpr (CHANNEL) prep = prep_channels_kernel<D, T>;
     else prep = prep_head_kernel<D, T>;
     constexpr size_t smem = CHANNEL ? prep_channels_smem<D>() : prep_head_smem<D, T>();
@@ -901,14 +955,23 @@ static inline int launch(const PrepArgs& a, const Scratch& z, float* state, cons
     if (e != cudaSuccess) return (int)e;
     e = cudaFuncSetAttribute(out_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem<D>());
     if (e != cudaSuccess) return (int)e;
-    e = sllm_launch_pdl(prep, dim3(slots, a.H), dim3(PREP_THREADS), smem, stream, a, z);
-    if (e != cudaSuccess) return (int)e;
-    e = sllm_launch_pdl(pass_kernel<D>, dim3((a.V + NC - 1) / NC, a.H, a.n_rows), dim3(2 * D), 0, stream,
-                        z, state, a.row_start, row_slot, a.min_chunked, a.H, a.V);
-    if (e != cudaSuccess) return (int)e;
-    return (int)sllm_launch_pdl(out_kernel<D>, dim3((a.V + OUT_COLS - 1) / OUT_COLS, a.H, slots),
-                                dim3(OUT_THREADS), out_smem<D>(), stream, z, a.row_start, out, a.n_rows,
-                                a.min_chunked, a.H, a.V);
+    const int rows = std::min(a.n_rows, n_tokens / a.min_chunked), chunks = n_tokens / TC + rows;
+    const int per_row = (a.min_chunked + TC - 1) / TC;
+    if (rows == 0) return 0;
+    for (Group g = {0, 0}; g.first < chunks; g.first += slots) {
+        g.count = std::min(slots, chunks - g.first);
+        e = sllm_launch_pdl(prep, dim3(g.count, a.H), dim3(PREP_THREADS), smem, stream, a, z, g);
+        if (e != cudaSuccess) return (int)e;
+        // (rows of at least per_row chunks: this many can have some in the group)
+        const int group_rows = std::min(rows, g.count / per_row + 2);
+        e = sllm_launch_pdl(pass_kernel<D>, dim3((a.V + NC - 1) / NC, a.H, group_rows), dim3(2 * D), 0, stream, z, g,
+                            state, a.row_start, row_slot, a.n_rows, a.min_chunked, a.H, a.V);
+        if (e != cudaSuccess) return (int)e;
+        e = sllm_launch_pdl(out_kernel<D>, dim3((a.V + OUT_COLS - 1) / OUT_COLS, a.H, g.count), dim3(OUT_THREADS),
+                            out_smem<D>(), stream, z, g, a.row_start, out, a.n_rows, a.min_chunked, a.H, a.V);
+        if (e != cudaSuccess) return (int)e;
+    }
+    return 0;
 }
 
 }  // namespace chunks

@@ -700,16 +700,15 @@ SLLM_EXPORT int sllm_delta_rule_head_dim() { return D; }
 // chunk's keys, queries and sums of decays fit shared memory together: these key sizes.
 constexpr bool CHUNKS = D == 32 || D == 64 || D == 128;
 
-// Floats of scratch the chunk kernels take per chunk slot and head; 0: this key size has none.
+// Floats of scratch the chunk kernels take per chunk and head; 0: this key size has none.
 SLLM_EXPORT int64_t sllm_delta_rule_chunk_floats(int V) {
     return CHUNKS ? chunks::scratch_floats(D, V) : 0;
 }
 
 template <typename T, bool CHANNEL>
-static int launch_chunks(const DeltaArgs& a, float* scratch, int n_tokens, int n_rows, cudaStream_t stream) {
+static int launch_chunks(const DeltaArgs& a, float* scratch, int slots, int n_tokens, int n_rows,
+                         cudaStream_t stream) {
     if constexpr (CHUNKS) {
-        const int slots = n_tokens / sllm::TC + n_rows + 1;
-        if (slots > 65535) return (int)cudaErrorInvalidValue;
         const chunks::Scratch z = chunks::scratch_at(scratch, (int64_t)slots * a.H, D, a.V);
         chunks::PrepArgs p = {};
         p.x = a.act; p.ld = a.ld_act; p.k0 = a.G * D; p.v0 = 2 * a.G * D; p.per = a.H / a.G;
@@ -718,23 +717,23 @@ static int launch_chunks(const DeltaArgs& a, float* scratch, int n_tokens, int n
         p.min_chunked = a.min_chunked; p.H = a.H; p.V = a.V;
         p.vec4 = a.ld_act % 4 == 0 && ((uintptr_t)a.act & 15) == 0 &&
                  (!CHANNEL || (a.ld_decay % 4 == 0 && ((uintptr_t)a.log_decay & 15) == 0));
-        return chunks::launch<D, T, CHANNEL>(p, z, a.state, a.row_slot, a.out, slots, stream);
+        return chunks::launch<D, T, CHANNEL>(p, z, a.state, a.row_slot, a.out, n_tokens, slots, stream);
     }
     return (int)cudaErrorInvalidValue;
 }
 
 // dtype: 0 = float32, 1 = bfloat16 (of act).  n_rows rows of the packed batch (row_start has
 // n_rows + 1 entries); state slots are indexed by row_slot.  max_new: the most tokens any row
-// brings (1 selects the kernel for decode steps).  chunk_scratch (or null): room for (n_tokens / 64 + n_rows
-// + 1) x H x sllm_delta_rule_chunk_floats floats on a 16-byte boundary; rows of at least min_chunked tokens
-// then run in chunks.  shortest: no row brings fewer tokens (rows without tokens apart).
+// brings (1 selects the kernel for decode steps).  chunk_scratch (or null): room for chunk_slots x H x
+// sllm_delta_rule_chunk_floats floats on a 16-byte boundary; rows of at least min_chunked tokens then run in
+// chunks, so many at a time.  shortest: no row brings fewer tokens (rows without tokens apart).
 SLLM_EXPORT int sllm_delta_rule(const void* act, int64_t ld_act, const float* ab, int64_t ld_ab,
                                 const float* A_log, const float* dt_bias, float* state,
                                 const int* row_start, const int* row_slot, float* out, int n_rows,
                                 int max_new, int H, int G, int V, const float* log_decay,
                                 int64_t ld_decay, int b_col, float* tables, int longest,
-                                float* chunk_scratch, int n_tokens, int min_chunked, int shortest,
-                                int dtype, cudaStream_t stream) {
+                                float* chunk_scratch, int chunk_slots, int n_tokens, int min_chunked,
+                                int shortest, int dtype, cudaStream_t stream) {
     if (n_rows <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G != 0 || V <= 0 || n_rows > 65535 || H > 65535 ||
         ld_act < 2 * (int64_t)G * D + (int64_t)H * V || b_col < 0 || ld_ab < b_col + H ||
@@ -769,13 +768,14 @@ SLLM_EXPORT int sllm_delta_rule(const void* act, int64_t ld_act, const float* ab
                         ((int64_t)G * D) % vec == 0;
     if (dtype != 0 && dtype != 1) return (int)cudaErrorInvalidValue;
     if (chunk_scratch) {
-        if (min_chunked < 2 || n_tokens < 0 || ((uintptr_t)chunk_scratch & 15) || ((uintptr_t)state & 15))
+        if (min_chunked < 2 || n_tokens < 0 || chunk_slots < 1 || chunk_slots > 65535 ||
+            ((uintptr_t)chunk_scratch & 15) || ((uintptr_t)state & 15))
             return (int)cudaErrorInvalidValue;
         const int code = log_decay
-            ? (dtype == 0 ? launch_chunks<float, true>(a, chunk_scratch, n_tokens, n_rows, stream)
-                          : launch_chunks<__nv_bfloat16, true>(a, chunk_scratch, n_tokens, n_rows, stream))
-            : (dtype == 0 ? launch_chunks<float, false>(a, chunk_scratch, n_tokens, n_rows, stream)
-                          : launch_chunks<__nv_bfloat16, false>(a, chunk_scratch, n_tokens, n_rows, stream));
+            ? (dtype == 0 ? launch_chunks<float, true>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, stream)
+                          : launch_chunks<__nv_bfloat16, true>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, stream))
+            : (dtype == 0 ? launch_chunks<float, false>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, stream)
+                          : launch_chunks<__nv_bfloat16, false>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, stream));
         if (code || shortest >= min_chunked) return code;
     }
     if (log_decay) {

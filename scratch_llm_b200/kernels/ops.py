@@ -1591,20 +1591,29 @@ def moe_combine(y: torch.Tensor, x: torch.Tensor, shared: torch.Tensor | None, i
 DELTA_MIN_CHUNKED = 128
 
 
+#: the most scratch the chunk kernels take: more chunks than it holds are worked on in groups.  A chunk takes
+#: 213 KB per head of 128 x 128 (99 KB at 64 x 64): 113 MB for 2,048 tokens in one row and 16 heads.
+#: (8 rows of 1,024 tokens, 32 heads, one decay per head / per channel: 1,173 / 1,776 us in one group of 936 MB,
+#: 1,256 / 1,861 with this limit, 1,326 / 1,994 with half of it.)
+DELTA_SCRATCH_BYTES = 512 << 20
+
+
 def _delta_chunks(lib, n: int, n_rows: int, n_heads: int, value_dim: int, longest: int,
-                  min_chunked: int | None, state: torch.Tensor) -> tuple[torch.Tensor | None, int]:
-    """(scratch of the delta rule's chunk kernels or None, from how many tokens on a row takes them)."""
+                  min_chunked: int | None, state: torch.Tensor) -> tuple[torch.Tensor | None, int, int]:
+    """(scratch of the delta rule's chunk kernels or None, the chunks it holds, from how many tokens
+    on a row takes them)."""
     if min_chunked is None:
         min_chunked = DELTA_MIN_CHUNKED
-    slots = n // 64 + n_rows + 1
-    if not min_chunked or longest < max(2, min_chunked) or slots > 65535 or state.data_ptr() % 16:
-        return None, 0
+    if not min_chunked or min(longest, n) < max(2, min_chunked) or state.data_ptr() % 16:
+        return None, 0, 0
+    min_chunked = max(2, min_chunked)
     lib.sllm_delta_rule_chunk_floats.restype = c_int64
-    floats = lib.sllm_delta_rule_chunk_floats(c_int(value_dim))
+    floats = lib.sllm_delta_rule_chunk_floats(c_int(value_dim)) * n_heads
     if floats == 0:
-        return None, 0
-    return torch.empty(slots * n_heads * floats, dtype=torch.float32, device=state.device), \
-        max(2, min_chunked)
+        return None, 0, 0
+    chunks = n // 64 + min(n_rows, n // min_chunked)       # (a row with chunks has at most one that is not full)
+    slots = min(chunks, max(1, DELTA_SCRATCH_BYTES // (4 * floats)), 65535)
+    return torch.empty(slots * floats, dtype=torch.float32, device=state.device), slots, min_chunked
 
 
 def delta_rule(act: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
@@ -1647,14 +1656,14 @@ def delta_rule(act: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias
     if not 1 <= key_dim <= DELTA_MAX_KEY_DIM:
         raise KernelError(f"delta_rule takes key sizes up to {DELTA_MAX_KEY_DIM}, got {key_dim}")
     lib = _load(*delta_rule_library(key_dim))
-    scratch, min_chunked = _delta_chunks(lib, n, n_rows, n_heads, value_dim,
+    scratch, slots, min_chunked = _delta_chunks(lib, n, n_rows, n_heads, value_dim,
                                          0 if max_new == 1 else longest, min_chunked, state)
     _check(lib.sllm_delta_rule(
         _ptr(act), c_int64(act.stride(0)), _ptr(ab), c_int64(ab.stride(0)), _ptr(a_log),
         _ptr(dt_bias), _ptr(state), _ptr(row_start), _ptr(row_slot), _ptr(out), c_int(n_rows),
         c_int(max_new), c_int(n_heads), c_int(n_kv_heads), c_int(value_dim), c_void_p(0),
-        c_int64(0), c_int(n_heads), c_void_p(0), c_int(0), _ptr(scratch), c_int(n),
-        c_int(min_chunked), c_int(shortest), c_int(_code(act.dtype)), _stream()),
+        c_int64(0), c_int(n_heads), c_void_p(0), c_int(0), _ptr(scratch),
+        c_int(slots), c_int(n), c_int(min_chunked), c_int(shortest), c_int(_code(act.dtype)), _stream()),
         "delta_rule")
     return out
 
@@ -1687,19 +1696,18 @@ def _delta_rule_channels(act, ab, state, row_start, row_slot, out, n_rows, n_hea
         raise KernelError(f"delta_rule with a decay per channel takes key sizes up to "
                           f"{DELTA_CHANNEL_MAX_KEY_DIM}, got {key_dim}")
     lib = _load(*delta_rule_library(key_dim))
-    scratch, min_chunked = _delta_chunks(lib, n, n_rows, n_heads, value_dim,
+    scratch, slots, min_chunked = _delta_chunks(lib, n, n_rows, n_heads, value_dim,
                                          0 if max_new == 1 else longest, min_chunked, state)
     tables = None
     if longest > 1 and max_new != 1 and (scratch is None or shortest < min_chunked):
-        slots = n // DELTA_CHUNK + n_rows + 1
-        tables = torch.empty((slots, n_heads, 2 * DELTA_CHUNK, DELTA_CHUNK), dtype=torch.float32,
+        tables = torch.empty((n // DELTA_CHUNK + n_rows + 1, n_heads, 2 * DELTA_CHUNK, DELTA_CHUNK), dtype=torch.float32,
                              device=act.device)
     _check(lib.sllm_delta_rule(
         _ptr(act), c_int64(act.stride(0)), _ptr(ab), c_int64(ab.stride(0)), c_void_p(0),
         c_void_p(0), _ptr(state), _ptr(row_start), _ptr(row_slot), _ptr(out), c_int(n_rows),
         c_int(max_new), c_int(n_heads), c_int(n_kv_heads), c_int(value_dim), _ptr(log_decay),
         c_int64(log_decay.stride(0)), c_int(b_col), _ptr(tables), c_int(longest), _ptr(scratch),
-        c_int(n), c_int(min_chunked), c_int(shortest), c_int(_code(act.dtype)), _stream()),
+        c_int(slots), c_int(n), c_int(min_chunked), c_int(shortest), c_int(_code(act.dtype)), _stream()),
         "delta_rule")
     return out
 

@@ -113,3 +113,63 @@ def test_chunks_are_as_exact_as_the_order_of_tokens(dtype, channels, decay, D, V
     # both are walks of as many roundings in another order: 0.6 to 1.35 measured (4 with sums cut off by mma.sync)
     for what, chunked, in_order in zip(("read-outs", "state"), *errors):
         assert chunked < 1.5 * in_order, f"{what}: {chunked:.2e}, in order {in_order:.2e}"
+
+
+def rows_case(lengths, H, G, D, V, channels, dtype=torch.bfloat16):
+    """A function that runs the given rows of a step (all of them, or some alone); their outputs and states."""
+    n, g = sum(lengths), torch.Generator(device=DEV).manual_seed(sum(lengths))
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    act, ab, start = r(n, 2 * G * D + H * V).to(dtype), r(n, 2 * H), r(len(lengths), H, V, D)
+    A_log, dt_bias, log_decay = r(H), r(H), -torch.exp(r(n, H * D) - 2)
+    first = [sum(lengths[:i]) for i in range(len(lengths))]
+
+    def run(rows, **more):
+        tokens = torch.cat([torch.arange(first[i], first[i] + lengths[i], device=DEV) for i in rows])
+        some = [lengths[i] for i in rows]
+        S, out = start.clone(), torch.full((sum(some), H * V), float("nan"), device=DEV)
+        ops().delta_rule(act[tokens], ab[tokens], None if channels else A_log, None if channels else dt_bias, S,
+                         i32([sum(some[:i]) for i in range(len(some) + 1)]), i32(rows), out, len(some), H, G, D, V,
+                         max_new=1 if max(some) == 1 else 0, longest=max(some), shortest=min(some),
+                         log_decay=log_decay[tokens] if channels else None, **more)
+        return list(out.split(some)), S
+
+    return run
+
+
+@pytest.mark.parametrize("channels", [False, True])
+@pytest.mark.parametrize("D,V", [(128, 40), (64, 64)])
+@pytest.mark.parametrize("chunks", [1, 3, 7])
+def test_groups_of_chunks_and_rows_alone(monkeypatch, channels, D, V, chunks):
+    """However many chunks the scratch holds, and whatever rows are beside a row: the same bits."""
+    lengths = [129, 3, 0, 500, 1, 193, 64] + [0] * 28 + [128, 1, 300]
+    run = rows_case(lengths, 2, 1, D, V, channels)
+    rows = list(range(len(lengths)))
+    out, S = run(rows)
+    floats = (3 * 64 * D + 64 * V + 64 * 64 + V * D + D) * 2
+    monkeypatch.setattr(ops(), "DELTA_SCRATCH_BYTES", 4 * floats * chunks)
+    again, S_again = run(rows)
+    assert torch.equal(torch.cat(out), torch.cat(again)) and torch.equal(S, S_again)
+    for i in (0, 1, 3, 4, 5, 36, 37):
+        alone, S_alone = run([i])
+        assert torch.equal(out[i], alone[0]) and torch.equal(S[i], S_alone[i]), lengths[i]
+
+
+@pytest.mark.parametrize("lengths,limit", [([130] + [1] * 64, 4), ([200] * 8, 33), ([8192], 78)])
+def test_scratch_goes_with_the_chunks(lengths, limit):
+    """What a step takes beside its tensors: no more than its chunks (32 heads of 128 x 128), nor than the
+    limit that chunks are grouped to."""
+    run = rows_case(lengths, 32, 16, 128, 128, False)
+    seen, empty = [], torch.empty
+
+    def counting(*a, **k):
+        t = empty(*a, **k)
+        seen.append(t.numel() * t.element_size())
+        return t
+
+    rows = list(range(len(lengths)))
+    run(rows)
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(torch, "empty", counting)
+        run(rows)
+    chunk = 32 * 4 * (3 * 64 * 128 + 64 * 128 + 64 * 64 + 128 * 128 + 128)
+    assert sum(seen) <= limit * chunk and sum(seen) <= 512 << 20
