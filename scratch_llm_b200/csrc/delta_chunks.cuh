@@ -66,7 +66,7 @@ static inline Scratch scratch_at(float* at, int64_t n, int D, int64_t V) {
 
 // The chunks of a step are numbered over the rows that have any (at least min_chunked tokens), row after
 // row.  They are worked on in groups of as many as the scratch has slots: chunk `first` + i has slot i.
-struct Group { int first, count; };
+struct Group { int first, count; bool beside; };     // beside: see launch()
 struct RowAt { int row, t0, n_new, first; };     // first: the number of the row's first chunk
 // BY_CHUNK: the row of the group's chunk number `which`; else the row number `which` of those that have chunks
 // in the group or after it.
@@ -323,15 +323,13 @@ template <int D, typename T> constexpr size_t prep_head_smem() {
 // tokens.  52 us at 2,048 tokens and 16 heads of 128 x 128; bound by the substitution's shared-memory reads
 // (544 of 16 bytes a warp) and, with two CTAs of eight warps an SM, by latencies.
 template <int D, typename T>
-__global__ void __launch_bounds__(PREP_THREADS, 2) prep_head_kernel(const PrepArgs a, const Scratch z, const Group group) {
+__device__ __forceinline__ void prep_head(const PrepArgs& a, const Scratch& z, const Group& group) {
     constexpr int LD = HEAD_LD<D, T>;
     extern __shared__ __align__(16) float sm[];
     float* At = sm;
     T* ks = reinterpret_cast<T*>(At + TC * LDT);
     T* qs = ks + TC * LD;
     __shared__ float log_g[TC], beta[TC], loc[TC], grow[TC], bgrow[TC], rest[TC], tot[NB], unit_k[TC], unit_q[TC];
-    pdl_wait();
-    pdl_trigger();
     const int slot = blockIdx.x, head = blockIdx.y;
     RowAt row;
     if (!find_row<true>(a.row_start, a.n_rows, a.min_chunked, group, slot, row)) return;
@@ -546,7 +544,7 @@ __device__ __forceinline__ void block_pairs(const float* x, const float* y, cons
 // k e^{l}; L = the decays, then k e^{border - l} (l: sums of logarithms from the block's border on).  One
 // CTA an SM (127 KB at D = 128); 256 us at 3,001 tokens in four rows and 16 heads of 128 x 128.
 template <int D, typename T>
-__global__ void __launch_bounds__(PREP_THREADS, 1) prep_channels_kernel(const PrepArgs a, const Scratch z, const Group group) {
+__device__ __forceinline__ void prep_channels(const PrepArgs& a, const Scratch& z, const Group& group) {
     constexpr int LD = D + 4;
     extern __shared__ __align__(16) float sm[];
     float* R = sm;
@@ -558,8 +556,6 @@ __global__ void __launch_bounds__(PREP_THREADS, 1) prep_channels_kernel(const Pr
     float* post = pre + NB * D;                   // [NB][D]: e^{blocks after}
     float* mids = post + NB * D;                  // [3][D]: e^{blocks between} of (2,0), (3,1), (3,0)
     __shared__ float beta[TC];
-    pdl_wait();
-    pdl_trigger();
     const int slot = blockIdx.x, head = blockIdx.y;
     RowAt row;
     if (!find_row<true>(a.row_start, a.n_rows, a.min_chunked, group, slot, row)) return;
@@ -674,6 +670,17 @@ __global__ void __launch_bounds__(PREP_THREADS, 1) prep_channels_kernel(const Pr
         if (at_col < D + a.V)
             store_column(acc, z.W + at * TC * D, col < D ? col : -1, z.X + (at * a.V + (col - D)) * TC);
     }
+}
+
+// `beside`: the kernel runs beside its predecessor, whose results it does not use, and ends after it.
+template <int D, typename T, bool CHANNEL>
+__global__ void __launch_bounds__(PREP_THREADS, CHANNEL ? 1 : 2)
+prep_kernel(const PrepArgs a, const Scratch z, const Group group) {
+    if (!group.beside) pdl_wait();
+    pdl_trigger();
+    if constexpr (CHANNEL) prep_channels<D, T>(a, z, group);
+    else prep_head<D, T>(a, z, group);
+    if (group.beside) pdl_wait();
 }
 
 // ------------------------------------------------------------------------------------- pass
@@ -942,14 +949,18 @@ out_kernel(const Scratch z, const Group group, const int* __restrict__ row_start
 
 // --------------------------------------------------------------------------------- launches
 
+// beside: the kernel before this launch in the stream belongs to the same step (the rows without chunks), was
+// launched as an ordinary kernel, so that all before it is done once it runs, and lets its successor start.  It
+// shares only inputs with the first prep, which then runs at its side; as prep ends after it, every later kernel
+// waits for both.  Rows of 127 and 128 tokens, 4 heads of 128 x 128, one decay per head / per channel: 81 / 93 us
+// one after the other, 64 / 64 so (47 / 49 if the tokens of both were taken in order); 16 heads: 95 / 103,
+// 95 / 97 (92 / 92); 32 heads: 143 / 148, 142 / 148 (181 / 176).
 // `slots`: room of the scratch.  Launches for every chunk that a step of n_tokens tokens can have: a row with
 // chunks ends at most one short of a whole one more than its tokens fill.
 template <int D, typename T, bool CHANNEL>
 static inline int launch(const PrepArgs& a, const Scratch& z, float* state, const int* row_slot, float* out,
-                         int n_tokens, int slots, cudaStream_t stream) {
-    void (*prep)(PrepArgs, Scratch, Group);
-    if constexpr (CHANNEL) prep = prep_channels_kernel<D, T>;
-    else prep = prep_head_kernel<D, T>;
+                         int n_tokens, int slots, bool beside, cudaStream_t stream) {
+    const auto prep = prep_kernel<D, T, CHANNEL>;
     constexpr size_t smem = CHANNEL ? prep_channels_smem<D>() : prep_head_smem<D, T>();
     cudaError_t e = cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
@@ -958,7 +969,7 @@ static inline int launch(const PrepArgs& a, const Scratch& z, float* state, cons
     const int rows = std::min(a.n_rows, n_tokens / a.min_chunked), chunks = n_tokens / TC + rows;
     const int per_row = (a.min_chunked + TC - 1) / TC;
     if (rows == 0) return 0;
-    for (Group g = {0, 0}; g.first < chunks; g.first += slots) {
+    for (Group g = {0, 0, beside}; g.first < chunks; g.first += slots, g.beside = false) {
         g.count = std::min(slots, chunks - g.first);
         e = sllm_launch_pdl(prep, dim3(g.count, a.H), dim3(PREP_THREADS), smem, stream, a, z, g);
         if (e != cudaSuccess) return (int)e;

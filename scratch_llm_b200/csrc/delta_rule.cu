@@ -706,7 +706,7 @@ SLLM_EXPORT int64_t sllm_delta_rule_chunk_floats(int V) {
 }
 
 template <typename T, bool CHANNEL>
-static int launch_chunks(const DeltaArgs& a, float* scratch, int slots, int n_tokens, int n_rows,
+static int launch_chunks(const DeltaArgs& a, float* scratch, int slots, int n_tokens, int n_rows, bool beside,
                          cudaStream_t stream) {
     if constexpr (CHUNKS) {
         const chunks::Scratch z = chunks::scratch_at(scratch, (int64_t)slots * a.H, D, a.V);
@@ -717,7 +717,28 @@ static int launch_chunks(const DeltaArgs& a, float* scratch, int slots, int n_to
         p.min_chunked = a.min_chunked; p.H = a.H; p.V = a.V;
         p.vec4 = a.ld_act % 4 == 0 && ((uintptr_t)a.act & 15) == 0 &&
                  (!CHANNEL || (a.ld_decay % 4 == 0 && ((uintptr_t)a.log_decay & 15) == 0));
-        return chunks::launch<D, T, CHANNEL>(p, z, a.state, a.row_slot, a.out, n_tokens, slots, stream);
+        return chunks::launch<D, T, CHANNEL>(p, z, a.state, a.row_slot, a.out, n_tokens, slots, beside, stream);
+    }
+    return (int)cudaErrorInvalidValue;
+}
+
+// The rows without chunks.  tables (or null): room for the weights of (tokens / CT + n_rows + 1) slots of
+// H * 2 CT * CT floats; longest: the most tokens any row of the step brings.
+template <typename T, bool CHANNEL>
+static int launch_in_order(DeltaArgs& a, float* tables, int longest, int n_rows, bool vector, cudaStream_t stream) {
+    if constexpr (CHANNEL_FITS || !CHANNEL) {
+        if (CHANNEL && tables != nullptr && longest > 1) {       // all chunks' tables at once
+            const dim3 tgrid((std::min(longest, a.min_chunked - 1) + CT - 1) / CT, a.H, n_rows);
+            if (tgrid.x > 65535u * 32u) return (int)cudaErrorInvalidValue;
+            delta_weights_kernel<T><<<tgrid, TABLE_THREADS, 0, stream>>>(a, tables);
+            SLLM_LAUNCH_CHECK();
+            a.tables = tables;
+        }
+        const dim3 grid((a.V + COLS - 1) / COLS, a.H, n_rows);
+        if (vector) delta_rule_kernel<T, D % (16 / sizeof(T)) == 0, CHANNEL><<<grid, THREADS, 0, stream>>>(a);
+        else delta_rule_kernel<T, false, CHANNEL><<<grid, THREADS, 0, stream>>>(a);
+        SLLM_LAUNCH_CHECK();
+        return 0;
     }
     return (int)cudaErrorInvalidValue;
 }
@@ -760,51 +781,28 @@ SLLM_EXPORT int sllm_delta_rule(const void* act, int64_t ld_act, const float* ab
         SLLM_LAUNCH_CHECK();
         return 0;
     }
-    dim3 grid((V + COLS - 1) / COLS, H, n_rows);
     const size_t esize = dtype == 0 ? 4 : 2;
     const int vec = (int)(16 / esize);
     // 16-byte pieces need every key, query and row of `act` to start on a 16-byte boundary
     const bool vector = D % vec == 0 && ld_act % vec == 0 && ((uintptr_t)act & 15) == 0 &&
                         ((int64_t)G * D) % vec == 0;
     if (dtype != 0 && dtype != 1) return (int)cudaErrorInvalidValue;
-    if (chunk_scratch) {
-        if (min_chunked < 2 || n_tokens < 0 || chunk_slots < 1 || chunk_slots > 65535 ||
-            ((uintptr_t)chunk_scratch & 15) || ((uintptr_t)state & 15))
-            return (int)cudaErrorInvalidValue;
+    if (chunk_scratch && (min_chunked < 2 || n_tokens < 0 || chunk_slots < 1 || chunk_slots > 65535 ||
+                          ((uintptr_t)chunk_scratch & 15) || ((uintptr_t)state & 15)))
+        return (int)cudaErrorInvalidValue;
+    const bool in_order = !chunk_scratch || shortest < min_chunked;     // rows without chunks may be there
+    if (in_order) {
         const int code = log_decay
-            ? (dtype == 0 ? launch_chunks<float, true>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, stream)
-                          : launch_chunks<__nv_bfloat16, true>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, stream))
-            : (dtype == 0 ? launch_chunks<float, false>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, stream)
-                          : launch_chunks<__nv_bfloat16, false>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, stream));
-        if (code || shortest >= min_chunked) return code;
+            ? (dtype == 0 ? launch_in_order<float, true>(a, tables, longest, n_rows, vector, stream)
+                          : launch_in_order<__nv_bfloat16, true>(a, tables, longest, n_rows, vector, stream))
+            : (dtype == 0 ? launch_in_order<float, false>(a, tables, longest, n_rows, vector, stream)
+                          : launch_in_order<__nv_bfloat16, false>(a, tables, longest, n_rows, vector, stream));
+        if (code) return code;
     }
-    if (log_decay) {
-        if constexpr (CHANNEL_FITS) {
-            if (tables != nullptr && longest > 1) {
-                // all chunks' tables at once; `tables` holds (tokens / CT + n_rows + 1) slots of
-                // H * 2 CT * CT floats, `longest` is the most tokens any row brings
-                dim3 tgrid((longest + CT - 1) / CT, H, n_rows);
-                if (tgrid.x > 65535u * 32u) return (int)cudaErrorInvalidValue;
-                if (dtype == 0) delta_weights_kernel<float><<<tgrid, TABLE_THREADS, 0, stream>>>(a, tables);
-                else delta_weights_kernel<__nv_bfloat16><<<tgrid, TABLE_THREADS, 0, stream>>>(a, tables);
-                SLLM_LAUNCH_CHECK();
-                a.tables = tables;
-            }
-            if (dtype == 0) {
-                if (vector) delta_rule_kernel<float, (D % 4 == 0), true><<<grid, THREADS, 0, stream>>>(a);
-                else delta_rule_kernel<float, false, true><<<grid, THREADS, 0, stream>>>(a);
-            } else {
-                if (vector) delta_rule_kernel<__nv_bfloat16, (D % 8 == 0), true><<<grid, THREADS, 0, stream>>>(a);
-                else delta_rule_kernel<__nv_bfloat16, false, true><<<grid, THREADS, 0, stream>>>(a);
-            }
-        }
-    } else if (dtype == 0) {
-        if (vector) delta_rule_kernel<float, (D % 4 == 0), false><<<grid, THREADS, 0, stream>>>(a);
-        else delta_rule_kernel<float, false, false><<<grid, THREADS, 0, stream>>>(a);
-    } else {
-        if (vector) delta_rule_kernel<__nv_bfloat16, (D % 8 == 0), false><<<grid, THREADS, 0, stream>>>(a);
-        else delta_rule_kernel<__nv_bfloat16, false, false><<<grid, THREADS, 0, stream>>>(a);
-    }
-    SLLM_LAUNCH_CHECK();
-    return 0;
+    if (!chunk_scratch) return 0;
+    return log_decay
+        ? (dtype == 0 ? launch_chunks<float, true>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, in_order, stream)
+                      : launch_chunks<__nv_bfloat16, true>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, in_order, stream))
+        : (dtype == 0 ? launch_chunks<float, false>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, in_order, stream)
+                      : launch_chunks<__nv_bfloat16, false>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, in_order, stream));
 }
