@@ -90,93 +90,23 @@ struct DeltaArgs {
 // the kernel for a decay per channel stages a third [CT][D] table in (static) shared memory
 constexpr bool CHANNEL_FITS = D <= 192;
 
-// One token of one column by one warp: the rule as it stands.  Every warp norms the key and
-// the query itself (its lanes hold the same quads of them as of its column).  S: the lane's
-// elements of the column (already loaded), st: where they live.
-template <typename T, bool CHANNEL>
-__device__ __forceinline__ void single_token(const DeltaArgs& a, float* S, float* st, int t0,
-                                             int head, int g, int col, bool live, int lane) {
-    const T* act = reinterpret_cast<const T*>(a.act);
-    const int64_t k_col0 = (int64_t)a.G * D, v_col0 = 2 * (int64_t)a.G * D;
-    const float decay_rate = CHANNEL ? 0.f : expf(a.A_log[head]);
-    const float dt_bias = CHANNEL ? 0.f : a.dt_bias[head];
-    const float q_scale = rsqrtf((float)D);
-        float kq[4 * QPL], qq[4 * QPL];
-        float sk = 0.f, sq = 0.f;
-        const T* row = act + (int64_t)t0 * a.ld_act + (int64_t)g * D;
-#pragma unroll
-        for (int i = 0; i < QPL; ++i)
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                const int e = (i * 32 + lane) * 4 + w;
-                kq[4 * i + w] = e < D ? to_float(row[k_col0 + e]) : 0.f;
-                qq[4 * i + w] = e < D ? to_float(row[e]) : 0.f;
-                sk += kq[4 * i + w] * kq[4 * i + w];
-                sq += qq[4 * i + w] * qq[4 * i + w];
-            }
-        sk = warp_sum(sk);
-        sq = warp_sum(sq);
-        const float ik = 1.0f / sqrtf(sk + 1e-6f), iq = q_scale / sqrtf(sq + 1e-6f);
-        const float* ab = a.ab + (int64_t)t0 * a.ld_ab;
-        float decay = 1.f;
-        if (CHANNEL) {      // this lane's channels fade by their own factors
-            const float* lg = a.log_decay + (int64_t)t0 * a.ld_decay + (int64_t)head * D;
-#pragma unroll
-            for (int i = 0; i < QPL; ++i)
-#pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    const int e = (i * 32 + lane) * 4 + w;
-                    if (e < D) S[4 * i + w] *= expf(lg[e]);
-                }
-        } else {
-            const float x = ab[head] + dt_bias;
-            decay = expf(-decay_rate * (x > 20.f ? x : log1pf(expf(x))));
-        }
-        const float beta = 1.0f / (1.0f + expf(-ab[a.b_col + head]));
-        const float value = live ? to_float(act[(int64_t)t0 * a.ld_act + v_col0 +
-                                                (int64_t)head * a.V + col]) : 0.f;
-        float p = 0.f, rq = 0.f, kdq = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4 * QPL; ++i) {
-            kq[i] *= ik;
-            qq[i] *= iq;
-            if (!CHANNEL) S[i] *= decay;
-            p = fmaf(S[i], kq[i], p);
-            rq = fmaf(S[i], qq[i], rq);
-            kdq = fmaf(kq[i], qq[i], kdq);
-        }
-        p = warp_sum(p);
-        rq = warp_sum(rq);
-        kdq = warp_sum(kdq);
-        const float u1 = beta * (value - p);
-        if (live) {
-            if (lane == 0)
-                a.out[(int64_t)t0 * a.H * a.V + (int64_t)head * a.V + col] = rq + u1 * kdq;
-#pragma unroll
-            for (int i = 0; i < QPL; ++i)
-#pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    const int e = (i * 32 + lane) * 4 + w;
-                    if (e < D) st[e] = fmaf(kq[4 * i + w], u1, S[4 * i + w]);
-                }
-        }
-}
-
-// Steps in which every row brings one token (decoding).  A warp has CPW columns, all of them requested at
-// once: unit vectors, gates and decays are formed once for the CPW, and the lanes' partial products of
-// all columns are summed together, each round halving what a lane still carries (16 shuffles for 8
-// columns' two sums instead of 80).  48 rows x 32 heads of 128 x 128 (200 MB of states read and written):
-// 89 us with a column a warp, bound by its instructions; 27 us now, states partly in L2 (memory alone: 31).
+// Rows of one token (decoding).  A warp has CPW columns, all of them requested at once: unit vectors, gates
+// and decays are formed once for the CPW, and the lanes' partial products of all columns are summed together,
+// each round halving what a lane still carries (16 shuffles for 8 columns' two sums instead of 80).  48 rows x
+// 32 heads of 128 x 128 (200 MB of states read and written): 89 us with a column a warp, bound by its
+// instructions; 27 us now, states partly in L2 (memory alone: 31).
+// `beside`: the kernel before it in the stream (other rows of the same step) shares only inputs with it; it
+// runs at that kernel's side and ends after it (see launch() in delta_chunks.cuh).  64 such rows beside one of
+// 130 tokens, 16 heads, one decay per head / per channel: 175 / 191 us when the kernel for several tokens
+// took them a warp per column, 71 / 87 so (149 / 152 before rows of 130 tokens ran in chunks).
 constexpr int CPW = QPL == 1 ? 8 : 4;
 constexpr int STEP_WARPS = 4, STEP_COLS = STEP_WARPS * CPW;
 template <typename T, bool CHANNEL>
-__global__ void __launch_bounds__(32 * STEP_WARPS) delta_rule_step_kernel(const DeltaArgs a) {
+__device__ __forceinline__ void step(const DeltaArgs& a) {
     constexpr int LANES = 32 / CPW;       // lanes that end with a column's sums
-    pdl_wait();
-    pdl_trigger();
     const int r = blockIdx.z, head = blockIdx.y;
-    const int t0 = a.row_start[r], n_new = a.row_start[r + 1] - t0;
-    if (n_new <= 0) return;
+    const int t0 = a.row_start[r];
+    if (a.row_start[r + 1] - t0 != 1) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int col0 = blockIdx.x * STEP_COLS + warp * CPW;
     if (col0 >= a.V) return;
@@ -293,6 +223,14 @@ __global__ void __launch_bounds__(32 * STEP_WARPS) delta_rule_step_kernel(const 
     }
 }
 
+template <typename T, bool CHANNEL>
+__global__ void __launch_bounds__(32 * STEP_WARPS) delta_rule_step_kernel(const DeltaArgs a, bool beside) {
+    if (!beside) pdl_wait();
+    pdl_trigger();
+    step<T, CHANNEL>(a);
+    if (beside) pdl_wait();
+}
+
 // VECTOR: keys and queries are fetched in 16-byte pieces (D a multiple of 16 / sizeof(T), rows
 // and base 16-byte aligned); else element by element.
 template <typename T, bool VECTOR, bool CHANNEL>
@@ -320,7 +258,7 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
     pdl_trigger();
     const int r = blockIdx.z, head = blockIdx.y;
     const int t0 = a.row_start[r], n_new = a.row_start[r + 1] - t0;
-    if (n_new <= 0 || n_new >= a.min_chunked) return;
+    if (n_new <= 1 || n_new >= a.min_chunked) return;     // (one token: the step kernel)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = head / (a.H / a.G);
     const int col0 = blockIdx.x * COLS;
@@ -342,10 +280,6 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const DeltaArgs a) 
     const float dt_bias = CHANNEL ? 0.f : a.dt_bias[head];
     const float q_scale = rsqrtf((float)D);
 
-    if (n_new == 1) {   // decoding: no shared memory, no barrier
-        single_token<T, CHANNEL>(a, S, st, t0, head, g, col, live, lane);
-        return;
-    }
     // columns beyond D (where D is no multiple of 4) stay zero for good
     for (int idx = tid; idx < CT * LDK; idx += THREADS) {
         (&ks[0][0])[idx] = 0.f;
@@ -625,7 +559,7 @@ __global__ void __launch_bounds__(TABLE_THREADS) delta_weights_kernel(const Delt
     pdl_trigger();
     const int r = blockIdx.z, head = blockIdx.y, c0 = blockIdx.x * CT;
     const int t0 = a.row_start[r], n_new = a.row_start[r + 1] - t0;
-    if (c0 >= n_new || n_new <= 1 || n_new >= a.min_chunked) return;     // (rows of one token take the kernel's plain path)
+    if (c0 >= n_new || n_new <= 1 || n_new >= a.min_chunked) return;     // (rows of one token need no table)
     const int nt = min(CT, n_new - c0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = head / (a.H / a.G);
@@ -743,23 +677,37 @@ static int launch_in_order(DeltaArgs& a, float* tables, int longest, int n_rows,
     return (int)cudaErrorInvalidValue;
 }
 
+template <typename T, bool CHANNEL>
+static int launch_step(const DeltaArgs& a, int n_rows, bool beside, cudaStream_t stream) {
+    if constexpr (CHANNEL_FITS || !CHANNEL) {
+        const dim3 grid((a.V + STEP_COLS - 1) / STEP_COLS, a.H, n_rows);
+        if (beside)
+            return (int)sllm_launch_pdl(delta_rule_step_kernel<T, CHANNEL>, grid, dim3(32 * STEP_WARPS), 0, stream, a, true);
+        delta_rule_step_kernel<T, CHANNEL><<<grid, 32 * STEP_WARPS, 0, stream>>>(a, false);
+        SLLM_LAUNCH_CHECK();
+        return 0;
+    }
+    return (int)cudaErrorInvalidValue;
+}
+
 // dtype: 0 = float32, 1 = bfloat16 (of act).  n_rows rows of the packed batch (row_start has
 // n_rows + 1 entries); state slots are indexed by row_slot.  max_new: the most tokens any row
 // brings (1 selects the kernel for decode steps).  chunk_scratch (or null): room for chunk_slots x H x
 // sllm_delta_rule_chunk_floats floats on a 16-byte boundary; rows of at least min_chunked tokens then run in
-// chunks, so many at a time.  shortest: no row brings fewer tokens (rows without tokens apart).
+// chunks, so many at a time.  shortest: no row brings fewer tokens (rows without tokens apart);
+// shortest_multi: no row of several tokens brings fewer.
 SLLM_EXPORT int sllm_delta_rule(const void* act, int64_t ld_act, const float* ab, int64_t ld_ab,
                                 const float* A_log, const float* dt_bias, float* state,
                                 const int* row_start, const int* row_slot, float* out, int n_rows,
                                 int max_new, int H, int G, int V, const float* log_decay,
                                 int64_t ld_decay, int b_col, float* tables, int longest,
                                 float* chunk_scratch, int chunk_slots, int n_tokens, int min_chunked,
-                                int shortest, int dtype, cudaStream_t stream) {
+                                int shortest, int shortest_multi, int dtype, cudaStream_t stream) {
     if (n_rows <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G != 0 || V <= 0 || n_rows > 65535 || H > 65535 ||
         ld_act < 2 * (int64_t)G * D + (int64_t)H * V || b_col < 0 || ld_ab < b_col + H ||
         (!log_decay && (ld_ab < H || !A_log || !dt_bias)) ||
-        (log_decay && (ld_decay < (int64_t)H * D || !CHANNEL_FITS)))
+        (log_decay && (ld_decay < (int64_t)H * D || !CHANNEL_FITS)) || (dtype != 0 && dtype != 1))
         return (int)cudaErrorInvalidValue;
     DeltaArgs a;
     a.log_decay = log_decay; a.ld_decay = ld_decay; a.b_col = b_col;
@@ -768,41 +716,36 @@ SLLM_EXPORT int sllm_delta_rule(const void* act, int64_t ld_act, const float* ab
     a.act = act; a.ld_act = ld_act; a.ab = ab; a.ld_ab = ld_ab; a.A_log = A_log;
     a.dt_bias = dt_bias; a.state = state; a.row_start = row_start; a.row_slot = row_slot;
     a.out = out; a.H = H; a.G = G; a.V = V;
-    if (max_new == 1) {   // no row brings more than one token
-        dim3 sgrid((V + STEP_COLS - 1) / STEP_COLS, H, n_rows);
-        if (dtype != 0 && dtype != 1) return (int)cudaErrorInvalidValue;
-        if (log_decay) {
-            if (dtype == 0) delta_rule_step_kernel<float, true><<<sgrid, 32 * STEP_WARPS, 0, stream>>>(a);
-            else delta_rule_step_kernel<__nv_bfloat16, true><<<sgrid, 32 * STEP_WARPS, 0, stream>>>(a);
-        } else {
-            if (dtype == 0) delta_rule_step_kernel<float, false><<<sgrid, 32 * STEP_WARPS, 0, stream>>>(a);
-            else delta_rule_step_kernel<__nv_bfloat16, false><<<sgrid, 32 * STEP_WARPS, 0, stream>>>(a);
-        }
-        SLLM_LAUNCH_CHECK();
-        return 0;
-    }
     const size_t esize = dtype == 0 ? 4 : 2;
     const int vec = (int)(16 / esize);
     // 16-byte pieces need every key, query and row of `act` to start on a 16-byte boundary
     const bool vector = D % vec == 0 && ld_act % vec == 0 && ((uintptr_t)act & 15) == 0 &&
                         ((int64_t)G * D) % vec == 0;
-    if (dtype != 0 && dtype != 1) return (int)cudaErrorInvalidValue;
     if (chunk_scratch && (min_chunked < 2 || n_tokens < 0 || chunk_slots < 1 || chunk_slots > 65535 ||
                           ((uintptr_t)chunk_scratch & 15) || ((uintptr_t)state & 15)))
         return (int)cudaErrorInvalidValue;
-    const bool in_order = !chunk_scratch || shortest < min_chunked;     // rows without chunks may be there
-    if (in_order) {
-        const int code = log_decay
+    // The rows by their tokens: several, fewer than min_chunked: in order; one: the step kernel; the others in
+    // chunks.  Each launch runs beside the one before it (the weights' tables apart).
+    const bool in_order = max_new != 1 && (!chunk_scratch || shortest_multi < min_chunked);
+    const bool single = max_new == 1 || shortest <= 1;
+    int code = 0;
+    if (in_order)
+        code = log_decay
             ? (dtype == 0 ? launch_in_order<float, true>(a, tables, longest, n_rows, vector, stream)
                           : launch_in_order<__nv_bfloat16, true>(a, tables, longest, n_rows, vector, stream))
             : (dtype == 0 ? launch_in_order<float, false>(a, tables, longest, n_rows, vector, stream)
                           : launch_in_order<__nv_bfloat16, false>(a, tables, longest, n_rows, vector, stream));
-        if (code) return code;
-    }
-    if (!chunk_scratch) return 0;
+    if (!code && single)
+        code = log_decay
+            ? (dtype == 0 ? launch_step<float, true>(a, n_rows, in_order, stream)
+                          : launch_step<__nv_bfloat16, true>(a, n_rows, in_order, stream))
+            : (dtype == 0 ? launch_step<float, false>(a, n_rows, in_order, stream)
+                          : launch_step<__nv_bfloat16, false>(a, n_rows, in_order, stream));
+    if (code || !chunk_scratch || max_new == 1) return code;
+    const bool beside = in_order || single;
     return log_decay
-        ? (dtype == 0 ? launch_chunks<float, true>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, in_order, stream)
-                      : launch_chunks<__nv_bfloat16, true>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, in_order, stream))
-        : (dtype == 0 ? launch_chunks<float, false>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, in_order, stream)
-                      : launch_chunks<__nv_bfloat16, false>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, in_order, stream));
+        ? (dtype == 0 ? launch_chunks<float, true>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, beside, stream)
+                      : launch_chunks<__nv_bfloat16, true>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, beside, stream))
+        : (dtype == 0 ? launch_chunks<float, false>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, beside, stream)
+                      : launch_chunks<__nv_bfloat16, false>(a, chunk_scratch, chunk_slots, n_tokens, n_rows, beside, stream));
 }

@@ -1621,7 +1621,7 @@ def delta_rule(act: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias
                out: torch.Tensor, n_rows: int, n_heads: int, n_kv_heads: int, key_dim: int,
                value_dim: int, max_new: int = 0, log_decay: torch.Tensor | None = None,
                b_col: int | None = None, longest: int = 0, shortest: int = 1,
-               min_chunked: int | None = None) -> torch.Tensor:
+               min_chunked: int | None = None, shortest_multi: int = 2) -> torch.Tensor:
     """The gated delta rule over the packed batch (csrc/delta_rule.cu): ``act`` [N, 2 G D + H V]
     holds query heads, key heads and value heads after the convolution; ``ab`` float32
     [N, 2 H] the decay and step inputs; ``state`` float32 [slots, H, V, D] is read and written
@@ -1632,14 +1632,18 @@ def delta_rule(act: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias
     logarithm; ``a_log`` and ``dt_bias`` are then not read (may be None), and head h's step input
     is column ``b_col + h`` of ``ab`` (any width).  ``longest``: the most tokens any row brings,
     if known and above 1: the chunks' tables of weights are then all formed at once by a kernel
-    of their own before the scan (0: every CTA of the scan forms its own)."""
+    of their own before the scan (0: every CTA of the scan forms its own).
+
+    ``longest`` also says whether rows may run in chunks (``min_chunked``: from how many tokens on; 0:
+    none).  ``shortest`` / ``shortest_multi``: no row with tokens / with several tokens brings fewer; the
+    kernels of rows that cannot be there are not launched."""
     _need(act, None, "act", contiguous=False)
     _need(ab, torch.float32, "ab", contiguous=False)
     if log_decay is not None:
         return _delta_rule_channels(act, ab, state, row_start, row_slot, out, n_rows, n_heads,
                                     n_kv_heads, key_dim, value_dim, max_new, log_decay,
                                     n_heads if b_col is None else b_col, longest, shortest,
-                                    min_chunked)
+                                    min_chunked, shortest_multi)
     _need(a_log, torch.float32, "A_log")
     _need(dt_bias, torch.float32, "dt_bias")
     _need(state, torch.float32, "state")
@@ -1663,7 +1667,8 @@ def delta_rule(act: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias
         _ptr(dt_bias), _ptr(state), _ptr(row_start), _ptr(row_slot), _ptr(out), c_int(n_rows),
         c_int(max_new), c_int(n_heads), c_int(n_kv_heads), c_int(value_dim), c_void_p(0),
         c_int64(0), c_int(n_heads), c_void_p(0), c_int(0), _ptr(scratch),
-        c_int(slots), c_int(n), c_int(min_chunked), c_int(shortest), c_int(_code(act.dtype)), _stream()),
+        c_int(slots), c_int(n), c_int(min_chunked), c_int(shortest),
+        c_int(max(shortest, shortest_multi)), c_int(_code(act.dtype)), _stream()),
         "delta_rule")
     return out
 
@@ -1678,7 +1683,7 @@ DELTA_CHUNK = 16
 
 def _delta_rule_channels(act, ab, state, row_start, row_slot, out, n_rows, n_heads, n_kv_heads,
                          key_dim, value_dim, max_new, log_decay, b_col, longest, shortest,
-                         min_chunked) -> torch.Tensor:
+                         min_chunked, shortest_multi) -> torch.Tensor:
     _need(log_decay, torch.float32, "log_decay", contiguous=False)
     _need(state, torch.float32, "state")
     _need(row_start, torch.int32, "row_start")
@@ -1699,7 +1704,7 @@ def _delta_rule_channels(act, ab, state, row_start, row_slot, out, n_rows, n_hea
     scratch, slots, min_chunked = _delta_chunks(lib, n, n_rows, n_heads, value_dim,
                                          0 if max_new == 1 else longest, min_chunked, state)
     tables = None
-    if longest > 1 and max_new != 1 and (scratch is None or shortest < min_chunked):
+    if longest > 1 and max_new != 1 and (scratch is None or max(shortest, shortest_multi) < min_chunked):
         tables = torch.empty((n // DELTA_CHUNK + n_rows + 1, n_heads, 2 * DELTA_CHUNK, DELTA_CHUNK), dtype=torch.float32,
                              device=act.device)
     _check(lib.sllm_delta_rule(
@@ -1707,7 +1712,8 @@ def _delta_rule_channels(act, ab, state, row_start, row_slot, out, n_rows, n_hea
         c_void_p(0), _ptr(state), _ptr(row_start), _ptr(row_slot), _ptr(out), c_int(n_rows),
         c_int(max_new), c_int(n_heads), c_int(n_kv_heads), c_int(value_dim), _ptr(log_decay),
         c_int64(log_decay.stride(0)), c_int(b_col), _ptr(tables), c_int(longest), _ptr(scratch),
-        c_int(slots), c_int(n), c_int(min_chunked), c_int(shortest), c_int(_code(act.dtype)), _stream()),
+        c_int(slots), c_int(n), c_int(min_chunked), c_int(shortest),
+        c_int(max(shortest, shortest_multi)), c_int(_code(act.dtype)), _stream()),
         "delta_rule")
     return out
 

@@ -166,7 +166,7 @@ class GatedDeltaRule(Mixer):
         if self.decay_rank is None:
             ops.delta_rule(act, ab, self.a_log, self.dt_bias, S, batch.row_start, batch.row_slot,
                            o, batch.n_rows, H, G, D, V, max_new=max_new, longest=batch.max_new,
-                           shortest=batch.min_new)
+                           shortest=batch.min_new, shortest_multi=batch.min_new_multi)
             b_end = 2 * H
         else:
             # the logarithms of the channels' decays, 32-bit from the first product's output on
@@ -181,7 +181,7 @@ class GatedDeltaRule(Mixer):
             ops.delta_rule(act, ab, None, None, S, batch.row_start, batch.row_slot, o,
                            batch.n_rows, H, G, D, V, max_new=max_new, log_decay=log_decay,
                            b_col=self.decay_rank, longest=batch.max_new,
-                           shortest=batch.min_new)
+                           shortest=batch.min_new, shortest_multi=batch.min_new_multi)
             b_end = self.decay_rank + H
         if self.gate_rank is None:
             gate = proj[:, C:C + H * V]
