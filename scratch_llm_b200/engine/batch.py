@@ -40,6 +40,14 @@ class PadPlan:
     n_multi: int
     n_out: int
 
+    @property
+    def max_row(self) -> int:
+        """The most tokens a row of such a step can bring: the other rows, of which there are more than
+        :func:`pad_plan` rounds away, bring one each, or two."""
+        if self.n_multi == 0:
+            return 1
+        return self.n_tokens - max(0, self.n_single - 7) - 2 * (self.n_multi // 2)
+
 
 #: steps of up to this many tokens are padded and replayed as graphs; larger ones keep the
 #: device busy for longer than the host needs to launch them
@@ -110,6 +118,9 @@ class StepBatch:
     n_single: int = 0
     n_multi: int = 0
     max_new_multi: int = 0
+    #: the most tokens a row brings, or an upper bound that a padded step's sizes allow (above 1 only
+    #: where rows of several tokens may be there)
+    max_row: int = 0
     min_new: int = 1          # the fewest tokens a row brings (a lower bound)
     min_new_multi: int = 2    # the fewest a row of several brings (a lower bound)
     max_context_single: int = 0
@@ -299,7 +310,7 @@ def build_batch(cache, stager: BatchStager, rows: Sequence[RowInput], vocab_size
         row_pos0=dev[4], row_slot=dev[5], logit_index=dev[6], single_rows=dev[7],
         multi_rows=dev[8], block_tables=dev[9:], n_single=len(single), n_multi=len(multi),
         max_new_multi=max((lens[i] for i in multi), default=0), min_new=min(lens),
-        min_new_multi=min((lens[i] for i in multi), default=2),
+        max_row=max(lens), min_new_multi=min((lens[i] for i in multi), default=2),
         max_context_single=ctx_single, context_bucket=context_bucket(ctx_single),
         wants_every_token=bool(li.size == n_tokens and (li == np.arange(n_tokens)).all()),
         host_row_new=lens, host_row_pos0=row_pos0.tolist(), n_real_tokens=n_tokens,
@@ -337,7 +348,8 @@ def _padded_batch(stager: BatchStager, plan: PadPlan, token_ids, positions, toke
         token_ids=dev[0], positions=dev[1], token_row=dev[2], row_start=dev[3],
         row_pos0=dev[4], row_slot=dev[5], logit_index=dev[6], single_rows=dev[7],
         multi_rows=dev[8], block_tables=dev[9:], n_single=plan.n_single, n_multi=plan.n_multi,
-        max_new_multi=plan.n_tokens if plan.n_multi else 0, min_new=1 if plan.n_single else 2,
+        max_new_multi=plan.n_tokens if plan.n_multi else 0, max_row=plan.max_row,
+        min_new=1 if plan.n_single else 2,
         max_context_single=ctx_single, context_bucket=context_bucket(ctx_single),
         host_row_new=list(lens) + [0] * (rows_padded - n_rows),
         host_row_pos0=row_pos0.tolist() + [0] * (rows_padded - n_rows),

@@ -165,7 +165,7 @@ class GatedDeltaRule(Mixer):
         max_new = 1 if batch.n_multi == 0 else 0
         if self.decay_rank is None:
             ops.delta_rule(act, ab, self.a_log, self.dt_bias, S, batch.row_start, batch.row_slot,
-                           o, batch.n_rows, H, G, D, V, max_new=max_new, longest=batch.max_new,
+                           o, batch.n_rows, H, G, D, V, max_new=max_new, longest=batch.max_row,
                            shortest=batch.min_new, shortest_multi=batch.min_new_multi)
             b_end = 2 * H
         else:
@@ -180,7 +180,7 @@ class GatedDeltaRule(Mixer):
                                also=also if self.gate_rank is not None else None)
             ops.delta_rule(act, ab, None, None, S, batch.row_start, batch.row_slot, o,
                            batch.n_rows, H, G, D, V, max_new=max_new, log_decay=log_decay,
-                           b_col=self.decay_rank, longest=batch.max_new,
+                           b_col=self.decay_rank, longest=batch.max_row,
                            shortest=batch.min_new, shortest_multi=batch.min_new_multi)
             b_end = self.decay_rank + H
         if self.gate_rank is None:

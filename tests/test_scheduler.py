@@ -321,6 +321,26 @@ def test_padding_plan_of_small_steps():
     assert len({t for t, _, _ in seen}) == 8 + 6   # 16..128 in steps of 16, 192..512 in steps of 64
 
 
+def test_longest_row_of_a_padded_step():
+    """The padded sizes bound the longest row: never below it, 1 where every row brings one token, and not by
+    the tokens that the other rows have to bring."""
+    from scratch_llm_b200.engine.batch import pad_plan
+    rng = random.Random(3)
+    for _ in range(3000):
+        n_single, multi = rng.randint(0, 70), [rng.randint(2, 120) for _ in range(rng.randint(0, 6))]
+        n_tokens = n_single + sum(multi)
+        if not 0 < n_tokens <= 512:
+            continue
+        plan = pad_plan(n_tokens, n_single, len(multi), rng.choice([0, 1, n_single + len(multi)]))
+        longest = max(multi, default=1)
+        assert longest <= plan.max_row <= plan.n_tokens
+        others = n_single + sum(sorted(multi)[:-1])
+        if len(multi) < 2:       # one row of several: off by the rounding of tokens and single rows only
+            assert plan.max_row < n_tokens - others + 64 + 8
+    assert pad_plan(64, 64, 0, 64).max_row == 1 and pad_plan(70, 70, 0, 0).max_row == 1
+    assert pad_plan(128, 63, 1, 64).max_row == 71
+
+
 def test_wave_policy_admits_only_into_an_empty_engine():
     """The reference's comparator: nobody joins a running wave, a wave runs until its longest
     request has ended; a wave whose prompts the token budget cuts is admitted over several
