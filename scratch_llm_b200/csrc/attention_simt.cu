@@ -26,10 +26,13 @@ constexpr int BKV = 32, THREADS = 128, WARPS = THREADS / 32;
 constexpr int DPL = (HD + 31) / 32;  // head dims per lane
 constexpr bool QUADS = HD % 4 == 0;  // rows of whole 16-byte words
 constexpr int KS_LD = QUADS ? HD + 4 : HD + 1;     // (neighbouring keys start on other banks)
+// Quads of keys and of values that a thread requests before it stores them: left to the compiler, a request
+// waited for the stores before it (777 tokens, 32 heads of 128: 347 us, 307 so; a decoded token 418, 219).
+constexpr int TRIPS = (HD + 15) / 16 <= 5 ? (HD + 15) / 16 : 4;
 constexpr bool PAIRS = HD % 64 == 0; // a lane's dims are pairs of neighbours
 // Queries of a warp: a read of a key or a value in shared memory serves all of them, and a tile of keys
 // that a CTA fetches serves WARPS times as many.  Eight for long portions, where registers and shared
-// memory hold them; one for steps of a few tokens, whose other queries would be worked on for nothing.
+// memory hold them; one for rows of a few tokens, whose other queries would be worked on for nothing.
 // 777 tokens, 32 heads of 64: 317 us with four queries a warp and a read per operand, 220 with eight.
 constexpr int LONG_QUERIES = HD <= 128 ? 8 : 4;
 
@@ -38,49 +41,49 @@ constexpr size_t smem_floats(int rpw) {
 }
 
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
-    const uint2 r = *reinterpret_cast<const uint2*>(p);
+// of the cache: read-only loads, which leave together however many stores lie between them
+__device__ __forceinline__ float4 fetch4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 fetch4(const __nv_bfloat16* p) {
+    const uint2 r = __ldg(reinterpret_cast<const uint2*>(p));
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
     return make_float4(__low2float(h[0]), __high2float(h[0]), __low2float(h[1]), __high2float(h[1]));
 }
 
-// RPW queries a warp.  vec: pages allow reads of four elements.  Every query is one chain over the dims per
-// score and over the keys per output, whatever RPW is.
+struct Args {
+    int64_t q_stride, out_stride;
+    int table_stride, page_size;
+    int H, G;
+    float scale, softcap;
+    int window, chunk, planes;
+    int vec;                             // pages allow reads of four elements
+};
+
+// Queries q0 .. q0 + nq - 1 of row r, RPW a warp.  Every query is one chain over the dims per score and over
+// the keys per output, whatever RPW is.
 template <typename T, int RPW>
-__global__ void __launch_bounds__(THREADS)
-attn_simt_kernel(const T* __restrict__ q, int64_t q_stride, const T* __restrict__ pages,
-                 const int* __restrict__ block_table, int table_stride, int page_size,
-                 const int* __restrict__ row_start, const int* __restrict__ row_pos0,
-                 T* __restrict__ out, int64_t out_stride, int H, int G, float scale, int window,
-                 const float* __restrict__ slopes, const float* __restrict__ sinks, int planes,
-                 float softcap, int chunk, int vec) {
+__device__ __forceinline__ void
+attend(const T* __restrict__ q, const T* __restrict__ pages, const int* __restrict__ table, int pos0,
+       T* __restrict__ out, float slope, const float* __restrict__ sinks, const Args& args, float* smem,
+       long long* key_base, int h, int t0, int q0, int nq) {
     constexpr int BQ = WARPS * RPW;
-    extern __shared__ __align__(16) float smem[];
-    __shared__ long long key_base[BKV];  // element offset of each key's K row, -1 if absent
+    const int page_size = args.page_size, planes = args.planes, G = args.G, window = args.window, chunk = args.chunk;
+    const float scale = args.scale, softcap = args.softcap;
     float* Qs = smem;                    // [BQ][HD]
     float* Ks = Qs + BQ * HD;            // [BKV][KS_LD]
     float* Vs = Ks + BKV * KS_LD;        // [BKV][HD]
     float* Ss = Vs + BKV * HD;           // [WARPS][BKV][RPW]: probabilities
-
-    const int r = blockIdx.y, h = blockIdx.z;
-    const int g = h / (H / G);
-    const int t0 = row_start[r];
-    const int n_new = row_start[r + 1] - t0;
-    const int q0 = (gridDim.x - 1 - blockIdx.x) * BQ;    // the queries with the most keys first
-    if (q0 >= n_new) return;
-    const int nq = min(BQ, n_new - q0);
-    const int first_pos = row_pos0[r] + q0;
+    const int g = h / (args.H / G);
+    const int first_pos = pos0 + q0;
     const int last_pos = first_pos + nq - 1;
     int k_lo = 0;
     if (window > 0) k_lo = max(0, first_pos - window + 1) / BKV * BKV;
     if (chunk > 0) k_lo = max(k_lo, first_pos / chunk * chunk / BKV * BKV);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const float slope = slopes ? slopes[h] : 0.f;
 
     for (int idx = tid; idx < BQ * HD; idx += THREADS) {
         const int i = idx / HD, d = idx - i * HD;
-        Qs[idx] = i < nq ? to_float(q[(int64_t)(t0 + q0 + i) * q_stride + (int64_t)h * HD + d])
+        Qs[idx] = i < nq ? to_float(__ldg(q + (int64_t)(t0 + q0 + i) * args.q_stride + (int64_t)h * HD + d))
                          : 0.f;
     }
 
@@ -104,25 +107,34 @@ attn_simt_kernel(const T* __restrict__ q, int64_t q_stride, const T* __restrict_
             const int kpos = kt + tid;
             long long base = -1;
             if (kpos <= last_pos) {
-                const int page = block_table[(int64_t)r * table_stride + kpos / page_size];
+                const int page = table[kpos / page_size];
                 if (page >= 0)
                     base = (((long long)page * planes * G + g) * page_size + kpos % page_size) * HD;
             }
             key_base[tid] = base;
         }
         __syncthreads();
-        if (QUADS && vec) {
-#pragma unroll 4
-            for (int idx = tid; idx < BKV * HD / 4; idx += THREADS) {
-                const int j = idx / (HD / 4), d = (idx - j * (HD / 4)) * 4;
-                const long long base = key_base[j];
-                float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
-                if (base >= 0) {
-                    kv = load4(pages + base + d);
-                    vv = load4(pages + base + v_offset + d);
+        if (QUADS && args.vec) {
+            for (int at = tid; at < BKV * HD / 4; at += TRIPS * THREADS) {      // all requests, then all stores
+                float4 kv[TRIPS], vv[TRIPS];
+#pragma unroll
+                for (int u = 0; u < TRIPS; ++u) {
+                    const int idx = at + u * THREADS, j = idx / (HD / 4), d = (idx - j * (HD / 4)) * 4;
+                    kv[u] = vv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    const long long base = idx < BKV * HD / 4 ? key_base[j] : -1;
+                    if (base >= 0) {
+                        kv[u] = fetch4(pages + base + d);
+                        vv[u] = fetch4(pages + base + v_offset + d);
+                    }
                 }
-                *reinterpret_cast<float4*>(Ks + j * KS_LD + d) = kv;
-                *reinterpret_cast<float4*>(Vs + j * HD + d) = vv;
+#pragma unroll
+                for (int u = 0; u < TRIPS; ++u) {
+                    const int idx = at + u * THREADS, j = idx / (HD / 4), d = (idx - j * (HD / 4)) * 4;
+                    if (idx < BKV * HD / 4) {
+                        *reinterpret_cast<float4*>(Ks + j * KS_LD + d) = kv[u];
+                        *reinterpret_cast<float4*>(Vs + j * HD + d) = vv[u];
+                    }
+                }
             }
         } else {
             for (int idx = tid; idx < BKV * HD; idx += THREADS) {
@@ -130,8 +142,8 @@ attn_simt_kernel(const T* __restrict__ q, int64_t q_stride, const T* __restrict_
                 const long long base = key_base[j];
                 float kv = 0.f, vv = 0.f;
                 if (base >= 0) {
-                    kv = to_float(pages[base + d]);
-                    vv = to_float(pages[base + v_offset + d]);
+                    kv = to_float(__ldg(pages + base + d));
+                    vv = to_float(__ldg(pages + base + v_offset + d));
                 }
                 Ks[j * KS_LD + d] = kv;
                 Vs[j * HD + d] = vv;
@@ -229,7 +241,7 @@ attn_simt_kernel(const T* __restrict__ q, int64_t q_stride, const T* __restrict_
             total = total * keep + expf(sink - top);
         }
         const float inv = total > 0.f ? keep / total : 0.f;
-        T* o = out + (int64_t)(t0 + q0 + i) * out_stride + (int64_t)h * HD;
+        T* o = out + (int64_t)(t0 + q0 + i) * args.out_stride + (int64_t)h * HD;
 #pragma unroll
         for (int c = 0; c < DPL; ++c) {
             const int d = PAIRS ? 32 * (c & ~1) + 2 * lane + (c & 1) : lane + 32 * c;
@@ -238,29 +250,55 @@ attn_simt_kernel(const T* __restrict__ q, int64_t q_stride, const T* __restrict_
     }
 }
 
-template <typename T, int RPW>
-static int launch(const void* q, int64_t q_stride, const void* pages, const int* block_table, int table_stride,
-                  int page_size, const int* row_start, const int* row_pos0, void* out, int64_t out_stride,
-                  int n_rows, int max_new, int H, int G, float scale, int window, const float* slopes,
-                  const float* sinks, int planes, float softcap, int chunk, cudaStream_t stream) {
-    const size_t smem = smem_floats(RPW) * sizeof(float);
-    const cudaError_t e = cudaFuncSetAttribute(attn_simt_kernel<T, RPW>,
+// Blocks of WARPS * MOST queries; a block with fewer (a row's last, a decoded token beside a prompt or in a
+// padded step) takes as few a warp as they need.  Registers for the CTAs that an SM's shared memory holds.
+// 64 rows of one token and 2,000 keys, 32 heads of 64 / 128, in a launch for 64 new tokens: 1,714 / 4,463 us with
+// 16 queries a block, 1,934 / 3,142 with 32 that all blocks worked on, 614 / 1,213 so.
+template <typename T, int MOST>
+__global__ void __launch_bounds__(THREADS, HD <= 64 ? 5 : HD <= 128 ? 4 : 1)
+attn_simt_kernel(const T* __restrict__ q, const T* __restrict__ pages, const int* __restrict__ block_table,
+                 const int* __restrict__ row_start, const int* __restrict__ row_pos0, T* __restrict__ out,
+                 const float* __restrict__ slopes, const float* __restrict__ sinks, const Args args) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ long long key_base[BKV];  // element offset of each key's K row, -1 if absent
+    constexpr int BQ = WARPS * MOST;
+    const int r = blockIdx.y, h = blockIdx.z;
+    const int t0 = row_start[r], n_new = row_start[r + 1] - t0;
+    const int q0 = (gridDim.x - 1 - blockIdx.x) * BQ;    // the queries with the most keys first
+    if (q0 >= n_new) return;
+    const int nq = min(BQ, n_new - q0);
+    const int* table = block_table + (int64_t)r * args.table_stride;
+    const float slope = slopes ? slopes[h] : 0.f;
+    const int pos0 = row_pos0[r];
+    if (MOST > 1 && nq <= WARPS)
+        attend<T, 1>(q, pages, table, pos0, out, slope, sinks, args, smem, key_base, h, t0, q0, nq);
+    else if (MOST > 4 && nq <= 4 * WARPS)
+        attend<T, 4>(q, pages, table, pos0, out, slope, sinks, args, smem, key_base, h, t0, q0, nq);
+    else
+        attend<T, MOST>(q, pages, table, pos0, out, slope, sinks, args, smem, key_base, h, t0, q0, nq);
+}
+
+template <typename T, int MOST>
+static int launch(const void* q, const void* pages, const int* block_table, const int* row_start,
+                  const int* row_pos0, void* out, const float* slopes, const float* sinks, const Args& args,
+                  int n_rows, int max_new, cudaStream_t stream) {
+    const size_t smem = smem_floats(MOST) * sizeof(float);
+    const cudaError_t e = cudaFuncSetAttribute(attn_simt_kernel<T, MOST>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    constexpr int BQ = WARPS * RPW;
-    const int vec = ((uintptr_t)pages & 15) == 0;
-    attn_simt_kernel<T, RPW><<<dim3((max_new + BQ - 1) / BQ, n_rows, H), THREADS, smem, stream>>>(
-        (const T*)q, q_stride, (const T*)pages, block_table, table_stride, page_size, row_start, row_pos0,
-        (T*)out, out_stride, H, G, scale, window, slopes, sinks, planes, softcap, chunk, vec);
+    constexpr int BQ = WARPS * MOST;
+    attn_simt_kernel<T, MOST><<<dim3((max_new + BQ - 1) / BQ, n_rows, args.H), THREADS, smem, stream>>>(
+        (const T*)q, (const T*)pages, block_table, row_start, row_pos0, (T*)out, slopes, sinks, args);
     SLLM_LAUNCH_CHECK();
     return 0;
 }
 
-template <typename T, typename... Args>
-static int launch_for(int max_new, Args... args) {
-    if (max_new <= WARPS) return launch<T, 1>(args...);
-    if (max_new <= 4 * WARPS) return launch<T, 4>(args...);
-    return launch<T, LONG_QUERIES>(args...);
+// max_new decides the shared memory and the number of blocks; what a block computes with goes by its own queries.
+template <typename T, typename... Rest>
+static int launch_for(int max_new, Rest... rest) {
+    if (max_new <= WARPS) return launch<T, 1>(rest...);
+    if (max_new <= 4 * WARPS) return launch<T, 4>(rest...);
+    return launch<T, LONG_QUERIES>(rest...);
 }
 
 }  // namespace sllm
@@ -290,13 +328,13 @@ SLLM_EXPORT int sllm_attn_simt(const void* q, int64_t q_stride, const void* page
     if (H <= 0 || G <= 0 || H % G != 0 || page_size <= 0 || window < 0 || chunk < 0 || planes < 1 || planes > 2)
         return (int)cudaErrorInvalidValue;
     if (n_rows > 65535 || H > 65535) return (int)cudaErrorInvalidValue;
+    const Args args = {q_stride, out_stride, table_stride, page_size, H, G, scale, softcap, window, chunk, planes,
+                       ((uintptr_t)pages & 15) == 0};
     if (dtype == 0)
-        return launch_for<float>(max_new, q, q_stride, pages, block_table, table_stride, page_size, row_start,
-                                 row_pos0, out, out_stride, n_rows, max_new, H, G, scale, window, slopes, sinks,
-                                 planes, softcap, chunk, stream);
+        return launch_for<float>(max_new, q, pages, block_table, row_start, row_pos0, out, slopes, sinks, args,
+                                 n_rows, max_new, stream);
     if (dtype == 1)
-        return launch_for<__nv_bfloat16>(max_new, q, q_stride, pages, block_table, table_stride, page_size,
-                                         row_start, row_pos0, out, out_stride, n_rows, max_new, H, G, scale,
-                                         window, slopes, sinks, planes, softcap, chunk, stream);
+        return launch_for<__nv_bfloat16>(max_new, q, pages, block_table, row_start, row_pos0, out, slopes, sinks,
+                                         args, n_rows, max_new, stream);
     return (int)cudaErrorInvalidValue;
 }

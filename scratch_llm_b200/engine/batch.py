@@ -137,6 +137,9 @@ class StepBatch:
     n_real_tokens: int = 0
     n_real_out: int = 0
 
+    def __post_init__(self) -> None:
+        self.max_row = self.max_row or self.max_new
+
 
 class BatchStager:
     """Packs step descriptors on the host and copies them to the device in one transfer.

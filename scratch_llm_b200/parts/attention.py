@@ -193,7 +193,7 @@ class GQAttention(Mixer):
         else:
             ops.attention_simt(q, cache.pages, cache.block_table, cache.page_size,
                                batch.row_start, batch.row_pos0, out, batch.n_rows,
-                               batch.max_new, H, G, hd, self.scale, self.window)
+                               batch.max_row, H, G, hd, self.scale, self.window)
         return out
 
     def _n_splits(self, batch) -> int:

@@ -127,7 +127,7 @@ class BiasedAttention(Mixer):
             self._attend_tensor_cores(q, out, batch, cache, gate)   # (the gate in its epilogue)
         else:
             ops.attention_simt(q, cache.pages, cache.block_table, cache.page_size,
-                               batch.row_start, batch.row_pos0, out, batch.n_rows, batch.max_new,
+                               batch.row_start, batch.row_pos0, out, batch.n_rows, batch.max_row,
                                H, G, hd, self.scale, self.window, self.slopes, self.sinks)
             if gate is not None:
                 ops.sigmoid_gate(out, gate)

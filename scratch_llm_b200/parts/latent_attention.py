@@ -228,7 +228,7 @@ class LatentAttention(Mixer):
         common = (q, cache.pages, cache.block_table, cache.page_size, batch.row_start,
                   batch.row_pos0, out)
         if not self._tensor_cores(q.dtype):
-            ops.attention_simt(*common, batch.n_rows, batch.max_new, H, 1, Dp, self.scale, None)
+            ops.attention_simt(*common, batch.n_rows, batch.max_row, H, 1, Dp, self.scale, None)
             return
         if batch.n_multi:
             if ops.attention_tc_supports(H, 1, Dp, cache.page_size, None) \

@@ -195,7 +195,7 @@ class NormedAttention(Mixer):
                 gate = None
         else:
             ops.attention_simt(q, cache.pages, cache.block_table, cache.page_size,
-                               batch.row_start, batch.row_pos0, out, batch.n_rows, batch.max_new,
+                               batch.row_start, batch.row_pos0, out, batch.n_rows, batch.max_row,
                                H, G, hd, self.scale, self.window, None, self.sinks,
                                softcap=self.softcap, chunk=self.chunk)
         if gate is not None:
