@@ -27,13 +27,13 @@ constexpr int DPL = (HD + 31) / 32;  // head dims per lane
 constexpr bool QUADS = HD % 4 == 0;  // rows of whole 16-byte words
 constexpr int KS_LD = QUADS ? HD + 4 : HD + 1;     // (neighbouring keys start on other banks)
 // Quads of keys and of values that a thread requests before it stores them: left to the compiler, a request
-// waited for the stores before it (777 tokens, 32 heads of 128: 347 us, 307 so; a decoded token 418, 219).
+// waited for the stores before it (777 tokens, 32 heads of 128: 347 us, 316 so; a decoded token 418, 226).
 constexpr int TRIPS = (HD + 15) / 16 <= 5 ? (HD + 15) / 16 : 4;
 constexpr bool PAIRS = HD % 64 == 0; // a lane's dims are pairs of neighbours
 // Queries of a warp: a read of a key or a value in shared memory serves all of them, and a tile of keys
 // that a CTA fetches serves WARPS times as many.  Eight for long portions, where registers and shared
 // memory hold them; one for rows of a few tokens, whose other queries would be worked on for nothing.
-// 777 tokens, 32 heads of 64: 317 us with four queries a warp and a read per operand, 220 with eight.
+// 777 tokens, 32 heads of 64: 317 us with four queries a warp and a read per operand, 213 with eight.
 constexpr int LONG_QUERIES = HD <= 128 ? 8 : 4;
 
 constexpr size_t smem_floats(int rpw) {
@@ -101,6 +101,12 @@ attend(const T* __restrict__ q, const T* __restrict__ pages, const int* __restri
     const float* kj = Ks + lane * KS_LD;
     float* ps = Ss + warp * BKV * RPW;
 
+    auto sees = [&](int a, int kpos) {             // query a of this warp, the key at that position
+        const int i = warp + WARPS * a, qpos = first_pos + i;
+        return i < nq && kpos <= qpos && (window <= 0 || kpos > qpos - window) &&
+               (chunk <= 0 || kpos >= qpos / chunk * chunk);
+    };
+    auto dim = [&](int c) { return PAIRS ? 32 * (c & ~1) + 2 * lane + (c & 1) : lane + 32 * c; };   // of entry c
     for (int kt = k_lo; kt <= last_pos; kt += BKV) {
         __syncthreads();  // the previous tile's Ks / Vs / key_base are no longer read
         if (tid < BKV) {
@@ -114,6 +120,7 @@ attend(const T* __restrict__ q, const T* __restrict__ pages, const int* __restri
             key_base[tid] = base;
         }
         __syncthreads();
+        float odd = 0.f;                 // NaN if a value of the tile is an infinity or a NaN
         if (QUADS && args.vec) {
             for (int at = tid; at < BKV * HD / 4; at += TRIPS * THREADS) {      // all requests, then all stores
                 float4 kv[TRIPS], vv[TRIPS];
@@ -133,6 +140,7 @@ attend(const T* __restrict__ q, const T* __restrict__ pages, const int* __restri
                     if (idx < BKV * HD / 4) {
                         *reinterpret_cast<float4*>(Ks + j * KS_LD + d) = kv[u];
                         *reinterpret_cast<float4*>(Vs + j * HD + d) = vv[u];
+                        odd = fmaf(vv[u].x, 0.f, fmaf(vv[u].y, 0.f, fmaf(vv[u].z, 0.f, fmaf(vv[u].w, 0.f, odd))));
                     }
                 }
             }
@@ -147,9 +155,10 @@ attend(const T* __restrict__ q, const T* __restrict__ pages, const int* __restri
                 }
                 Ks[j * KS_LD + d] = kv;
                 Vs[j * HD + d] = vv;
+                odd = fmaf(vv, 0.f, odd);
             }
         }
-        __syncthreads();
+        const bool guard = __syncthreads_or(odd != 0.f);
 
         const int kpos = kt + lane;
         float dot[RPW];
@@ -176,9 +185,8 @@ attend(const T* __restrict__ q, const T* __restrict__ pages, const int* __restri
         const bool there = key_base[lane] >= 0;
 #pragma unroll
         for (int a = 0; a < RPW; ++a) {
-            const int i = warp + WARPS * a, qpos = first_pos + i;
-            const bool valid = i < nq && kpos <= qpos && (window <= 0 || kpos > qpos - window) &&
-                               (chunk <= 0 || kpos >= qpos / chunk * chunk) && there;
+            const int qpos = first_pos + warp + WARPS * a;
+            const bool valid = sees(a, kpos) && there;
             float sc = dot[a] * scale;
             if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
             const float s = valid ? sc - slope * (float)(qpos - kpos) : -INFINITY;
@@ -195,6 +203,22 @@ attend(const T* __restrict__ q, const T* __restrict__ pages, const int* __restri
             ps[lane * RPW + a] = p;
         }
         __syncwarp();  // each warp reads back only what it wrote
+        if (guard) {   // zero times such a value is not zero: a query leaves out the keys that it does not see
+#pragma unroll 1
+            for (int j = 0; j < BKV; ++j) {
+#pragma unroll
+                for (int a = 0; a < RPW; ++a) {
+                    const float p = ps[j * RPW + a];
+                    if (!sees(a, kt + j)) continue;
+#pragma unroll
+                    for (int c = 0; c < DPL; ++c) {
+                        const int d = dim(c);
+                        if (d < HD) acc[a][c] = fmaf(p, Vs[j * HD + d], acc[a][c]);
+                    }
+                }
+            }
+            continue;
+        }
 #pragma unroll 4
         for (int j = 0; j < BKV; ++j) {
             float p[RPW];
@@ -244,7 +268,7 @@ attend(const T* __restrict__ q, const T* __restrict__ pages, const int* __restri
         T* o = out + (int64_t)(t0 + q0 + i) * args.out_stride + (int64_t)h * HD;
 #pragma unroll
         for (int c = 0; c < DPL; ++c) {
-            const int d = PAIRS ? 32 * (c & ~1) + 2 * lane + (c & 1) : lane + 32 * c;
+            const int d = dim(c);
             if (d < HD) o[d] = from_float<T>(acc[a][c] * inv);
         }
     }
@@ -253,7 +277,7 @@ attend(const T* __restrict__ q, const T* __restrict__ pages, const int* __restri
 // Blocks of WARPS * MOST queries; a block with fewer (a row's last, a decoded token beside a prompt or in a
 // padded step) takes as few a warp as they need.  Registers for the CTAs that an SM's shared memory holds.
 // 64 rows of one token and 2,000 keys, 32 heads of 64 / 128, in a launch for 64 new tokens: 1,714 / 4,463 us with
-// 16 queries a block, 1,934 / 3,142 with 32 that all blocks worked on, 614 / 1,213 so.
+// 16 queries a block, 1,934 / 3,142 with 32 that all blocks worked on, 663 / 1,208 so.
 template <typename T, int MOST>
 __global__ void __launch_bounds__(THREADS, HD <= 64 ? 5 : HD <= 128 ? 4 : 1)
 attn_simt_kernel(const T* __restrict__ q, const T* __restrict__ pages, const int* __restrict__ block_table,

@@ -90,3 +90,27 @@ def test_attention_simt_rows_of_all_lengths(dtype, hd, odd, window):
         want = torch.einsum("hnk,hkd->nhd", torch.softmax(s, -1), v).reshape(new, -1)
         tol = 2e-6 if dtype == torch.float32 else 2 ** -8       # (as above)
         assert ((mine.double() - want).norm() / want.norm()).item() < tol
+
+
+@pytest.mark.parametrize("hd", [64, 48])
+@pytest.mark.parametrize("window", [0, 9])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_attention_simt_values_of_unseen_keys(hd, window, bad):
+    """A value that is no number reaches the queries that see its key, and no other."""
+    from scratch_llm_b200.kernels import ops
+    n, H, page, at = 70, 2, 16, 41
+    gen = torch.Generator().manual_seed(hd)
+    pages = torch.randn(-(-n // page), 2, 1, page, hd, generator=gen).to(DEV)
+    q = torch.randn(n, H * hd, generator=gen).to(DEV)
+    table = torch.arange(len(pages), dtype=torch.int32, device=DEV).view(1, -1)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    outs = []
+    for value in (0.5, bad):
+        pages[at // page, 1, 0, at % page] = value
+        outs.append(torch.empty_like(q))
+        ops.attention_simt(q, pages, table, page, i32([0, n]), i32([0]), outs[-1], 1, n, H, 1, hd, hd ** -0.5, window or None)
+    sees = torch.arange(n) >= at
+    if window:
+        sees &= torch.arange(n) < at + window
+    assert torch.equal(outs[0][~sees], outs[1][~sees])
+    assert not torch.isfinite(outs[1][sees]).any()
