@@ -101,7 +101,7 @@ constexpr bool CHANNEL_FITS = D <= 192;
 // took them a warp per column, 71 / 87 so (149 / 152 before rows of 130 tokens ran in chunks).
 constexpr int CPW = QPL == 1 ? 8 : 4;
 constexpr int STEP_WARPS = 4, STEP_COLS = STEP_WARPS * CPW;
-template <typename T, bool CHANNEL>
+template <typename T, bool CHANNEL, bool WORDS>
 __device__ __forceinline__ void step(const DeltaArgs& a) {
     constexpr int LANES = 32 / CPW;       // lanes that end with a column's sums
     const int r = blockIdx.z, head = blockIdx.y;
@@ -118,7 +118,7 @@ __device__ __forceinline__ void step(const DeltaArgs& a) {
 #pragma unroll
         for (int i = 0; i < QPL; ++i) {
             const int e = (i * 32 + lane) * 4;
-            if (D % 4 == 0) {
+            if (WORDS) {
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (c < n_cols && e < D) v = *reinterpret_cast<const float4*>(st + c * D + e);
                 S[c][4 * i] = v.x; S[c][4 * i + 1] = v.y; S[c][4 * i + 2] = v.z; S[c][4 * i + 3] = v.w;
@@ -211,7 +211,7 @@ __device__ __forceinline__ void step(const DeltaArgs& a) {
                 float v[4];
 #pragma unroll
                 for (int w = 0; w < 4; ++w) v[w] = fmaf(kq[4 * i + w], uc, S[c][4 * i + w]);
-                if (D % 4 == 0) {
+                if (WORDS) {
                     if (e < D) *reinterpret_cast<float4*>(st + c * D + e) = make_float4(v[0], v[1], v[2], v[3]);
                 } else {
 #pragma unroll
@@ -223,11 +223,12 @@ __device__ __forceinline__ void step(const DeltaArgs& a) {
     }
 }
 
-template <typename T, bool CHANNEL>
+// WORDS: columns are whole 16-byte words on 16-byte boundaries; else the state goes element by element.
+template <typename T, bool CHANNEL, bool WORDS>
 __global__ void __launch_bounds__(32 * STEP_WARPS) delta_rule_step_kernel(const DeltaArgs a, bool beside) {
     if (!beside) pdl_wait();
     pdl_trigger();
-    step<T, CHANNEL>(a);
+    step<T, CHANNEL, WORDS>(a);
     if (beside) pdl_wait();
 }
 
@@ -681,9 +682,10 @@ template <typename T, bool CHANNEL>
 static int launch_step(const DeltaArgs& a, int n_rows, bool beside, cudaStream_t stream) {
     if constexpr (CHANNEL_FITS || !CHANNEL) {
         const dim3 grid((a.V + STEP_COLS - 1) / STEP_COLS, a.H, n_rows);
-        if (beside)
-            return (int)sllm_launch_pdl(delta_rule_step_kernel<T, CHANNEL>, grid, dim3(32 * STEP_WARPS), 0, stream, a, true);
-        delta_rule_step_kernel<T, CHANNEL><<<grid, 32 * STEP_WARPS, 0, stream>>>(a, false);
+        const bool words = D % 4 == 0 && ((uintptr_t)a.state & 15) == 0;
+        const auto kernel = words ? delta_rule_step_kernel<T, CHANNEL, D % 4 == 0> : delta_rule_step_kernel<T, CHANNEL, false>;
+        if (beside) return (int)sllm_launch_pdl(kernel, grid, dim3(32 * STEP_WARPS), 0, stream, a, true);
+        kernel<<<grid, 32 * STEP_WARPS, 0, stream>>>(a, false);
         SLLM_LAUNCH_CHECK();
         return 0;
     }

@@ -40,3 +40,27 @@ def test_delta_step(dtype, channels, D, V, H, G):
     assert ((out.double().cpu().view(rows, H, V) - want).norm() / want.norm()).item() < 3e-6
     assert ((S[[2, 3, 1]].double().cpu() - want_S).norm() / want_S.norm()).item() < 3e-6
     assert torch.equal(S[0].cpu(), start[0])
+
+
+@pytest.mark.parametrize("D,V", [(128, 33), (160, 37), (64, 7)])
+@pytest.mark.parametrize("lengths", [[1, 1], [1, 5, 1], [1, 130, 20]])
+def test_delta_state_on_any_boundary(D, V, lengths):
+    """A state that starts on no 16-byte boundary goes element by element: the same bits in steps of single
+    tokens, and in mixed ones where no row is long enough for chunks (which need the boundary)."""
+    from scratch_llm_b200.kernels import ops
+    H, n, rows = 2, sum(lengths), len(lengths)
+    gen = torch.Generator(device=DEV).manual_seed(D)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=gen)  # noqa: E731
+    act, ab, A_log, dt_bias, start = r(n, 4 * D + H * V), r(n, 2 * H), r(H), r(H), r(rows, H, V, D)
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device=DEV)  # noqa: E731
+    row_start, slots = i32([sum(lengths[:i]) for i in range(rows + 1)]), i32(list(range(rows)))
+    got = []
+    for shift in (0, 1):
+        S = torch.empty(start.numel() + 4, device=DEV)[shift:shift + start.numel()].view(start.shape).copy_(start)
+        assert S.data_ptr() % 16 == 4 * shift
+        out = torch.empty(n, H * V, device=DEV)
+        ops.delta_rule(act, ab, A_log, dt_bias, S, row_start, slots, out, rows, H, 2, D, V,
+                       max_new=1 if max(lengths) == 1 else 0, longest=max(lengths),
+                       min_chunked=0 if shift == 0 else None)
+        got.append((out, S.clone()))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
