@@ -79,11 +79,26 @@ def _pick_build_dir() -> Path:
     raise BuildError("no writable folder for compiled kernels; set SCRATCH_LLM_B200_BUILD_DIR")
 
 
+#: (name, size, time of change) of the headers and their hash so far: they are read again when one changes
+_headers: tuple[list[tuple], "hashlib._Hash"] | None = None
+
+
+def _header_hash() -> "hashlib._Hash":
+    global _headers
+    paths = sorted([*CSRC.glob("*.cuh"), *CSRC.glob("*.h")])
+    seen = [(p.name, (st := p.stat()).st_size, st.st_mtime_ns) for p in paths]
+    known = _headers
+    if known is None or known[0] != seen:
+        h = hashlib.sha256()
+        for p in paths:
+            h.update(p.name.encode())
+            h.update(p.read_bytes())
+        _headers = known = (seen, h)
+    return known[1].copy()
+
+
 def _digest(sources: Sequence[Path], flags: Sequence[str]) -> str:
-    h = hashlib.sha256()
-    for p in sorted([*CSRC.glob("*.cuh"), *CSRC.glob("*.h")]):
-        h.update(p.name.encode())
-        h.update(p.read_bytes())
+    h = _header_hash()
     for p in sources:
         h.update(p.name.encode())
         h.update(p.read_bytes())
