@@ -7,7 +7,7 @@
 // and N are, so a token's result does not depend on what else is in the batch.
 //
 // Three kernels.  32-bit operands whose rows allow 16-byte requests, by size:
-//   gemm_f32_wide_kernel   tiles of 64 x 64, where those give every SM two (296 tiles)
+//   gemm_f32_wide_kernel   tiles of 64 x 64, where those give every SM two
 //   gemm_f32_kernel        smaller tiles behind a ring of cp.async stages: few tokens are bound by the chain
 //                          of steps over k, whose loads the ring keeps ahead of.  Tiles of 32 x 32, and of
 //                          16 x 16 up to 16 tokens.
@@ -264,7 +264,11 @@ SLLM_EXPORT int sllm_gemm_simt(const void* X, const void* W, void* Y, int M, int
         const auto y = (float*)Y;
         const int64_t wide = (int64_t)((M + 63) / 64) * ((N + 63) / 64);
         if (M <= 16) return launch_f32<16, 16, 2, 2, 64, 4>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
-        if (wide < 296) return launch_f32<32, 32, 4, 4, 32, 4>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
+        int dev = 0, n_sm = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            return (int)cudaErrorInvalidDevice;
+        if (wide < 2 * n_sm) return launch_f32<32, 32, 4, 4, 32, 4>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
         const dim3 tiles((N + WIDE - 1) / WIDE, (M + WIDE - 1) / WIDE);
         if (tiles.y > 65535) return (int)cudaErrorInvalidValue;
         gemm_f32_wide_kernel<<<tiles, WIDE, 0, stream>>>(x, w, y, M, N, K, ldx, ldw, ldy);
