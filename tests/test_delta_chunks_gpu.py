@@ -173,3 +173,95 @@ def test_scratch_goes_with_the_chunks(lengths, limit):
         run(rows)
     chunk = 32 * 4 * (3 * 64 * 128 + 64 * 128 + 64 * 64 + 128 * 128 + 128)
     assert sum(seen) <= limit * chunk and sum(seen) <= 512 << 20
+
+
+@pytest.mark.parametrize("channels", [False, True])
+def test_captured_step_with_other_rows(channels):
+    """A captured step replayed with other rows of the same padded sizes: long rows, none, tokens of padding."""
+    D, V, H, G, n, rows = 64, 48, 2, 1, 320, 5
+    g = torch.Generator(device=DEV).manual_seed(5)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    act, ab, start = r(n, 2 * G * D + H * V).bfloat16(), r(n, 2 * H), r(rows, H, V, D)
+    A_log, dt_bias, log_decay = r(H), r(H), -torch.exp(r(n, H * D) - 2)
+    S, out, slots = start.clone(), torch.zeros(n, H * V, device=DEV), i32([4, 3, 2, 1, 0])
+    row_start = torch.zeros(rows + 1, dtype=torch.int32, device=DEV)
+
+    def step():
+        ops().delta_rule(act, ab, None if channels else A_log, None if channels else dt_bias, S, row_start, slots, out,
+                         rows, H, G, D, V, longest=n, log_decay=log_decay if channels else None)
+
+    def set_rows(lengths):
+        row_start.copy_(i32([sum(lengths[:i]) for i in range(rows + 1)]))
+        S.copy_(start)
+        out.zero_()
+
+    set_rows([320, 0, 0, 0, 0])
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        step()
+    for lengths in ([320, 0, 0, 0, 0], [1, 150, 7, 128, 1], [60, 70, 80, 1, 1], [127, 0, 1, 192, 0], [2, 1, 1, 1, 1]):
+        set_rows(lengths)
+        graph.replay()
+        got = out.clone(), S.clone()
+        set_rows(lengths)
+        step()
+        assert torch.equal(got[0], out) and torch.equal(got[1], S), lengths
+
+
+@pytest.mark.parametrize("channels", [False, True])
+@pytest.mark.parametrize("cut", [[128, 272], [127, 273], [1, 130, 5, 128, 1, 135], [64, 200, 127, 9]])
+def test_portions_above_and_below_the_limit(channels, cut):
+    """One row's tokens in one step, and cut into steps that continue from its state."""
+    D, V, H, G, n = 128, 40, 2, 1, 400
+    g = torch.Generator(device=DEV).manual_seed(6)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    act, ab, start = r(n, 2 * G * D + H * V), r(n, 2 * H), r(1, H, V, D)
+    A_log, dt_bias, log_decay = r(H), r(H), -torch.exp(r(n, H * D) - 3)
+    results = []
+    for lengths in ([n], cut):
+        S, outs, t = start.clone(), [], 0
+        for m in lengths:
+            outs.append(torch.empty(m, H * V, device=DEV))
+            ops().delta_rule(act[t:t + m], ab[t:t + m], None if channels else A_log, None if channels else dt_bias, S,
+                             i32([0, m]), i32([0]), outs[-1], 1, H, G, D, V, max_new=1 if m == 1 else 0, longest=m,
+                             shortest=m, log_decay=log_decay[t:t + m] if channels else None)
+            t += m
+        results.append((torch.cat(outs), S))
+    for what, a, b in zip(("out", "state"), *results):
+        close(b, a.double().cpu(), f"{what} of the portions")
+
+
+@pytest.mark.parametrize("channels", [False, True])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_row_that_is_no_number(channels, bad):
+    """A row with an infinity or a NaN in its tokens or its state leaves the rows beside it alone, and its own
+    tokens before the bad one's block of 16."""
+    lengths = [130, 200, 20, 1, 300]
+    H, G, D, V = 2, 1, 64, 48
+    n, rows = sum(lengths), len(lengths)
+    g = torch.Generator(device=DEV).manual_seed(7)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    act, ab, start = r(n, 2 * G * D + H * V), r(n, 2 * H), r(rows, H, V, D)
+    A_log, dt_bias, log_decay = r(H), r(H), -torch.exp(r(n, H * D) - 2)
+    results = []
+    for spoil in (False, True):
+        x, S, out = act.clone(), start.clone(), torch.empty(n, H * V, device=DEV)
+        if spoil:
+            x[130 + 100, G * D + 3] = bad          # a key of row 1, its token 100
+            x[350, :] = bad                        # the single row's token and state
+            S[3, 0, 0, 0] = bad
+        ops().delta_rule(x, ab, None if channels else A_log, None if channels else dt_bias, S,
+                         i32([sum(lengths[:i]) for i in range(rows + 1)]), i32(list(range(rows))), out, rows, H, G, D, V,
+                         longest=max(lengths), log_decay=log_decay if channels else None)
+        results.append((out, S))
+    clean = torch.ones(n, dtype=torch.bool)
+    clean[130 + 96:330] = False
+    clean[350] = False
+    assert torch.equal(results[0][0][clean], results[1][0][clean])
+    for row in (0, 2, 4):
+        assert torch.equal(results[0][1][row], results[1][1][row])
+    assert results[1][0][130 + 101:330].isnan().any(1).all()
