@@ -24,7 +24,9 @@
 //
 // Why: a row's tokens in order are a chain of 128 pieces of 16 tokens for 2,048 tokens, 5.9 us each
 // whatever the GPU's width.  In chunks the chain has 32 links of two small products.  2,048 tokens, 16
-// heads of 128 x 128, bfloat16: one decay per head 733 -> 246 us, per channel 666 -> 343 us.
+// heads of 128 x 128, bfloat16: one decay per head 733 -> 252 us, per channel 666 -> 343 us.  One by one, per head: 56,
+// 89 and 46 us; in a stream, where a kernel's CTAs take the places that the one before it leaves first and wait
+// there, 252.
 #pragma once
 
 #include <algorithm>
@@ -320,7 +322,7 @@ template <int D, typename T> constexpr size_t prep_head_smem() {
 
 // One decay per head.  The tables are products of keys and queries as they stand (bfloat16: on the tensor
 // cores, exact products summed in 32-bit); the norms and decays are factors per token and per pair of
-// tokens.  52 us at 2,048 tokens and 16 heads of 128 x 128; bound by the substitution's shared-memory reads
+// tokens.  56 us at 2,048 tokens and 16 heads of 128 x 128; bound by the substitution's shared-memory reads
 // (544 of 16 bytes a warp) and, with two CTAs of eight warps an SM, by latencies.
 template <int D, typename T>
 __device__ __forceinline__ void prep_head(const PrepArgs& a, const Scratch& z, const Group& group) {
@@ -542,7 +544,8 @@ __device__ __forceinline__ void block_pairs(const float* x, const float* y, cons
 
 // A decay per key channel.  Arrays in shared memory change what they hold: R = q, then q e^{l}; U = k, then
 // k e^{l}; L = the decays, then k e^{border - l} (l: sums of logarithms from the block's border on).  One
-// CTA an SM (127 KB at D = 128); 256 us at 3,001 tokens in four rows and 16 heads of 128 x 128.
+// CTA an SM: the 254 registers of the substitution's column allow no second, nor do 127 KB at D = 128.  245 us at
+// 3,001 tokens in four rows and 16 heads of 128 x 128 (960 CTAs, 6.5 rounds).
 template <int D, typename T>
 __device__ __forceinline__ void prep_channels(const PrepArgs& a, const Scratch& z, const Group& group) {
     constexpr int LD = D + 4;
@@ -722,9 +725,11 @@ constexpr int LDP = TC + 8;              // row stride of what the pass's warps 
 // each warp for its own channels, X split into parts once by whom adds it up.  W and y~ are used once per
 // CTA and come straight from memory into the registers of the thread that needs them, a chunk ahead.
 //
-// What bounds it: the chain of chunks, each two barriers and two products of K = 16 and 64, about 4,400
-// cycles at 128 x 128, of which the 192 mma.sync a scheduler issues take the most.  As fused multiply-adds
-// from shared memory a chunk took 4,700 cycles (shared-memory reads).
+// What bounds it, for one row: the chain of chunks, each two barriers and two products of K = 16 and 64, of
+// which the 192 mma.sync a scheduler issues take the most: 89 us for 32 chunks of 128 x 128 with 16 heads (128
+// CTAs), 2.8 us a chunk.  With more CTAs than SMs, the mma.sync and the reads of W and y~, which every 16 columns
+// repeat: four rows of 401 to 1,201 tokens 138 us, where the longest alone is 19 chunks.  As fused
+// multiply-adds from shared memory the layer of one row took 348 us where this took 333.
 template <int D>
 __global__ void __launch_bounds__(2 * D)
 pass_kernel(const Scratch z, const Group group, float* __restrict__ state, const int* __restrict__ row_start,
@@ -869,9 +874,10 @@ template <int D> constexpr size_t out_smem() { return (size_t)(TC + OUT_COLS) * 
 
 // o of a chunk, head and 64 columns: a warp has 16 tokens and 32 columns, both operands of both products
 // lie in shared memory with the summed index last and are split into parts as they are read.  Row strides
-// are 8 banks apart: a half-warp's reads of two elements meet every bank once.  Bound by mma.sync's rate
-// and the split's arithmetic, 7,000 of a CTA's 14,000 cycles; the rest are its loads, which the other CTA
-// of the SM covers.  (As fused multiply-adds it was bound by shared-memory reads.)
+// are 8 banks apart: a half-warp's reads of two elements meet every bank once.  46 us at
+// 2,048 tokens and 16 heads of 128 x 128, 78 us at 3,001 (1,056 and 1,920 CTAs, two an SM): mma.sync, the split's
+// arithmetic, and 106 KB of loads a CTA that only the other CTA of the SM covers.  (As fused multiply-adds it
+// was bound by shared-memory reads.)
 template <int D>
 __global__ void __launch_bounds__(OUT_THREADS, 2)
 out_kernel(const Scratch z, const Group group, const int* __restrict__ row_start, float* __restrict__ out,

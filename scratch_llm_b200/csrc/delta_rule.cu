@@ -31,10 +31,8 @@
 // announces u_s, every lane adds its row's weight times u_s to its own sum, so that the lanes
 // 16 + t end with the read-outs o_t.  Last comes the rank-16 update of its elements of S.
 // All of it is 32-bit.  A chunk's inputs are requested one chunk ahead and wait in registers.
-// The same kernel serves portions of prompts (many tokens per row) and decoding (a chunk of one
-// token); a row reads its state from its slot and writes it back; rows without tokens touch
-// nothing.
-//
+// A row reads its state from its slot and writes it back; rows without tokens touch nothing.  Rows of one
+// token (decoding) have a kernel of their own, delta_rule_step_kernel.
 //
 // A decay per key CHANNEL (log_decay != null: float [tokens, H * D], the logarithm of each
 // channel's factor, at most 0): S <- diag(g) S in the rule's first line.  With L_t now the vector
@@ -47,7 +45,9 @@
 // pair of tokens, shared by the CTA's 16 columns.  The step size then comes from column b_col +
 // head of `ab`, and A_log / dt_bias are the caller's business (they are inside log_decay).
 //
-// Rows of at least min_chunked tokens go to the kernels of delta_chunks.cuh where the key size fits them.
+// Rows of at least min_chunked tokens go to the kernels of delta_chunks.cuh where the key size fits them.  A row
+// takes one path whatever else is in its step, and the paths of a step run side by side as far as the stream's
+// order lets them (sllm_delta_rule).
 //
 // The weights depend on keys, queries and decays alone: delta_weights_kernel forms the tables of
 // ALL chunks of a step in parallel before the scan starts, which then reads its chunk's table.

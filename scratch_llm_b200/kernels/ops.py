@@ -1585,9 +1585,11 @@ def moe_combine(y: torch.Tensor, x: torch.Tensor, shared: torch.Tensor | None, i
 
 #: rows of at least so many tokens run in chunks in the delta rule.  In order against in chunks, one
 #: decay per head / per channel: 1 row of 96 tokens, 16 heads of 128 x 128: 39 / 41 and 44 / 53 us;
-#: of 128 tokens: 50 / 41 and 54 / 53 us, with 32 heads 97 / 49 and 95 / 55 us; of 2,048: 733 / 246 and
-#: 666 / 343 us.  (With more heads and rows shorter ones gain too, but a row takes one path
-#: whatever else is in the step.)
+#: of 128 tokens: 48 / 40 and 49 / 53 us, with 32 heads 95 / 49 and 91 / 55 us; of 2,048: 731 / 252 and
+#: 661 / 343 us.  (With more heads and rows shorter ones gain too, but a row takes one path
+#: whatever else is in the step.)  What that costs: rows on both sides of the limit take one path after the
+#: other but for the tables and solves, rows of 127 and 128 tokens with 4 heads 64 us where both in order
+#: take 48, with 16 heads 95 / 97 and 94 / 91, with 32 heads 142 / 148 and 187 / 176.
 DELTA_MIN_CHUNKED = 128
 
 
@@ -1626,7 +1628,7 @@ def delta_rule(act: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias
     holds query heads, key heads and value heads after the convolution; ``ab`` float32
     [N, 2 H] the decay and step inputs; ``state`` float32 [slots, H, V, D] is read and written
     at the rows' slots; ``out`` float32 [N, H * V].  ``max_new``: the most tokens a row brings,
-    if known (1 selects the kernel for decode steps; 0: not known).
+    if known (1: every row is for the kernel of one-token rows; 0: not known).
 
     ``log_decay`` (float32 [N, H * D], at most 0): a decay per key CHANNEL, given as its
     logarithm; ``a_log`` and ``dt_bias`` are then not read (may be None), and head h's step input
