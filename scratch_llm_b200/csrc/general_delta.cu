@@ -7,21 +7,32 @@
 // the unit key.  Both terms read the old state.  A column of S (one value channel) never meets
 // another column: s <- w * s - (a * u) (u . s) + k v_c, o_c = s . r.
 //
-// Layout: a column is spread over LANES neighbouring lanes of a warp, each with EPL = 16 of
-// its elements in registers (a thread holds such slices of CPT = 2 columns: the five vectors it
-// reads from shared memory per token serve both, and shared-memory bandwidth is what a token
-// costs an SM) (the key size D is padded to LANES * 16; the padding stays zero).
-// Lane l owns the float4 units l, l + LANES, l + 2 LANES, ... of the column, so that the lanes
-// of a column read consecutive 16-byte words of shared memory.  A CTA has one COMPUTE warp,
-// which owns 2 * 32 / LANES columns of one (row, head), and two LOADER warps; a head's columns are
-// spread over several CTAs (many SMs work on one sequence, and the shared-memory reads of a
-// token, five vectors per thread, are shared out with them).  The row's tokens come in chunks
-// through two buffers: while the compute warps run chunk c, the loader warps fetch chunk c + 1
-// (r, k, w, a of the head, v of the CTA's columns), form the unit key and a * u, and all
-// warps meet once per chunk.  Per token the only chain is (partial dot of 16 products) ->
-// log2(LANES) shuffles -> one multiply-add per element; the read-out s . r is kept as a partial
-// sum per token and summed across the lanes after the chunk, off the chain.  Rows of one token
-// (decode steps) take the same path with a chunk of one.
+// Layout: a column is spread over LANES neighbouring lanes of a warp, each with EPL = 4 of its
+// elements in registers as pairs (the key size D is padded to DP = 16 * 2^i; the padding stays
+// zero), and a thread holds such slices of CPT = 4 neighbouring columns, which the vectors that it
+// reads from shared memory per token serve together.  A CTA has four COMPUTE warps, one per
+// scheduler, which own 128 / LANES * CPT columns of one (row, head), and four LOADER warps; a
+// head's columns are spread over several CTAs.  The row's tokens come in chunks through two
+// buffers: while the compute warps run chunk c, the loader warps, which have requested chunk
+// c + 1 (r, k, w, a of the head, v of the CTA's columns) a chunk earlier, form -a * k, 1 / (|k|^2 +
+// eps) and the products of neighbouring tokens; all warps meet once per chunk.
+//
+// What bounds a long row is the chain from token to token, so the chain is cut: with
+// g_t = w_t s_{t-1} + k_t v_t (the new state before the removal), i_t = 1 / (|k_t|^2 + eps) and
+// d_t = i_t k_t . s_{t-1}, so that s_t = g_t - (a_t k_t) d_t,
+//     d_{t+1} = i_{t+1} k_{t+1} . s_t = i_{t+1} (k_{t+1} . g_t) - i_{t+1} (k_{t+1} . (a_t k_t)) d_t.
+// The dot product with g_t and its shuffles need d_{t-1}, not d_t: two tokens are in flight, and
+// what joins them is one multiply-add with a number that the loaders have formed.  Shuffles are
+// issued in the order in which they are written, so a token's step is written as the two tokens
+// run: the second half of one sum beside the first half of the next (`Pipe`).
+// Multiply-adds come in pairs (fma.rn.f32x2: the same rate, half the instructions).
+//
+// us before (a column a thread, sixteen elements a lane, five vectors) and now, bfloat16, 64 x 64:
+//   32 heads, a row of 2,048 tokens   592 / 300       64 heads, a row of 2,400       908 / 354
+//   32 heads, four rows of 1,024      485 / 246       64 heads, eight rows of 300    550 / 253
+//   32 heads, 64 single tokens         40 / 29        128 x 128, 16 heads, 2,048     734 / 367
+// It issues 138 instructions per token and scheduler in 300 cycles: latencies.  With two columns a thread
+// (twice the CTAs) the first takes 239, four rows of 1,024 348 and 64 single tokens 48.
 //
 // state: float32 [slots, H, V, DP] with DP = the padded key size; a fresh slot holds zeros.
 // Compiled once per key size (-DSLLM_HEAD_DIM=D).
@@ -34,31 +45,53 @@
 namespace sllm {
 
 constexpr int D = SLLM_HEAD_DIM;
-constexpr int EPL = 16;                       // elements of a column per lane
-constexpr int lanes_for(int d) {
-    int l = 1;
-    while (l * EPL < d) l *= 2;
-    return l;
+constexpr int padded(int d) {
+    int p = 16;
+    while (p < d) p *= 2;
+    return p;
 }
-constexpr int LANES = lanes_for(D);
-static_assert(LANES <= 32, "key sizes up to 512");
-constexpr int DP = LANES * EPL;               // padded key size
-constexpr int COMPUTE = 64, LOADERS = 64, THREADS = COMPUTE + LOADERS;
-// columns per compute thread (measured at 32 heads of 64 x 64, 2,048 tokens: 1 column and two
-// compute warps 571 us; 2 columns and one warp 844 us; a warp's issue rate, not shared memory,
-// is what a token costs)
-constexpr int CPT = 1;
+constexpr int DP = padded(D);                 // padded key size
+static_assert(DP <= 512, "key sizes up to 512");
+constexpr int EPL = DP <= 128 ? 4 : DP / 32;  // elements of a column per lane
+constexpr int LANES = DP / EPL;
+constexpr int CPT = EPL == 4 ? 4 : 16 / EPL;       // columns per compute thread
+constexpr int COMPUTE = 128, LOADERS = 128, THREADS = COMPUTE + LOADERS;
 constexpr int COLS = COMPUTE / LANES * CPT;   // columns of S per CTA
 constexpr int UNITS = EPL / 4;                // float4 units per lane
-// tokens per chunk: two buffers of five vectors of DP floats per token, within 40 KB
-constexpr int CHUNK = (20 * 1024 / (5 * DP * 4)) >= 16 ? 16 : (20 * 1024 / (5 * DP * 4));
+// tokens per chunk: two buffers of four vectors of DP floats per token, within 64 KB
+constexpr int CHUNK = DP <= 128 ? 16 : 2048 / DP;
 static_assert(CHUNK >= 2, "chunk too small");
 
 struct __align__(16) Staged {
-    float r[CHUNK][DP], k[CHUNK][DP], w[CHUNK][DP], u[CHUNK][DP], au[CHUNK][DP];
+    float k[CHUNK + 1][DP];     // (the last: the first key of the chunk that follows)
+    float r[CHUNK][DP], w[CHUNK][DP], nak[CHUNK][DP];   // nak: -a * k
     float v[CHUNK][COLS];
-    float inv[CHUNK];
+    float2 ic[CHUNK];           // i_t = 1 / (|k_t|^2 + eps), and i_t (k_t . nak_{t-1})
 };
+constexpr int SMEM = 2 * (int)sizeof(Staged);
+
+// two 32-bit numbers in one register pair
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f2 pair(float x) {
+    f2 d;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(x));
+    return d;
+}
+__device__ __forceinline__ float pair_sum(f2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+    return x + y;
+}
 
 __device__ __forceinline__ void loaders_sync() {
     asm volatile("bar.sync 1, %0;\n" ::"n"(LOADERS) : "memory");
@@ -75,76 +108,89 @@ __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
 
 constexpr int QUADS = CHUNK * DP / 4;                       // units of 4 elements in a chunk
 constexpr int QPT = (QUADS + LOADERS - 1) / LOADERS;        // of which a loader thread takes
-// a token's units fit the lanes of one warp (and LOADERS is a multiple of them): the unit key is
-// formed in registers
-constexpr bool FUSED_UNIT = DP / 4 <= 32;
+constexpr int VPT = (CHUNK * COLS + LOADERS - 1) / LOADERS; // values that a loader thread takes
+constexpr int APT = (DP / 4 + LOADERS - 1) / LOADERS;       // units of the key after the chunk
+// a token's units fit the lanes of one warp (and LOADERS is a multiple of them): its sums are
+// formed from registers
+constexpr bool FUSED = DP / 4 <= 32;
 
-// The loader warps fetch the tokens [tok0, tok0 + n) of one head into `st`.  VEC: every row of
-// every operand starts on a multiple of 4 elements, so four elements come per load; a thread
-// requests all its loads before it stores any (the chunk costs one round trip, not one per
-// element).
+template <typename T> struct Operands {
+    const T* __restrict__ rkv;
+    const float* __restrict__ wa;
+    int64_t ld, ldwa;
+    int r0, k0, v0, HD, head, V, col0;
+    float unit_eps;
+};
+
+// What a loader thread has requested of a chunk.  VEC: every row of every operand starts on a
+// multiple of 4 elements, so four elements come per load.
+template <bool VEC> struct Request {
+    float4 r[VEC ? QPT : 1], k[VEC ? QPT : 1], w[VEC ? QPT : 1], a[VEC ? QPT : 1];
+    float4 k_after[VEC ? APT : 1];
+    float v[VPT];
+};
+
 template <typename T, bool VEC>
-__device__ __forceinline__ void stage_chunk(Staged& st, int lt, const T* __restrict__ rkv,
-                                            int64_t ld, int r0, int k0, int v0,
-                                            const float* __restrict__ wa, int64_t ldwa, int HD,
-                                            int head, int V, int col0, int64_t tok0, int n,
-                                            float unit_eps) {
+__device__ __forceinline__ void request_chunk(Request<VEC>& q, int lt, const Operands<T>& x,
+                                              int64_t tok0, int n, bool more) {
     if (VEC) {
-        float4 r[QPT], k[QPT], w[QPT], a[QPT];
+#pragma unroll
+        for (int j = 0; j < APT; ++j) {
+            const int e = (lt + j * LOADERS) * 4;
+            q.k_after[j] = more && e < D ? load4(x.rkv + (tok0 + n) * x.ld + x.k0 + x.head * D + e)
+                                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
 #pragma unroll
         for (int j = 0; j < QPT; ++j) {
             const int i = lt + j * LOADERS;
             const int t = i / (DP / 4), e = (i - t * (DP / 4)) * 4;
-            r[j] = k[j] = w[j] = a[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            q.r[j] = q.k[j] = q.w[j] = q.a[j] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (i < QUADS && t < n && e < D) {
                 const int64_t tok = tok0 + t;
-                r[j] = load4(rkv + tok * ld + r0 + head * D + e);
-                k[j] = load4(rkv + tok * ld + k0 + head * D + e);
-                w[j] = load4(wa + tok * ldwa + head * D + e);
-                a[j] = load4(wa + tok * ldwa + HD + head * D + e);
+                q.r[j] = load4(x.rkv + tok * x.ld + x.r0 + x.head * D + e);
+                q.k[j] = load4(x.rkv + tok * x.ld + x.k0 + x.head * D + e);
+                q.w[j] = load4(x.wa + tok * x.ldwa + x.head * D + e);
+                q.a[j] = load4(x.wa + tok * x.ldwa + x.HD + x.head * D + e);
             }
         }
-        if (FUSED_UNIT) {
-            // a token's DP / 4 units lie in neighbouring lanes of one warp: |k|^2 is summed
-            // across them and the unit key and a * u are stored at once (no second pass)
-            for (int i = lt; i < n * COLS; i += LOADERS) {
-                const int t = i / COLS, c = i - t * COLS;
-                st.v[t][c] = col0 + c < V
-                    ? to_float(rkv[(tok0 + t) * ld + v0 + head * V + col0 + c]) : 0.f;
-            }
+    }
 #pragma unroll
-            for (int j = 0; j < QPT; ++j) {
-                const int i = lt + j * LOADERS;
-                const int t = i / (DP / 4), e = (i - t * (DP / 4)) * 4;
-                float ss = fmaf(k[j].x, k[j].x, fmaf(k[j].y, k[j].y,
-                                fmaf(k[j].z, k[j].z, k[j].w * k[j].w)));
+    for (int j = 0; j < VPT; ++j) {
+        const int i = lt + j * LOADERS, t = i / COLS, c = i - t * COLS;
+        q.v[j] = t < n && x.col0 + c < x.V
+            ? to_float(x.rkv[(tok0 + t) * x.ld + x.v0 + x.head * x.V + x.col0 + c]) : 0.f;
+    }
+}
+
+// The loader warps bring the chunk [tok0, tok0 + n), which they have requested, into `st`, and
+// request what is left of the `left` tokens after it.  `before`: the row of nak of the token before
+// tok0, or null.
+template <typename T, bool VEC>
+__device__ __forceinline__ void stage_chunk(Staged& st, Request<VEC>& q, int lt,
+                                            const Operands<T>& x, const float* before,
+                                            int64_t tok0, int n, int left) {
 #pragma unroll
-                for (int o = (DP / 4) >> 1; o > 0; o >>= 1)
-                    ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                const float inv = 1.0f / sqrtf(ss + unit_eps);
-                if (i < QUADS && t < n) {
-                    const float4 u = make_float4(k[j].x * inv, k[j].y * inv, k[j].z * inv,
-                                                 k[j].w * inv);
-                    *reinterpret_cast<float4*>(&st.r[t][e]) = r[j];
-                    *reinterpret_cast<float4*>(&st.k[t][e]) = k[j];
-                    *reinterpret_cast<float4*>(&st.w[t][e]) = w[j];
-                    *reinterpret_cast<float4*>(&st.u[t][e]) = u;
-                    *reinterpret_cast<float4*>(&st.au[t][e]) =
-                        make_float4(a[j].x * u.x, a[j].y * u.y, a[j].z * u.z, a[j].w * u.w);
-                }
-            }
-        } else {
+    for (int j = 0; j < VPT; ++j) {
+        const int i = lt + j * LOADERS, t = i / COLS, c = i - t * COLS;
+        if (i < CHUNK * COLS) st.v[t][c] = q.v[j];
+    }
+    if (VEC) {
+#pragma unroll
+        for (int j = 0; j < APT; ++j)
+            if ((lt + j * LOADERS) * 4 < DP)
+                *reinterpret_cast<float4*>(&st.k[CHUNK][(lt + j * LOADERS) * 4]) = q.k_after[j];
 #pragma unroll
         for (int j = 0; j < QPT; ++j) {
             const int i = lt + j * LOADERS;
             const int t = i / (DP / 4), e = (i - t * (DP / 4)) * 4;
             if (i < QUADS && t < n) {
-                *reinterpret_cast<float4*>(&st.r[t][e]) = r[j];
-                *reinterpret_cast<float4*>(&st.k[t][e]) = k[j];
-                *reinterpret_cast<float4*>(&st.w[t][e]) = w[j];
-                *reinterpret_cast<float4*>(&st.au[t][e]) = a[j];
+                *reinterpret_cast<float4*>(&st.r[t][e]) = q.r[j];
+                *reinterpret_cast<float4*>(&st.k[t][e]) = q.k[j];
+                *reinterpret_cast<float4*>(&st.w[t][e]) = q.w[j];
+                *reinterpret_cast<float4*>(&st.nak[t][e]) =
+                    make_float4(-q.a[j].x * q.k[j].x, -q.a[j].y * q.k[j].y,
+                                -q.a[j].z * q.k[j].z, -q.a[j].w * q.k[j].w);
             }
-        }
         }
     } else {
         for (int i = lt; i < n * DP; i += LOADERS) {
@@ -152,186 +198,302 @@ __device__ __forceinline__ void stage_chunk(Staged& st, int lt, const T* __restr
             const int64_t tok = tok0 + t;
             float r = 0.f, k = 0.f, w = 0.f, a = 0.f;
             if (e < D) {
-                r = to_float(rkv[tok * ld + r0 + head * D + e]);
-                k = to_float(rkv[tok * ld + k0 + head * D + e]);
-                w = wa[tok * ldwa + head * D + e];
-                a = wa[tok * ldwa + HD + head * D + e];
+                r = to_float(x.rkv[tok * x.ld + x.r0 + x.head * D + e]);
+                k = to_float(x.rkv[tok * x.ld + x.k0 + x.head * D + e]);
+                w = x.wa[tok * x.ldwa + x.head * D + e];
+                a = x.wa[tok * x.ldwa + x.HD + x.head * D + e];
             }
-            st.r[t][e] = r; st.k[t][e] = k; st.w[t][e] = w; st.au[t][e] = a;
+            st.r[t][e] = r; st.k[t][e] = k; st.w[t][e] = w; st.nak[t][e] = -a * k;
+        }
+        for (int e = lt; e < DP; e += LOADERS)
+            st.k[CHUNK][e] = left > 0 && e < D
+                ? to_float(x.rkv[(tok0 + n) * x.ld + x.k0 + x.head * D + e]) : 0.f;
+    }
+    loaders_sync();
+    if (VEC && FUSED) {
+        // a token's DP / 4 units lie in neighbouring lanes of one warp
+        float ss[QPT], c[QPT];
+#pragma unroll
+        for (int j = 0; j < QPT; ++j) {
+            const int i = lt + j * LOADERS;
+            const int t = i / (DP / 4), e = (i - t * (DP / 4)) * 4;
+            const float* p = t == 0 ? before : st.nak[t < CHUNK ? t - 1 : 0];
+            const float4 k = q.k[j];
+            ss[j] = fmaf(k.x, k.x, fmaf(k.y, k.y, fmaf(k.z, k.z, k.w * k.w)));
+            c[j] = 0.f;
+            if (i < QUADS && t < n && p) {
+                const float4 y = load4(p + e);
+                c[j] = fmaf(k.x, y.x, fmaf(k.y, y.y, fmaf(k.z, y.z, k.w * y.w)));
+            }
+        }
+#pragma unroll
+        for (int o = (DP / 4) >> 1; o > 0; o >>= 1)
+#pragma unroll
+            for (int j = 0; j < QPT; ++j) {
+                ss[j] += __shfl_xor_sync(0xffffffffu, ss[j], o);
+                c[j] += __shfl_xor_sync(0xffffffffu, c[j], o);
+            }
+#pragma unroll
+        for (int j = 0; j < QPT; ++j) {
+            const int i = lt + j * LOADERS;
+            const int t = i / (DP / 4), e = (i - t * (DP / 4)) * 4;
+            const float inv = 1.0f / (ss[j] + x.unit_eps);
+            if (i < QUADS && t < n && e == 0) st.ic[t] = make_float2(inv, inv * c[j]);
+        }
+    } else {
+        for (int t = lt >> 5; t < n; t += LOADERS / 32) {   // a warp per token
+            const float* p = t == 0 ? before : st.nak[t - 1];
+            float ss = 0.f, c = 0.f;
+            for (int e = lt & 31; e < DP; e += 32) {
+                const float k = st.k[t][e];
+                ss = fmaf(k, k, ss);
+                if (p) c = fmaf(k, p[e], c);
+            }
+            ss = warp_sum(ss);
+            c = warp_sum(c);
+            const float inv = 1.0f / (ss + x.unit_eps);
+            if ((lt & 31) == 0) st.ic[t] = make_float2(inv, inv * c);
         }
     }
-    if (!(VEC && FUSED_UNIT)) {     // (else stored above, unit key and all)
-        for (int i = lt; i < n * COLS; i += LOADERS) {
-            const int t = i / COLS, c = i - t * COLS;
-            st.v[t][c] = col0 + c < V
-                ? to_float(rkv[(tok0 + t) * ld + v0 + head * V + col0 + c]) : 0.f;
-        }
-        loaders_sync();
-        for (int t = lt >> 5; t < n; t += LOADERS / 32) {   // a warp per token: |k|^2
-            float ss = 0.f;
-            for (int e = lt & 31; e < D; e += 32) ss = fmaf(st.k[t][e], st.k[t][e], ss);
-            ss = warp_sum(ss);
-            if ((lt & 31) == 0) st.inv[t] = 1.0f / sqrtf(ss + unit_eps);
-        }
-        loaders_sync();
-        for (int i = lt; i < n * DP; i += LOADERS) {
-            const int t = i / DP, e = i - t * DP;
-            const float u = st.k[t][e] * st.inv[t];
-            st.u[t][e] = u;
-            st.au[t][e] *= u;
-        }
+    if (left > 0) request_chunk<T, VEC>(q, lt, x, tok0 + n, min(CHUNK, left), left > CHUNK);
+}
+
+constexpr int SHARE = LANES / CPT;          // lanes that go on with the same column
+static_assert(SHARE >= 1 && CPT <= 4, "no more columns a thread than lanes a column");
+
+// Sums across a column's lanes begin with CPT values per lane (one per column) that become one: each
+// exchange halves the columns that a lane goes on with.  A lane goes on with column
+// lane_in_col / SHARE.  One exchange of x's `have` pairs:
+template <int HAVE>
+__device__ __forceinline__ void share(float (&x)[CPT], int lane_in_col) {
+    constexpr int SH = LANES / CPT * HAVE;
+    const bool upper = lane_in_col & SH;
+#pragma unroll
+    for (int i = 0; i < HAVE; ++i) {
+        const float send = upper ? x[i] : x[i + HAVE], keep = upper ? x[i + HAVE] : x[i];
+        x[i] = keep + __shfl_xor_sync(0xffffffffu, send, SH);
+    }
+}
+// ... of two sums at a time, until one value of each is left.
+__device__ __forceinline__ void share_both(float (&x)[CPT], float (&y)[CPT], int lane_in_col) {
+    if constexpr (CPT >= 4) {
+        share<2>(x, lane_in_col);
+        share<2>(y, lane_in_col);
+    }
+    if constexpr (CPT >= 2) {
+        share<1>(x, lane_in_col);
+        share<1>(y, lane_in_col);
     }
 }
 
-// The compute warps' part of a chunk: n tokens of `st` through this thread's slices of its
-// columns.  out_head: the output row of the chunk's first token at this head, rows ld_out apart.
-// (A variant without the `t < n` conditions for whole chunks, which lets a token's loads be
-// requested during the chain of the one before, gained 8 % at key size 64 and lost 70 % at 128,
-// where it held too many values in flight; it was dropped.)
-__device__ __forceinline__ void run_chunk(const Staged& st, float (&s)[CPT][EPL], int n,
-                                          int lane_in_col, int col_local, int col0, int V,
-                                          float* __restrict__ out_head, int64_t ld_out) {
-    float o_part[CHUNK][CPT];
+template <int N> __device__ __forceinline__ void fetch(f2 (&x)[2 * UNITS], const float* row) {
 #pragma unroll
-    for (int t = 0; t < CHUNK; ++t) {
-        if (t < n) {
-            float dot[CPT];
-            {
-                float d[CPT][4];
+    for (int i = 0; i < UNITS; ++i) {
+        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(row + N * i);
+        x[2 * i] = y.x;
+        x[2 * i + 1] = y.y;
+    }
+}
+__device__ __forceinline__ float dot(const f2 (&x)[2 * UNITS], const f2 (&y)[2 * UNITS]) {
+    f2 acc = mul2(x[0], y[0]);
 #pragma unroll
-                for (int c = 0; c < CPT; ++c) d[c][0] = d[c][1] = d[c][2] = d[c][3] = 0.f;
+    for (int i = 1; i < 2 * UNITS; ++i) acc = fma2(x[i], y[i], acc);
+    return pair_sum(acc);
+}
+
+// What a thread carries from token t - 1 to token t: g_{t-1}, d_{t-1}, its slices of a_{t-1} k_{t-1}
+// (negated), r_{t-1} and k_t, and k_t . g_{t-1} summed as far as `share` goes.
+struct Pipe {
+    f2 g[CPT][2 * UNITS], nak[2 * UNITS], r[2 * UNITS], k[2 * UNITS];
+    float d[CPT], x;
+    int lane_in_col, col_local;
+
+    // The state after token t - 1.
+    __device__ __forceinline__ void state(f2 (&s)[CPT][2 * UNITS]) const {
 #pragma unroll
-                for (int u = 0; u < UNITS; ++u) {
-                    const float4 x = *reinterpret_cast<const float4*>(
-                        &st.u[t][4 * (lane_in_col + LANES * u)]);
+        for (int c = 0; c < CPT; ++c) {
+            const f2 dd = pair(d[c]);
 #pragma unroll
-                    for (int c = 0; c < CPT; ++c) {
-                        d[c][0] = fmaf(x.x, s[c][4 * u], d[c][0]);
-                        d[c][1] = fmaf(x.y, s[c][4 * u + 1], d[c][1]);
-                        d[c][2] = fmaf(x.z, s[c][4 * u + 2], d[c][2]);
-                        d[c][3] = fmaf(x.w, s[c][4 * u + 3], d[c][3]);
-                    }
-                }
-#pragma unroll
-                for (int c = 0; c < CPT; ++c)
-                    dot[c] = (d[c][0] + d[c][1]) + (d[c][2] + d[c][3]);
-            }
-#pragma unroll
-            for (int o = LANES >> 1; o > 0; o >>= 1)
-#pragma unroll
-                for (int c = 0; c < CPT; ++c)
-                    dot[c] += __shfl_xor_sync(0xffffffffu, dot[c], o);
-            float v[CPT], p[CPT][4];
-#pragma unroll
-            for (int c = 0; c < CPT; ++c) {
-                v[c] = st.v[t][col_local + c];
-                p[c][0] = p[c][1] = p[c][2] = p[c][3] = 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < UNITS; ++u) {
-                const int e = 4 * (lane_in_col + LANES * u);
-                const float4 w = *reinterpret_cast<const float4*>(&st.w[t][e]);
-                const float4 au = *reinterpret_cast<const float4*>(&st.au[t][e]);
-                const float4 k = *reinterpret_cast<const float4*>(&st.k[t][e]);
-                const float4 r = *reinterpret_cast<const float4*>(&st.r[t][e]);
-#pragma unroll
-                for (int c = 0; c < CPT; ++c) {
-                    float* sc = &s[c][4 * u];
-                    sc[0] = fmaf(k.x, v[c], fmaf(-au.x, dot[c], w.x * sc[0]));
-                    sc[1] = fmaf(k.y, v[c], fmaf(-au.y, dot[c], w.y * sc[1]));
-                    sc[2] = fmaf(k.z, v[c], fmaf(-au.z, dot[c], w.z * sc[2]));
-                    sc[3] = fmaf(k.w, v[c], fmaf(-au.w, dot[c], w.w * sc[3]));
-                    p[c][0] = fmaf(sc[0], r.x, p[c][0]);
-                    p[c][1] = fmaf(sc[1], r.y, p[c][1]);
-                    p[c][2] = fmaf(sc[2], r.z, p[c][2]);
-                    p[c][3] = fmaf(sc[3], r.w, p[c][3]);
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < CPT; ++c)
-                o_part[t][c] = (p[c][0] + p[c][1]) + (p[c][2] + p[c][3]);
+            for (int i = 0; i < 2 * UNITS; ++i) s[c][i] = fma2(nak[i], dd, g[c][i]);
         }
     }
+    // k_t . g_{t-1} and the read-out of token t - 1, as far as `share` goes.
+    __device__ __forceinline__ float begin(const f2 (&s)[CPT][2 * UNITS]) {
+        float xp[CPT], op[CPT];
 #pragma unroll
-    for (int t = 0; t < CHUNK; ++t) {
-        if (t < n) {
+        for (int c = 0; c < CPT; ++c) xp[c] = dot(k, g[c]);
 #pragma unroll
-            for (int c = 0; c < CPT; ++c) {
-                float o = o_part[t][c];
+        for (int c = 0; c < CPT; ++c) op[c] = dot(r, s[c]);
+        share_both(xp, op, lane_in_col);
+        x = xp[0];
+        return op[0];
+    }
+    // Token t of the chunk; returns the read-out of the token before it (see begin).
+    __device__ __forceinline__ float step(const Staged& st, int t) {
+        const int e0 = 4 * lane_in_col;
+        f2 w[2 * UNITS], kn[2 * UNITS], s[CPT][2 * UNITS], rn[2 * UNITS], an[2 * UNITS];
+        fetch<4 * LANES>(w, &st.w[t][e0]);
+        fetch<4 * LANES>(kn, &st.k[t + 1][e0]);
+        const float2 ic = st.ic[t];
+        float v[CPT];
 #pragma unroll
-                for (int sh = LANES >> 1; sh > 0; sh >>= 1)
-                    o += __shfl_xor_sync(0xffffffffu, o, sh);
-                const int col = col0 + col_local + c;
-                if (lane_in_col == 0 && col < V)
-                    out_head[(int64_t)t * ld_out + col] = o;
+        for (int c = 0; c < CPT; ++c) v[c] = st.v[t][col_local + c];
+        fetch<4 * LANES>(an, &st.nak[t][e0]);
+        fetch<4 * LANES>(rn, &st.r[t][e0]);
+        float y;
+        if (SHARE >= 2) y = __shfl_xor_sync(0xffffffffu, x, SHARE / 2);
+        state(s);
+        if (SHARE >= 2) x += y;
+        if (SHARE >= 4) y = __shfl_xor_sync(0xffffffffu, x, SHARE / 4);
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+            const f2 vv = pair(v[c]);
+#pragma unroll
+            for (int i = 0; i < 2 * UNITS; ++i) g[c][i] = fma2(w[i], s[c][i], mul2(k[i], vv));
+        }
+        if (SHARE >= 4) x += y;
+#pragma unroll
+        for (int o = SHARE / 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        float sum[CPT];      // every lane gets its columns' sums from the lanes that have them
+#pragma unroll
+        for (int c = 0; c < CPT; ++c)
+            sum[c] = CPT == 1 ? x : __shfl_sync(0xffffffffu, x, c * SHARE, LANES);
+        float xp[CPT], op[CPT];
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) xp[c] = dot(kn, g[c]);
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) op[c] = dot(r, s[c]);
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) d[c] = fmaf(ic.y, d[c], ic.x * sum[c]);
+        share_both(xp, op, lane_in_col);
+        x = xp[0];
+#pragma unroll
+        for (int i = 0; i < 2 * UNITS; ++i) {
+            k[i] = kn[i];
+            nak[i] = an[i];
+            r[i] = rn[i];
+        }
+        return op[0];
+    }
+};
+
+// Sums of GROUP tokens' read-outs across the lanes of a column: each exchange halves the tokens
+// that a lane goes on with; a lane ends with the tokens first .. of its column.
+constexpr int GROUP = CHUNK < 4 ? CHUNK : 4;
+constexpr int KEPT = GROUP >= SHARE ? GROUP / SHARE : 1;
+__device__ __forceinline__ int share_tokens(float (&o)[GROUP], int lane_in_col) {
+    int first = 0, have = GROUP;
+#pragma unroll
+    for (int sh = SHARE >> 1; sh > 0; sh >>= 1) {
+        if (have > 1) {
+            have >>= 1;
+            const bool upper = lane_in_col & sh;
+#pragma unroll
+            for (int i = 0; i < GROUP / 2; ++i) {
+                if (i >= have) break;
+                const float send = upper ? o[i] : o[i + have], keep = upper ? o[i + have] : o[i];
+                o[i] = keep + __shfl_xor_sync(0xffffffffu, send, sh);
             }
+            first += upper ? have : 0;
+        } else {
+            o[0] += __shfl_xor_sync(0xffffffffu, o[0], sh);
         }
     }
+    return first;
 }
 
 // rkv: [N, ld] with the heads' r at column r0, k at k0, v at v0 (each heads x D or heads x V);
 // wa: float32 [N, ldwa] with the decays at column 0 and the removal rates at column H * D.
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, DP <= 128 ? 2 : 1)
 general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int v0,
                      const float* __restrict__ wa, int64_t ldwa, float* __restrict__ state,
                      const int* __restrict__ row_start, const int* __restrict__ row_slot,
                      float* __restrict__ out, int H, int V, float unit_eps) {
     pdl_wait();
     pdl_trigger();
-    __shared__ Staged stage[2];
+    extern __shared__ __align__(16) uint8_t smem[];
+    Staged* stage = reinterpret_cast<Staged*>(smem);
     const int row = blockIdx.z, head = blockIdx.y;
     const int t0 = row_start[row], n_new = row_start[row + 1] - t0;
     if (n_new <= 0) return;
     const int tid = threadIdx.x;
     const bool loader = tid >= COMPUTE;
-    const int lane_in_col = tid % LANES;
-    const int col_local = (tid % COMPUTE) / LANES * CPT, col0 = blockIdx.x * COLS;
-    // this thread's columns: col0 + col_local + c, c < CPT
-    float* sp = state + (((int64_t)row_slot[row] * H + head) * V) * DP;
-    float s[CPT][EPL];
+    const int col0 = blockIdx.x * COLS;
+    if (loader) {
+        const int lt = tid - COMPUTE;
+        const Operands<T> x{rkv, wa, ld, ldwa, r0, k0, v0, H * D, head, V, col0, unit_eps};
+        Request<VEC> q;
+        request_chunk<T, VEC>(q, lt, x, t0, min(CHUNK, n_new), n_new > CHUNK);
+        for (int c0 = 0, buf = 0; c0 < n_new; c0 += CHUNK, buf ^= 1) {
+            stage_chunk<T, VEC>(stage[buf], q, lt, x, c0 ? stage[buf ^ 1].nak[CHUNK - 1] : nullptr,
+                                (int64_t)t0 + c0, min(CHUNK, n_new - c0), n_new - c0 - CHUNK);
+            __syncthreads();    // chunk c is staged, chunk c - 1 is done with
+        }
+        return;
+    }
+    Pipe p;
+    p.lane_in_col = tid % LANES;
+    p.col_local = tid / LANES * CPT;
+    const int e0 = 4 * p.lane_in_col, col = col0 + p.col_local;
+    float* sp = state + (((int64_t)row_slot[row] * H + head) * V + col) * DP + e0;
 #pragma unroll
     for (int c = 0; c < CPT; ++c) {
-        const int col = col0 + col_local + c;
-        const bool live = !loader && col < V;
-#pragma unroll
-        for (int u = 0; u < UNITS; ++u) {
-            const float4 x = live ? *reinterpret_cast<const float4*>(
-                                        sp + (int64_t)col * DP + 4 * (lane_in_col + LANES * u))
-                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-            s[c][4 * u] = x.x; s[c][4 * u + 1] = x.y; s[c][4 * u + 2] = x.z; s[c][4 * u + 3] = x.w;
-        }
-    }
-    const int HD = H * D;
-    if (loader)
-        stage_chunk<T, VEC>(stage[0], tid - COMPUTE, rkv, ld, r0, k0, v0, wa, ldwa, HD, head, V, col0,
-                    (int64_t)t0, min(CHUNK, n_new), unit_eps);
-    __syncthreads();
-    int buf = 0;
-    for (int c0 = 0; c0 < n_new; c0 += CHUNK, buf ^= 1) {
-        const int n = min(CHUNK, n_new - c0);
-        if (loader) {
-            if (c0 + CHUNK < n_new)
-                stage_chunk<T, VEC>(stage[buf ^ 1], tid - COMPUTE, rkv, ld, r0, k0, v0, wa, ldwa, HD, head,
-                            V, col0, (int64_t)t0 + c0 + CHUNK, min(CHUNK, n_new - c0 - CHUNK),
-                            unit_eps);
+        p.d[c] = 0.f;
+        if (col + c < V) {
+            fetch<4 * LANES>(p.g[c], sp + c * DP);
         } else {
-            run_chunk(stage[buf], s, n, lane_in_col, col_local, col0, V,
-                      out + (int64_t)(t0 + c0) * H * V + head * V, (int64_t)H * V);
-        }
-        __syncthreads();    // chunk c is done with, chunk c + 1 is staged
-    }
-    if (!loader) {
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) {
-            const int col = col0 + col_local + c;
-            if (col >= V) continue;
-#pragma unroll
-            for (int u = 0; u < UNITS; ++u)
-                *reinterpret_cast<float4*>(sp + (int64_t)col * DP + 4 * (lane_in_col + LANES * u)) =
-                    make_float4(s[c][4 * u], s[c][4 * u + 1], s[c][4 * u + 2], s[c][4 * u + 3]);
+            for (int i = 0; i < 2 * UNITS; ++i) p.g[c][i] = 0;
         }
     }
+#pragma unroll
+    for (int i = 0; i < 2 * UNITS; ++i) p.nak[i] = p.r[i] = 0;
+    const int64_t ld_out = (int64_t)H * V;
+    const int o_col = col0 + p.col_local + p.lane_in_col / SHARE;
+    const bool stores = o_col < V;
+    float* o_row = out + t0 * ld_out + (int64_t)head * V + o_col;    // of token 0
+    f2 s[CPT][2 * UNITS];
+    __syncthreads();            // the first chunk is staged
+    fetch<4 * LANES>(p.k, &stage[0].k[0][e0]);
+    p.state(s);
+    p.begin(s);
+    // (a step gives the read-out of the token before it: the first one's belongs to no token)
+    for (int c0 = 0, buf = 0; c0 < n_new; c0 += CHUNK, buf ^= 1) {
+        const int n = min(CHUNK, n_new - c0);
+        int t = 0;
+#pragma unroll 1
+        for (; t + GROUP <= n; t += GROUP) {
+            float o[GROUP];
+#pragma unroll
+            for (int i = 0; i < GROUP; ++i) o[i] = p.step(stage[buf], t + i);
+            const int first = c0 + t - 1 + share_tokens(o, p.lane_in_col);
+            // (with fewer tokens than lanes, the lanes that hold the same token store the same sum)
+#pragma unroll
+            for (int i = 0; i < KEPT; ++i)
+                if (stores && first + i >= 0) o_row[(first + i) * ld_out] = o[i];
+        }
+#pragma unroll 1
+        for (; t < n; ++t) {
+            float o = p.step(stage[buf], t);
+#pragma unroll
+            for (int sh = SHARE >> 1; sh > 0; sh >>= 1) o += __shfl_xor_sync(0xffffffffu, o, sh);
+            if (stores && c0 + t > 0) o_row[(c0 + t - 1) * ld_out] = o;
+        }
+        if (c0 + CHUNK < n_new) __syncthreads();
+    }
+    p.state(s);
+    float o = p.begin(s);
+#pragma unroll
+    for (int sh = SHARE >> 1; sh > 0; sh >>= 1) o += __shfl_xor_sync(0xffffffffu, o, sh);
+    if (stores) o_row[(n_new - 1) * ld_out] = o;
+#pragma unroll
+    for (int c = 0; c < CPT; ++c)
+        if (col + c < V)
+#pragma unroll
+            for (int i = 0; i < UNITS; ++i)
+                *reinterpret_cast<ulonglong2*>(sp + c * DP + 4 * LANES * i) =
+                    make_ulonglong2(s[c][2 * i], s[c][2 * i + 1]);
 }
 
 }  // namespace sllm
@@ -354,9 +516,14 @@ SLLM_EXPORT int sllm_general_delta(const void* rkv, int64_t ld, int r0, int k0, 
                      !(((uintptr_t)rkv | (uintptr_t)wa) & 15);
     typedef __nv_bfloat16 bf16;
 #define SLLM_GD_LAUNCH(T, VEC)                                                                  \
-    return (int)sllm_launch_pdl(general_delta_kernel<T, VEC>, grid, dim3(THREADS), 0, stream,   \
-                                (const T*)rkv, ld, r0, k0, v0, wa, ldwa, state, row_start,      \
-                                row_slot, out, H, V, unit_eps)
+    do {                                                                                        \
+        const cudaError_t e = cudaFuncSetAttribute(                                             \
+            general_delta_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);   \
+        if (e != cudaSuccess) return (int)e;                                                    \
+        return (int)sllm_launch_pdl(general_delta_kernel<T, VEC>, grid, dim3(THREADS), SMEM,    \
+                                    stream, (const T*)rkv, ld, r0, k0, v0, wa, ldwa, state,     \
+                                    row_start, row_slot, out, H, V, unit_eps);                  \
+    } while (0)
     if (dtype == 0) {
         if (vec) SLLM_GD_LAUNCH(float, true);
         SLLM_GD_LAUNCH(float, false);

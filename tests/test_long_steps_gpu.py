@@ -1,0 +1,57 @@
+"""Kernels for long steps at the edges of their tiles."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _i32(v):
+    return torch.tensor(v, dtype=torch.int32, device=DEV)
+
+
+@pytest.mark.parametrize("D,V", [(64, 64), (64, 20), (128, 33), (16, 70), (33, 5), (200, 9), (300, 3)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_general_delta_chunks(D, V, dtype):
+    """Rows around whole chunks of tokens, in one step and cut in two, against 64 bits."""
+    from scratch_llm_b200.kernels import ops
+    ops.prepare_jobs([ops.general_delta_library(D)], verbose=False)
+    H, lens = 2, [1, 3, 4, 15, 16, 17, 0, 32, 33, 70]
+    g = torch.Generator().manual_seed(D + V)
+    n, DP = sum(lens), ops.general_delta_padded_dim(D)
+    rkv = torch.randn(n, 2 * H * D + H * V, generator=g).to(dtype).to(DEV)
+    wa = torch.cat([torch.rand(n, H * D, generator=g) * 0.45 + 0.55, torch.rand(n, H * D, generator=g)], 1).to(DEV)
+    first = torch.zeros(len(lens), H, V, DP, device=DEV)
+    first[..., :D] = torch.randn(len(lens), H, V, D, generator=g).to(DEV)
+    slots = list(reversed(range(len(lens))))
+
+    def step(state, counts, at):
+        pick = torch.cat([torch.arange(a, a + c) for a, c in zip(at, counts)]).to(DEV)
+        starts = [sum(counts[:i]) for i in range(len(counts) + 1)]
+        out = torch.empty(len(pick), H * V, device=DEV)
+        ops.general_delta(rkv[pick], (0, H * D, 2 * H * D), wa[pick], state, _i32(starts), _i32(slots), out,
+                          len(counts), H, D, V, 1e-6)
+        return pick, out
+
+    at = [sum(lens[:i]) for i in range(len(lens))]
+    whole, cut, o2 = first.clone(), first.clone(), torch.empty(n, H * V, device=DEV)
+    _, o1 = step(whole, lens, at)
+    head = [m * 2 // 5 for m in lens]
+    for counts, begin in ((head, at), ([m - k for m, k in zip(lens, head)], [a + k for a, k in zip(at, head)])):
+        pick, out = step(cut, counts, begin)
+        o2[pick] = out
+
+    r, k, v = rkv.double().split([H * D, H * D, H * V], 1)
+    r, k, v, (w, a) = r.view(n, H, D), k.view(n, H, D), v.view(n, H, V), wa.double().view(n, 2, H, D).unbind(1)
+    u = k / (k.square().sum(-1, keepdim=True) + 1e-6).sqrt()
+    want, state = torch.empty(n, H, V, device=DEV, dtype=torch.float64), first.double().clone()
+    for i, m in enumerate(lens):
+        S = state[slots[i], ..., :D].clone()
+        for t in range(at[i], at[i] + m):
+            S = S * w[t][:, None] - (S @ u[t][..., None]) * (a[t] * u[t])[:, None] + v[t][..., None] * k[t][:, None]
+            want[t] = (S @ r[t][..., None])[..., 0]
+        state[slots[i], ..., :D] = S
+    # decays of at least 0.55: a few tokens' roundings, each a few of 2^-24
+    for got, ref in ((o1, want.flatten(1)), (o2, want.flatten(1)), (whole, state), (cut, state)):
+        assert ((got.double() - ref).norm() / ref.norm()).item() < 1e-6
