@@ -24,9 +24,8 @@
 //
 // Why: a row's tokens in order are a chain of 128 pieces of 16 tokens for 2,048 tokens, 5.9 us each
 // whatever the GPU's width.  In chunks the chain has 32 links of two small products.  2,048 tokens, 16
-// heads of 128 x 128, bfloat16: one decay per head 733 -> 252 us, per channel 666 -> 343 us.  One by one, per head: 56,
-// 89 and 46 us; in a stream, where a kernel's CTAs take the places that the one before it leaves first and wait
-// there, 252.
+// heads of 128 x 128, bfloat16: one decay per head 733 -> 186 us, per channel 666 -> 277 us.  One by one, per
+// head: 56, 89 and 46 us.
 #pragma once
 
 #include <algorithm>
@@ -981,8 +980,12 @@ static inline int launch(const PrepArgs& a, const Scratch& z, float* state, cons
         if (e != cudaSuccess) return (int)e;
         // (rows of at least per_row chunks: this many can have some in the group)
         const int group_rows = std::min(rows, g.count / per_row + 2);
-        e = sllm_launch_pdl(pass_kernel<D>, dim3((a.V + NC - 1) / NC, a.H, group_rows), dim3(2 * D), 0, stream, z, g,
-                            state, a.row_start, row_slot, a.n_rows, a.min_chunked, a.H, a.V);
+        // (an ordinary launch: begun beside prep, its CTAs take the places that prep leaves first, two on some
+        // SMs and none on others, and one row's chain of chunks goes by the slowest: the three kernels took
+        // 256 us so, 186 now, 350 and 277 per channel; four rows of 601 to 1,201 tokens 314 and 303)
+        pass_kernel<D><<<dim3((a.V + NC - 1) / NC, a.H, group_rows), 2 * D, 0, stream>>>(
+            z, g, state, a.row_start, row_slot, a.n_rows, a.min_chunked, a.H, a.V);
+        e = cudaGetLastError();
         if (e != cudaSuccess) return (int)e;
         e = sllm_launch_pdl(out_kernel<D>, dim3((a.V + OUT_COLS - 1) / OUT_COLS, a.H, g.count), dim3(OUT_THREADS),
                             out_smem<D>(), stream, z, g, a.row_start, out, a.n_rows, a.min_chunked, a.H, a.V);
