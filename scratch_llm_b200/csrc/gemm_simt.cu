@@ -7,18 +7,19 @@
 // and N are, so a token's result does not depend on what else is in the batch.
 //
 // Three kernels.  32-bit operands whose rows allow 16-byte requests, by size:
-//   gemm_f32_wide_kernel   tiles of 64 x 64, where those give every SM two
+//   gemm_f32_wide_kernel   tiles of 64 x 64, 64 x 48 or 64 x 32, where those give every SM two
 //   gemm_f32_kernel        smaller tiles behind a ring of cp.async stages: few tokens are bound by the chain
 //                          of steps over k, whose loads the ring keeps ahead of.  Tiles of 32 x 32, and of
 //                          16 x 16 up to 16 tokens.
 // gemm_simt_kernel: every other type and layout (one step of loads, then its arithmetic).
-// us before (all on gemm_simt_kernel) and after, K = 2,048:
-//   1 token    N 3,072: 116 / 25     16,384: 213 / 70     128,256: 1,161 / 419 (2.5 TB/s)
-//   64         134 / 62              236 / 184            1,369 / 1,235
-//   256        214 / 138             701 / 560            5,258 / 4,300
-//   777        497 / 366             2,194 / 1,598
-//   2,048      1,067 / 820           5,337 / 3,790 (36 TF/s)
-// The wide kernel reaches 36 TF/s with one multiply-add an instruction or two (f32x2) alike.
+// us (all on gemm_simt_kernel / with the wide kernel's rows a lane / now), K = 2,048:
+//   1 token    N 3,072: 116 / 25 / 25         16,384: 213 / 70 / 70          128,256: 1,161 / 419 / 419
+//   64         134 / 62 / 62                  236 / 184 / 184                1,369 / 1,235 / 1,235
+//   256        214 / 137 / 124                701 / 560 / -                  5,258 / 4,300 / -
+//   777        497 / 365 / 257                2,194 / 1,598 / -
+//   2,048      1,067 / 820 / -                5,337 / 3,788 / 3,050 (45 TF/s)
+// What bounds the wide kernel now is shared memory: a read of 16 bytes a lane takes four cycles of it
+// whether or not lanes ask for the same, 16 per 64 multiply-adds a lane, as many as the four schedulers have.
 #include "common.cuh"
 
 namespace sllm {
@@ -163,45 +164,56 @@ gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, float*
     }
 }
 
-// The widest tiles: 64 x 64 by 64 threads of 8 x 8 outputs.  A thread requests its row's next 16 elements
-// of X and of W while a step is worked on and stores them [k][row], so that per k four reads of 16
-// bytes feed 64 multiply-adds without a move between registers.
+// The widest tiles: 64 x (8 TN) by 64 threads of 8 x TN outputs, TN = 4, 6 or 8.  Four neighbouring lanes
+// request a row's next 16 elements (64 bytes) while a step is worked on, so that a warp's request touches 8
+// rows (a row a lane: 365 us for 777 tokens by 3,072 in tiles of 64 x 64, 320 so).  They are
+// stored [k][row], so that per k four reads of 16 bytes feed 64 multiply-adds without a move between
+// registers; quad k / 4 of the row's elements stands 8 k / 4 places further (modulo the tile), so that the
+// four lanes of a row store to different banks.
 constexpr int WIDE = 64, WK = 16;
+template <int TN>
 __global__ void __launch_bounds__(WIDE, 6)
 gemm_f32_wide_kernel(const float* __restrict__ X, const float* __restrict__ W, float* __restrict__ Y, int M, int N,
                      int K, int64_t ldx, int64_t ldw, int64_t ldy) {
+    constexpr int COLS = 8 * TN, XN = WIDE / 16, WN = COLS / 16;     // pieces of 16 rows
     __shared__ __align__(16) float xs[2][WK][WIDE];
-    __shared__ __align__(16) float ws[2][WK][WIDE];
+    __shared__ __align__(16) float ws[2][WK][WIDE];     // (rows of 64 places whatever the tile)
     const int tid = threadIdx.x, tx = tid % 8 * 4, ty = tid / 8 * 4;
-    const int bm = blockIdx.y * WIDE, bn = blockIdx.x * WIDE;
+    const int bm = blockIdx.y * WIDE, bn = blockIdx.x * COLS;
+    const int q = tid % 4, lr = tid / 4;                // this thread's quad of a step, and rows lr + 16 i
     // (rows beyond the matrices read the last one again; their outputs are not stored)
-    const float* x = X + (int64_t)min(bm + tid, M - 1) * ldx;
-    const float* w = W + (int64_t)min(bn + tid, N - 1) * ldw;
-    float4 xr[WK / 4], wr[WK / 4];
-    auto request = [&](int k0) {
+    const float* x[XN];
+    const float* w[WN];
 #pragma unroll
-        for (int q = 0; q < WK / 4; ++q) {
-            const int k = k0 + 4 * q;
-            xr[q] = wr[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (k < K) {
-                xr[q] = *reinterpret_cast<const float4*>(x + k);
-                wr[q] = *reinterpret_cast<const float4*>(w + k);
-            }
-        }
+    for (int i = 0; i < XN; ++i) x[i] = X + (int64_t)min(bm + lr + 16 * i, M - 1) * ldx + 4 * q;
+#pragma unroll
+    for (int i = 0; i < WN; ++i) w[i] = W + (int64_t)min(bn + lr + 16 * i, N - 1) * ldw + 4 * q;
+    float4 xr[XN], wr[WN];
+    auto request = [&](int k0) {
+        const bool there = k0 + 4 * q < K;
+#pragma unroll
+        for (int i = 0; i < XN; ++i)
+            xr[i] = there ? *reinterpret_cast<const float4*>(x[i] + k0) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < WN; ++i)
+            wr[i] = there ? *reinterpret_cast<const float4*>(w[i] + k0) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     auto store = [&](int buf) {
 #pragma unroll
-        for (int k = 0; k < WK; ++k) {
-            xs[buf][k][tid] = part(xr[k / 4], k % 4);
-            ws[buf][k][tid] = part(wr[k / 4], k % 4);
-        }
+        for (int i = 0; i < XN; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) xs[buf][4 * q + k][(lr + 16 * i + 8 * q) % WIDE] = part(xr[i], k);
+#pragma unroll
+        for (int i = 0; i < WN; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) ws[buf][4 * q + k][(lr + 16 * i + 8 * q) % WIDE] = part(wr[i], k);
     };
-    // rows ty .. + 3 and 32 + ty .., columns tx .. and 32 + tx ..
-    float acc[8][8];
+    // rows ty .. + 3 and 32 + ty .., columns tx .. and 32 + (TN - 4) / 4 tx ..
+    float acc[8][TN];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
     request(0);
     store(0);
     __syncthreads();
@@ -209,15 +221,21 @@ gemm_f32_wide_kernel(const float* __restrict__ X, const float* __restrict__ W, f
         if (k0 + WK < K) request(k0 + WK);
 #pragma unroll
         for (int k = 0; k < WK; ++k) {
-            float a[8], b[8];
-            *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&xs[buf][k][ty]);
-            *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&xs[buf][k][32 + ty]);
-            *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&ws[buf][k][tx]);
-            *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(&ws[buf][k][32 + tx]);
+            const int shift = 8 * (k / 4);
+            const int a0 = (ty + shift) % WIDE, b0 = (tx + shift) % WIDE;
+            float a[8], b[TN];
+            *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&xs[buf][k][a0]);
+            *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&xs[buf][k][a0 ^ 32]);
+            *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&ws[buf][k][b0]);
+            if constexpr (TN == 8)
+                *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(&ws[buf][k][b0 ^ 32]);
+            if constexpr (TN == 6)
+                *reinterpret_cast<float2*>(b + 4) =
+                    *reinterpret_cast<const float2*>(&ws[buf][k][(32 + tx / 2 + shift) % WIDE]);
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
         if (k0 + WK < K) store(buf ^ 1);
         __syncthreads();
@@ -227,11 +245,21 @@ gemm_f32_wide_kernel(const float* __restrict__ X, const float* __restrict__ W, f
         const int m = bm + ty + i % 4 + i / 4 * 32;
         if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int n = bn + tx + j % 4 + j / 4 * 32;
+        for (int j = 0; j < TN; ++j) {
+            const int n = bn + (j < 4 ? tx + j : 32 + tx * (TN - 4) / 4 + j - 4);
             if (n < N) Y[(int64_t)m * ldy + n] = acc[i][j];
         }
     }
+}
+
+template <int TN>
+static int launch_wide(const float* X, const float* W, float* Y, int M, int N, int K, int64_t ldx, int64_t ldw,
+                       int64_t ldy, cudaStream_t stream) {
+    const dim3 tiles((N + 8 * TN - 1) / (8 * TN), (M + WIDE - 1) / WIDE);
+    if (tiles.y > 65535) return (int)cudaErrorInvalidValue;
+    gemm_f32_wide_kernel<TN><<<tiles, WIDE, 0, stream>>>(X, W, Y, M, N, K, ldx, ldw, ldy);
+    SLLM_LAUNCH_CHECK();
+    return 0;
 }
 
 template <int BM, int BN, int TM, int TN, int BK, int STAGES>
@@ -262,18 +290,34 @@ SLLM_EXPORT int sllm_gemm_simt(const void* X, const void* W, void* Y, int M, int
         !(((uintptr_t)X | (uintptr_t)W) & 15)) {
         const auto x = (const float*)X, w = (const float*)W;
         const auto y = (float*)Y;
-        const int64_t wide = (int64_t)((M + 63) / 64) * ((N + 63) / 64);
         if (M <= 16) return launch_f32<16, 16, 2, 2, 64, 4>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
         int dev = 0, n_sm = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||
             cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             return (int)cudaErrorInvalidDevice;
-        if (wide < 2 * n_sm) return launch_f32<32, 32, 4, 4, 32, 4>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
-        const dim3 tiles((N + WIDE - 1) / WIDE, (M + WIDE - 1) / WIDE);
-        if (tiles.y > 65535) return (int)cudaErrorInvalidValue;
-        gemm_f32_wide_kernel<<<tiles, WIDE, 0, stream>>>(x, w, y, M, N, K, ldx, ldw, ldy);
-        SLLM_LAUNCH_CHECK();
-        return 0;
+        // Few tiles even of the narrowest width (of the widest, where half of a tile's rows stay empty): the
+        // ring's small tiles (128 tokens by 3,072: 93 us, 103 with tiles 32 wide; 256 tokens: 137 and, 48
+        // wide, 124).
+        const int narrow = M <= 32 ? 64 : 32;
+        if ((int64_t)((M + 63) / 64) * ((N + narrow - 1) / narrow) < 2 * n_sm)
+            return launch_f32<32, 32, 4, 4, 32, 4>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
+        // The tiles' width by what the SM with the most tiles takes: rounds of six tiles (twelve warps, three a
+        // scheduler); one or two tiles take half a full round, three or four 0.73 of it, latencies being
+        // hidden less.  A narrow tile reads more of shared memory per multiply-add.  Measured over sizes of 33
+        // to 2,048 tokens by 2,048 to 128,256, this is within 3 % of the best width (the widest always: 777
+        // tokens by 3,072 320 us, 257 so).
+        static const int tail[6] = {0, 15, 15, 22, 22, 30};
+        int best = 0;
+        int64_t cost = 0;
+        for (int tn = 8; tn >= 4; tn -= 2) {
+            const int64_t tiles = (int64_t)((M + 63) / 64) * ((N + 8 * tn - 1) / (8 * tn));
+            const int64_t per_sm = (tiles + n_sm - 1) / n_sm;
+            const int64_t now = (per_sm / 6 * 30 + tail[per_sm % 6]) * (tn == 8 ? 80 : tn == 6 ? 62 : 48);
+            if (!best || now < cost) { best = tn; cost = now; }
+        }
+        if (best == 8) return launch_wide<8>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
+        if (best == 6) return launch_wide<6>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
+        return launch_wide<4>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
     }
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return (int)cudaErrorInvalidValue;

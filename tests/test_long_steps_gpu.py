@@ -55,3 +55,15 @@ def test_general_delta_chunks(D, V, dtype):
     # decays of at least 0.55: a few tokens' roundings, each a few of 2^-24
     for got, ref in ((o1, want.flatten(1)), (o2, want.flatten(1)), (whole, state), (cut, state)):
         assert ((got.double() - ref).norm() / ref.norm()).item() < 1e-6
+
+
+@pytest.mark.parametrize("m,n,k", [(777, 3072, 64), (65, 20480, 20), (640, 1000, 36), (2000, 700, 8), (64, 64 * 300, 12),
+                                   (513, 6144, 8), (300, 3072, 24), (256, 3072, 16), (33, 9500, 20)])
+def test_32bit_product_widths_of_tiles(m, n, k):
+    """Every width of the tiles gives the bits of the plainest kernel (rows that allow no 16-byte requests)."""
+    from scratch_llm_b200.kernels import ops
+    g = torch.Generator().manual_seed(m + n)
+    x, w = torch.randn(m, k, generator=g).to(DEV), torch.randn(n, k, generator=g).to(DEV)
+    odd = torch.empty(m, k + 1, device=DEV)[:, :k].copy_(x)
+    got = ops.gemm_simt(x, w, torch.full((m, n), float("nan"), device=DEV))
+    assert torch.equal(got, ops.gemm_simt(odd, w, torch.empty(m, n, device=DEV)))
