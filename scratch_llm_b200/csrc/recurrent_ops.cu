@@ -315,6 +315,88 @@ head_norm_gate_vec_kernel(const float* __restrict__ o, const T* __restrict__ gat
     store_few<4>(out + n * ldo + (int64_t)head * V + e, v);
 }
 
+// The second product of a low-rank pair in long steps: hidden [N, R] by w2t [R, C] for 64 tokens and 128
+// channels a CTA of 128 threads.  Up to 64 rows of both operands stand in shared memory, r by r; a thread
+// has 8 x 8 outputs, so that four reads of 16 bytes feed 64 multiply-adds (a channel a thread for 8 tokens: as
+// many reads of the weights from L2 as multiply-adds / 8).  Per output one chain over r in ascending order, as
+// in the kernel for few tokens.
+constexpr int LR_TOKENS = 64, LR_COLS = 128, LR_THREADS = 128, LR_STEP = 64;
+struct __align__(16) LowrankTile {
+    float w[LR_STEP][LR_COLS];
+    float h[LR_STEP][LR_TOKENS];     // (quad r / 4 stands r / 4 * 4 places further, modulo the row)
+};
+__device__ __forceinline__ void lowrank_weights(LowrankTile& s, const float* __restrict__ w2t, int R, int C,
+                                                int r0, int c0) {
+#pragma unroll 8
+    for (int i = threadIdx.x; i < LR_STEP * LR_COLS / 4; i += LR_THREADS) {
+        const int r = i / (LR_COLS / 4), c = i % (LR_COLS / 4) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r0 + r < R && c0 + c < C) v = *reinterpret_cast<const float4*>(w2t + (int64_t)(r0 + r) * C + c0 + c);
+        *reinterpret_cast<float4*>(&s.w[r][c]) = v;
+    }
+}
+__device__ __forceinline__ void lowrank_hidden(LowrankTile& s, const float* __restrict__ hidden, int64_t ldp,
+                                               int R, int r0, int nt, bool vec, bool tanh_in) {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < LR_TOKENS * LR_STEP / 4; i += LR_THREADS) {
+        // (8 quads of 4 tokens a warp: the stores below meet 32 banks)
+        const int q = i % 8 + i / (8 * LR_TOKENS) * 8, t = i / 8 % LR_TOKENS, r = r0 + 4 * q;
+        const float* p = hidden + (int64_t)t * ldp + r;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (t < nt) {
+            if (vec && r + 4 <= R) {
+                *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (r + k < R) v[k] = p[k];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            s.h[4 * q + k][(t + 4 * q) % LR_TOKENS] = tanh_in ? tanhf(v[k]) : v[k];
+    }
+}
+// acc = hidden w2t of the CTA's tile.  Thread (ty, tx): tokens 4 ty .. and 32 + 4 ty .., channels 4 tx ..
+// and 64 + 4 tx ...  The first rows of w2t are there already (they may be requested before the wait for the
+// kernels ahead).
+__device__ __forceinline__ void lowrank_tile(LowrankTile& s, float (&acc)[8][8], const float* __restrict__ hidden,
+                                             int64_t ldp, const float* __restrict__ w2t, int R, int C, int c0,
+                                             int nt, bool vec, bool tanh_in) {
+    const int tx = threadIdx.x % 16 * 4, ty = threadIdx.x / 16 * 4;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int r0 = 0; r0 < R; r0 += LR_STEP) {
+        if (r0) {
+            __syncthreads();
+            lowrank_weights(s, w2t, R, C, r0, c0);
+        }
+        lowrank_hidden(s, hidden, ldp, R, r0, nt, vec, tanh_in);
+        __syncthreads();
+        const int steps = min(LR_STEP, R - r0);
+        for (int q = 0; q < (steps + 3) / 4; ++q) {      // (rows from R on are zeros)
+            const int t0 = (ty + 4 * q) % LR_TOKENS;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int r = 4 * q + k;
+                float a[8], b[8];
+                *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&s.h[r][t0]);
+                *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&s.h[r][t0 ^ 32]);
+                *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&s.w[r][tx]);
+                *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(&s.w[r][64 + tx]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(b[j], a[i], acc[i][j]);
+            }
+        }
+    }
+}
+__device__ __forceinline__ int lowrank_token(int i) { return threadIdx.x / 16 * 4 + i % 4 + i / 4 * 32; }
+__device__ __forceinline__ int lowrank_col(int half) { return threadIdx.x % 16 * 4 + half * 64; }
+
 // Decays and removal rates of a delta-rule mixer whose decay comes through a low-rank pair of
 // matrices.  pre: float32 [N, ldp] holds the removal rates' inputs in columns [0, C) and the
 // low-rank hidden values in columns [C, C + R).  w2t: float32 [R, C] (the second matrix,
@@ -324,6 +406,8 @@ head_norm_gate_vec_kernel(const float* __restrict__ o, const T* __restrict__ gat
 // All in 32-bit; the sum runs over r in ascending order for every token, whatever the batch.
 // grid (ceil(C / 256), ceil(N / LOWRANK_TOKENS)); shared: LOWRANK_TOKENS * R floats.
 constexpr int LOWRANK_TOKENS = 8;
+__device__ __forceinline__ float rate_of(float z) { return 1.0f / (1.0f + expf(-z)); }
+__device__ __forceinline__ float decay_of(float z, float scale) { return expf(-scale * rate_of(z)); }
 __global__ void __launch_bounds__(256)
 lowrank_decay_kernel(const float* __restrict__ pre, int64_t ldp, const float* __restrict__ w2t,
                      const float* __restrict__ w0, const float* __restrict__ a_bias,
@@ -365,9 +449,52 @@ lowrank_decay_kernel(const float* __restrict__ pre, int64_t ldp, const float* __
     for (int t = 0; t < LOWRANK_TOKENS; ++t) {
         if (t < nt) {
             const int64_t n = n0 + t;
-            const float sg = 1.0f / (1.0f + expf(-(acc[t] + b0)));
-            out[n * 2 * C + c] = expf(-decay_scale * sg);
-            out[n * 2 * C + C + c] = 1.0f / (1.0f + expf(-(pre[n * ldp + c] + ab)));
+            out[n * 2 * C + c] = decay_of(acc[t] + b0, decay_scale);
+            out[n * 2 * C + C + c] = rate_of(pre[n * ldp + c] + ab);
+        }
+    }
+}
+
+// The same for long steps (C % 4 == 0, every operand on a 16-byte boundary).  C 2,048, R 64, us with 8 tokens a
+// CTA and so: 512 tokens 16.9 / 18.1, 2,048 43.8 / 29.1, 3,001 64 / 52; C 4,096, R 128, 4,096 tokens 265 / 184.
+// The exponentials and divisions of the two outputs take as long as the products.
+// grid (ceil(C / LR_COLS), ceil(N / LR_TOKENS)).
+constexpr int LR_MIN_TOKENS = 1024;
+__global__ void __launch_bounds__(LR_THREADS, 4)
+lowrank_decay_tile_kernel(const float* __restrict__ pre, int64_t ldp, const float* __restrict__ w2t,
+                          const float* __restrict__ w0, const float* __restrict__ a_bias,
+                          float decay_scale, float* __restrict__ out, int N, int C, int R, bool vec) {
+    __shared__ LowrankTile s;
+    const int n0 = blockIdx.y * LR_TOKENS, nt = min(LR_TOKENS, N - n0), c0 = blockIdx.x * LR_COLS;
+    lowrank_weights(s, w2t, R, C, 0, c0);
+    pdl_wait();
+    pdl_trigger();
+    const float* rows = pre + n0 * ldp;
+    float acc[8][8];
+    lowrank_tile(s, acc, rows + C, ldp, w2t, R, C, c0, nt, vec, true);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int c = c0 + lowrank_col(half);
+        if (c >= C) continue;
+        const float4 b0 = *reinterpret_cast<const float4*>(w0 + c), ab = *reinterpret_cast<const float4*>(a_bias + c);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int t = lowrank_token(i);
+            if (t >= nt) continue;
+            const float* x = acc[i] + 4 * half;
+            float p[4];
+            if (vec) {
+                *reinterpret_cast<float4*>(p) = *reinterpret_cast<const float4*>(rows + t * ldp + c);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) p[k] = rows[t * ldp + c + k];
+            }
+            float* o = out + (int64_t)(n0 + t) * 2 * C + c;
+            *reinterpret_cast<float4*>(o) =
+                make_float4(decay_of(x[0] + b0.x, decay_scale), decay_of(x[1] + b0.y, decay_scale),
+                            decay_of(x[2] + b0.z, decay_scale), decay_of(x[3] + b0.w, decay_scale));
+            *reinterpret_cast<float4*>(o + C) =
+                make_float4(rate_of(p[0] + ab.x), rate_of(p[1] + ab.y), rate_of(p[2] + ab.z), rate_of(p[3] + ab.w));
         }
     }
 }
@@ -824,6 +951,14 @@ SLLM_EXPORT int sllm_lowrank_decay(const float* pre, int64_t ldp, const float* w
                                    float* out, int n_tokens, int C, int R, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (C <= 0 || R <= 0 || R > 1024 || ldp < C + R) return (int)cudaErrorInvalidValue;
+    if (n_tokens >= LR_MIN_TOKENS && C % 4 == 0 &&
+        !(((uintptr_t)w2t | (uintptr_t)w0 | (uintptr_t)a_bias | (uintptr_t)out) & 15)) {
+        const dim3 tiles((C + LR_COLS - 1) / LR_COLS, (n_tokens + LR_TOKENS - 1) / LR_TOKENS);
+        if (tiles.y <= 65535)
+            return (int)sllm_launch_pdl(lowrank_decay_tile_kernel, tiles, dim3(LR_THREADS), 0, stream, pre, ldp,
+                                        w2t, w0, a_bias, decay_scale, out, n_tokens, C, R,
+                                        ldp % 4 == 0 && !((uintptr_t)pre & 15));
+    }
     dim3 grid((C + 255) / 256, (n_tokens + LOWRANK_TOKENS - 1) / LOWRANK_TOKENS);
     if (grid.y > 65535) return (int)cudaErrorInvalidValue;
     lowrank_decay_kernel<<<grid, 256, LOWRANK_TOKENS * R * sizeof(float), stream>>>(

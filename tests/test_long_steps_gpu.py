@@ -67,3 +67,25 @@ def test_32bit_product_widths_of_tiles(m, n, k):
     odd = torch.empty(m, k + 1, device=DEV)[:, :k].copy_(x)
     got = ops.gemm_simt(x, w, torch.full((m, n), float("nan"), device=DEV))
     assert torch.equal(got, ops.gemm_simt(odd, w, torch.empty(m, n, device=DEV)))
+
+
+@pytest.mark.parametrize("n,c,r,ld", [(1024, 128, 64, 0), (1025, 132, 5, 0), (1087, 4, 130, 0), (1030, 260, 64, 1)])
+def test_decays_of_a_low_rank_pair(n, c, r, ld):
+    """One chain of multiply-adds over the rank per output: a token's bits are those of a step of few tokens.
+    ``ld``: hidden values that allow no reads of 16 bytes."""
+    from scratch_llm_b200.kernels import ops
+    g = torch.Generator().manual_seed(n + c + r)
+    pre = torch.randn(n, c + r + ld, generator=g).to(DEV)[:, :c + r]
+    w2t = (torch.randn(r, c, generator=g) * r ** -0.5).to(DEV)
+    w0, ab = torch.randn(c, generator=g).to(DEV), torch.randn(c, generator=g).to(DEV)
+
+    def decays(pre):
+        return ops.lowrank_decay(pre, w2t, w0, ab, 0.6, torch.empty(len(pre), 2 * c, device=DEV))
+
+    got = decays(pre)
+    assert torch.equal(got, torch.cat([decays(pre[t:t + 200]) for t in range(0, n, 200)]))
+    x = pre.double()
+    want = torch.cat([torch.exp(-0.6 * torch.sigmoid(torch.tanh(x[:, c:]) @ w2t.double() + w0)),
+                      torch.sigmoid(x[:, :c] + ab)], 1)
+    # 32-bit sums of r products: r / 2 roundings of the largest partial sum at most
+    assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -24 * max(8, r / 2)
