@@ -1,4 +1,4 @@
-"""Kernels for long steps at the edges of their tiles."""
+"""Kernels for long steps at the edges of their tiles, edges of the nucleus."""
 
 import pytest
 import torch
@@ -89,3 +89,33 @@ def test_decays_of_a_low_rank_pair(n, c, r, ld):
                       torch.sigmoid(x[:, :c] + ab)], 1)
     # 32-bit sums of r products: r / 2 roundings of the largest partial sum at most
     assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -24 * max(8, r / 2)
+
+
+@pytest.mark.parametrize("V", [8192, 8200, 50001, 190001])
+def test_nucleus_of_flat_and_steep_rows(V):
+    """The search that starts from a histogram, on rows whose mass lies in one of its buckets, in the last one, or
+    on one value: the kept set is the smallest one above top_p that 64 bits give, up to the value at its edge."""
+    from scratch_llm_b200.kernels import ops
+    g = torch.Generator().manual_seed(V)
+    flat, two, steep = torch.zeros(V), torch.zeros(V), torch.arange(V) * -1e-3
+    two[::7] = 3.0
+    one = torch.full((V,), -60.0)
+    one[V // 2] = 0.0
+    rows = torch.stack([x for x in (flat, two, steep, one, torch.randn(V, generator=g) * 8) for _ in range(5)])
+    tops = torch.tensor([1e-6, 0.37, 0.9, 0.9998, 0.99999] * 5)
+    n = len(rows)
+    probs, out = torch.empty(n, V, device=DEV), torch.empty(n, dtype=torch.int32, device=DEV)
+    seed = torch.arange(n, device=DEV)
+    ops.sample(rows.to(DEV), out, torch.ones(n, device=DEV), tops.to(DEV), seed, seed, probs_out=probs)
+    kept = probs.cpu() > 0
+    assert kept[torch.arange(n), out.cpu().long()].all()
+    for r in range(n):
+        p = torch.softmax(rows[r].double(), -1)
+        k = kept[r]
+        # everything above the smallest kept value is kept, and that value is where the mass passes top_p
+        edge = p[k].min()
+        clear = (p / edge - 1).abs() > 1e-5
+        assert (k == (p >= edge))[clear].all()
+        slack = 1e-5 + float(edge)               # (32-bit sums; a value on the edge)
+        above, upto = float(p[p > edge * (1 + 1e-5)].sum()), float(p[p >= edge * (1 - 1e-5)].sum())
+        assert above <= float(tops[r]) + slack and upto >= float(tops[r]) - slack
