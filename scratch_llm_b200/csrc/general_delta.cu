@@ -54,21 +54,11 @@ constexpr int DP = padded(D);                 // padded key size
 static_assert(DP <= 512, "key sizes up to 512");
 constexpr int EPL = DP <= 128 ? 4 : DP / 32;  // elements of a column per lane
 constexpr int LANES = DP / EPL;
-constexpr int CPT = EPL == 4 ? 4 : 16 / EPL;       // columns per compute thread
 constexpr int COMPUTE = 128, LOADERS = 128, THREADS = COMPUTE + LOADERS;
-constexpr int COLS = COMPUTE / LANES * CPT;   // columns of S per CTA
 constexpr int UNITS = EPL / 4;                // float4 units per lane
 // tokens per chunk: two buffers of four vectors of DP floats per token, within 64 KB
 constexpr int CHUNK = DP <= 128 ? 16 : 2048 / DP;
 static_assert(CHUNK >= 2, "chunk too small");
-
-struct __align__(16) Staged {
-    float k[CHUNK + 1][DP];     // (the last: the first key of the chunk that follows)
-    float r[CHUNK][DP], w[CHUNK][DP], nak[CHUNK][DP];   // nak: -a * k
-    float v[CHUNK][COLS];
-    float2 ic[CHUNK];           // i_t = 1 / (|k_t|^2 + eps), and i_t (k_t . nak_{t-1})
-};
-constexpr int SMEM = 2 * (int)sizeof(Staged);
 
 // two 32-bit numbers in one register pair
 typedef unsigned long long f2;
@@ -100,19 +90,35 @@ __device__ __forceinline__ void loaders_sync() {
 __device__ __forceinline__ float4 load4(const float* p) {
     return *reinterpret_cast<const float4*>(p);
 }
-__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
-    const uint2 r = *reinterpret_cast<const uint2*>(p);
+// Four elements as they lie in memory, and as numbers.
+template <typename T> struct Four;
+template <> struct Four<float> { typedef float4 Raw; };
+template <> struct Four<__nv_bfloat16> { typedef uint2 Raw; };
+__device__ __forceinline__ float4 numbers(const float4& r) { return r; }
+__device__ __forceinline__ float4 numbers(const uint2& r) {
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
     return make_float4(__low2float(h[0]), __high2float(h[0]), __low2float(h[1]), __high2float(h[1]));
 }
 
-constexpr int QUADS = CHUNK * DP / 4;                       // units of 4 elements in a chunk
-constexpr int QPT = (QUADS + LOADERS - 1) / LOADERS;        // of which a loader thread takes
-constexpr int VPT = (CHUNK * COLS + LOADERS - 1) / LOADERS; // values that a loader thread takes
-constexpr int APT = (DP / 4 + LOADERS - 1) / LOADERS;       // units of the key after the chunk
+// The rule for threads with slices of CPT columns: 4, or 2 where that still leaves the launch within one CTA an
+// SM (half of each token's work a warp, twice the CTAs).
+template <int CPT> struct Rule {
+static constexpr int COLS = COMPUTE / LANES * CPT;   // columns of S per CTA
+struct alignas(16) Staged {
+    float k[CHUNK + 1][DP];     // (the last: the first key of the chunk that follows)
+    float r[CHUNK][DP], w[CHUNK][DP], nak[CHUNK][DP];   // nak: -a * k
+    float v[CHUNK][COLS];
+    float2 ic[CHUNK];           // i_t = 1 / (|k_t|^2 + eps), and i_t (k_t . nak_{t-1})
+};
+static constexpr int SMEM = 2 * (int)sizeof(Staged);
+
+static constexpr int QUADS = CHUNK * DP / 4;                       // units of 4 elements in a chunk
+static constexpr int QPT = (QUADS + LOADERS - 1) / LOADERS;        // of which a loader thread takes
+static constexpr int VPT = (CHUNK * COLS + LOADERS - 1) / LOADERS; // values that a loader thread takes
+static constexpr int APT = (DP / 4 + LOADERS - 1) / LOADERS;       // units of the key after the chunk
 // a token's units fit the lanes of one warp (and LOADERS is a multiple of them): its sums are
 // formed from registers
-constexpr bool FUSED = DP / 4 <= 32;
+static constexpr bool FUSED = DP / 4 <= 32;
 
 template <typename T> struct Operands {
     const T* __restrict__ rkv;
@@ -122,43 +128,49 @@ template <typename T> struct Operands {
     float unit_eps;
 };
 
-// What a loader thread has requested of a chunk.  VEC: every row of every operand starts on a
-// multiple of 4 elements, so four elements come per load.
-template <bool VEC> struct Request {
-    float4 r[VEC ? QPT : 1], k[VEC ? QPT : 1], w[VEC ? QPT : 1], a[VEC ? QPT : 1];
-    float4 k_after[VEC ? APT : 1];
-    float v[VPT];
+// What a loader thread has requested of a chunk, as it lies in memory: nothing waits for a request
+// before the chunk is staged.  VEC: every row of every operand starts on a multiple of 4 elements,
+// so four elements come per load.
+template <typename T, bool VEC> struct Request {
+    typename Four<T>::Raw r[VEC ? QPT : 1], k[VEC ? QPT : 1], k_after[VEC ? APT : 1];
+    float4 w[VEC ? QPT : 1], a[VEC ? QPT : 1];
+    T v[VPT];
 };
 
 template <typename T, bool VEC>
-__device__ __forceinline__ void request_chunk(Request<VEC>& q, int lt, const Operands<T>& x,
+static __device__ __forceinline__ void request_chunk(Request<T, VEC>& q, int lt, const Operands<T>& x,
                                               int64_t tok0, int n, bool more) {
+    typedef typename Four<T>::Raw Raw;
     if (VEC) {
 #pragma unroll
         for (int j = 0; j < APT; ++j) {
             const int e = (lt + j * LOADERS) * 4;
-            q.k_after[j] = more && e < D ? load4(x.rkv + (tok0 + n) * x.ld + x.k0 + x.head * D + e)
-                                         : make_float4(0.f, 0.f, 0.f, 0.f);
+            q.k_after[j] = Raw();
+            if (more && e < D)
+                q.k_after[j] = *reinterpret_cast<const Raw*>(x.rkv + (tok0 + n) * x.ld + x.k0 + x.head * D + e);
         }
 #pragma unroll
         for (int j = 0; j < QPT; ++j) {
             const int i = lt + j * LOADERS;
             const int t = i / (DP / 4), e = (i - t * (DP / 4)) * 4;
-            q.r[j] = q.k[j] = q.w[j] = q.a[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            q.r[j] = q.k[j] = Raw();
+            q.w[j] = q.a[j] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (i < QUADS && t < n && e < D) {
-                const int64_t tok = tok0 + t;
-                q.r[j] = load4(x.rkv + tok * x.ld + x.r0 + x.head * D + e);
-                q.k[j] = load4(x.rkv + tok * x.ld + x.k0 + x.head * D + e);
-                q.w[j] = load4(x.wa + tok * x.ldwa + x.head * D + e);
-                q.a[j] = load4(x.wa + tok * x.ldwa + x.HD + x.head * D + e);
+                const T* row = x.rkv + (tok0 + t) * x.ld + x.head * D + e;
+                const float* wa = x.wa + (tok0 + t) * x.ldwa + x.head * D + e;
+                q.r[j] = *reinterpret_cast<const Raw*>(row + x.r0);
+                q.k[j] = *reinterpret_cast<const Raw*>(row + x.k0);
+                q.w[j] = load4(wa);
+                q.a[j] = load4(wa + x.HD);
             }
         }
     }
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
         const int i = lt + j * LOADERS, t = i / COLS, c = i - t * COLS;
-        q.v[j] = t < n && x.col0 + c < x.V
-            ? to_float(x.rkv[(tok0 + t) * x.ld + x.v0 + x.head * x.V + x.col0 + c]) : 0.f;
+        q.v[j] = T(0.f);
+        if (t < n && x.col0 + c < x.V)
+            q.v[j] = x.rkv[(tok0 + t) * x.ld + x.v0 + x.head * x.V + x.col0 + c];
     }
 }
 
@@ -166,30 +178,31 @@ __device__ __forceinline__ void request_chunk(Request<VEC>& q, int lt, const Ope
 // request what is left of the `left` tokens after it.  `before`: the row of nak of the token before
 // tok0, or null.
 template <typename T, bool VEC>
-__device__ __forceinline__ void stage_chunk(Staged& st, Request<VEC>& q, int lt,
+static __device__ __forceinline__ void stage_chunk(Staged& st, Request<T, VEC>& q, int lt,
                                             const Operands<T>& x, const float* before,
                                             int64_t tok0, int n, int left) {
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
         const int i = lt + j * LOADERS, t = i / COLS, c = i - t * COLS;
-        if (i < CHUNK * COLS) st.v[t][c] = q.v[j];
+        if (i < CHUNK * COLS) st.v[t][c] = to_float(q.v[j]);
     }
     if (VEC) {
 #pragma unroll
         for (int j = 0; j < APT; ++j)
             if ((lt + j * LOADERS) * 4 < DP)
-                *reinterpret_cast<float4*>(&st.k[CHUNK][(lt + j * LOADERS) * 4]) = q.k_after[j];
+                *reinterpret_cast<float4*>(&st.k[CHUNK][(lt + j * LOADERS) * 4]) =
+                    numbers(q.k_after[j]);
 #pragma unroll
         for (int j = 0; j < QPT; ++j) {
             const int i = lt + j * LOADERS;
             const int t = i / (DP / 4), e = (i - t * (DP / 4)) * 4;
             if (i < QUADS && t < n) {
-                *reinterpret_cast<float4*>(&st.r[t][e]) = q.r[j];
-                *reinterpret_cast<float4*>(&st.k[t][e]) = q.k[j];
+                const float4 k = numbers(q.k[j]), a = q.a[j];
+                *reinterpret_cast<float4*>(&st.r[t][e]) = numbers(q.r[j]);
+                *reinterpret_cast<float4*>(&st.k[t][e]) = k;
                 *reinterpret_cast<float4*>(&st.w[t][e]) = q.w[j];
                 *reinterpret_cast<float4*>(&st.nak[t][e]) =
-                    make_float4(-q.a[j].x * q.k[j].x, -q.a[j].y * q.k[j].y,
-                                -q.a[j].z * q.k[j].z, -q.a[j].w * q.k[j].w);
+                    make_float4(-a.x * k.x, -a.y * k.y, -a.z * k.z, -a.w * k.w);
             }
         }
     } else {
@@ -218,7 +231,7 @@ __device__ __forceinline__ void stage_chunk(Staged& st, Request<VEC>& q, int lt,
             const int i = lt + j * LOADERS;
             const int t = i / (DP / 4), e = (i - t * (DP / 4)) * 4;
             const float* p = t == 0 ? before : st.nak[t < CHUNK ? t - 1 : 0];
-            const float4 k = q.k[j];
+            const float4 k = numbers(q.k[j]);
             ss[j] = fmaf(k.x, k.x, fmaf(k.y, k.y, fmaf(k.z, k.z, k.w * k.w)));
             c[j] = 0.f;
             if (i < QUADS && t < n && p) {
@@ -258,14 +271,14 @@ __device__ __forceinline__ void stage_chunk(Staged& st, Request<VEC>& q, int lt,
     if (left > 0) request_chunk<T, VEC>(q, lt, x, tok0 + n, min(CHUNK, left), left > CHUNK);
 }
 
-constexpr int SHARE = LANES / CPT;          // lanes that go on with the same column
+static constexpr int SHARE = LANES / CPT;          // lanes that go on with the same column
 static_assert(SHARE >= 1 && CPT <= 4, "no more columns a thread than lanes a column");
 
 // Sums across a column's lanes begin with CPT values per lane (one per column) that become one: each
 // exchange halves the columns that a lane goes on with.  A lane goes on with column
 // lane_in_col / SHARE.  One exchange of x's `have` pairs:
 template <int HAVE>
-__device__ __forceinline__ void share(float (&x)[CPT], int lane_in_col) {
+static __device__ __forceinline__ void share(float (&x)[CPT], int lane_in_col) {
     constexpr int SH = LANES / CPT * HAVE;
     const bool upper = lane_in_col & SH;
 #pragma unroll
@@ -275,7 +288,7 @@ __device__ __forceinline__ void share(float (&x)[CPT], int lane_in_col) {
     }
 }
 // ... of two sums at a time, until one value of each is left.
-__device__ __forceinline__ void share_both(float (&x)[CPT], float (&y)[CPT], int lane_in_col) {
+static __device__ __forceinline__ void share_both(float (&x)[CPT], float (&y)[CPT], int lane_in_col) {
     if constexpr (CPT >= 4) {
         share<2>(x, lane_in_col);
         share<2>(y, lane_in_col);
@@ -286,7 +299,7 @@ __device__ __forceinline__ void share_both(float (&x)[CPT], float (&y)[CPT], int
     }
 }
 
-template <int N> __device__ __forceinline__ void fetch(f2 (&x)[2 * UNITS], const float* row) {
+template <int N> static __device__ __forceinline__ void fetch(f2 (&x)[2 * UNITS], const float* row) {
 #pragma unroll
     for (int i = 0; i < UNITS; ++i) {
         const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(row + N * i);
@@ -294,7 +307,7 @@ template <int N> __device__ __forceinline__ void fetch(f2 (&x)[2 * UNITS], const
         x[2 * i + 1] = y.y;
     }
 }
-__device__ __forceinline__ float dot(const f2 (&x)[2 * UNITS], const f2 (&y)[2 * UNITS]) {
+static __device__ __forceinline__ float dot(const f2 (&x)[2 * UNITS], const f2 (&y)[2 * UNITS]) {
     f2 acc = mul2(x[0], y[0]);
 #pragma unroll
     for (int i = 1; i < 2 * UNITS; ++i) acc = fma2(x[i], y[i], acc);
@@ -379,9 +392,9 @@ struct Pipe {
 
 // Sums of GROUP tokens' read-outs across the lanes of a column: each exchange halves the tokens
 // that a lane goes on with; a lane ends with the tokens first .. of its column.
-constexpr int GROUP = CHUNK < 4 ? CHUNK : 4;
-constexpr int KEPT = GROUP >= SHARE ? GROUP / SHARE : 1;
-__device__ __forceinline__ int share_tokens(float (&o)[GROUP], int lane_in_col) {
+static constexpr int GROUP = CHUNK < 4 ? CHUNK : 4;
+static constexpr int KEPT = GROUP >= SHARE ? GROUP / SHARE : 1;
+static __device__ __forceinline__ int share_tokens(float (&o)[GROUP], int lane_in_col) {
     int first = 0, have = GROUP;
 #pragma unroll
     for (int sh = SHARE >> 1; sh > 0; sh >>= 1) {
@@ -401,10 +414,11 @@ __device__ __forceinline__ int share_tokens(float (&o)[GROUP], int lane_in_col) 
     }
     return first;
 }
+};
 
 // rkv: [N, ld] with the heads' r at column r0, k at k0, v at v0 (each heads x D or heads x V);
 // wa: float32 [N, ldwa] with the decays at column 0 and the removal rates at column H * D.
-template <typename T, bool VEC>
+template <typename T, bool VEC, int CPT>
 __global__ void __launch_bounds__(THREADS, DP <= 128 ? 2 : 1)
 general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int v0,
                      const float* __restrict__ wa, int64_t ldwa, float* __restrict__ state,
@@ -413,26 +427,29 @@ general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int 
     pdl_wait();
     pdl_trigger();
     extern __shared__ __align__(16) uint8_t smem[];
+    typedef Rule<CPT> R;
+    typedef typename R::Staged Staged;
+    constexpr int SHARE = R::SHARE, GROUP = R::GROUP;
     Staged* stage = reinterpret_cast<Staged*>(smem);
     const int row = blockIdx.z, head = blockIdx.y;
     const int t0 = row_start[row], n_new = row_start[row + 1] - t0;
     if (n_new <= 0) return;
     const int tid = threadIdx.x;
     const bool loader = tid >= COMPUTE;
-    const int col0 = blockIdx.x * COLS;
+    const int col0 = blockIdx.x * R::COLS;
     if (loader) {
         const int lt = tid - COMPUTE;
-        const Operands<T> x{rkv, wa, ld, ldwa, r0, k0, v0, H * D, head, V, col0, unit_eps};
-        Request<VEC> q;
-        request_chunk<T, VEC>(q, lt, x, t0, min(CHUNK, n_new), n_new > CHUNK);
+        const typename R::template Operands<T> x{rkv, wa, ld, ldwa, r0, k0, v0, H * D, head, V, col0, unit_eps};
+        typename R::template Request<T, VEC> q;
+        R::template request_chunk<T, VEC>(q, lt, x, t0, min(CHUNK, n_new), n_new > CHUNK);
         for (int c0 = 0, buf = 0; c0 < n_new; c0 += CHUNK, buf ^= 1) {
-            stage_chunk<T, VEC>(stage[buf], q, lt, x, c0 ? stage[buf ^ 1].nak[CHUNK - 1] : nullptr,
+            R::template stage_chunk<T, VEC>(stage[buf], q, lt, x, c0 ? stage[buf ^ 1].nak[CHUNK - 1] : nullptr,
                                 (int64_t)t0 + c0, min(CHUNK, n_new - c0), n_new - c0 - CHUNK);
             __syncthreads();    // chunk c is staged, chunk c - 1 is done with
         }
         return;
     }
-    Pipe p;
+    typename R::Pipe p;
     p.lane_in_col = tid % LANES;
     p.col_local = tid / LANES * CPT;
     const int e0 = 4 * p.lane_in_col, col = col0 + p.col_local;
@@ -441,7 +458,7 @@ general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int 
     for (int c = 0; c < CPT; ++c) {
         p.d[c] = 0.f;
         if (col + c < V) {
-            fetch<4 * LANES>(p.g[c], sp + c * DP);
+            R::template fetch<4 * LANES>(p.g[c], sp + c * DP);
         } else {
 #pragma unroll
             for (int i = 0; i < 2 * UNITS; ++i) p.g[c][i] = 0;
@@ -455,7 +472,7 @@ general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int 
     float* o_row = out + t0 * ld_out + (int64_t)head * V + o_col;    // of token 0
     f2 s[CPT][2 * UNITS];
     __syncthreads();            // the first chunk is staged
-    fetch<4 * LANES>(p.k, &stage[0].k[0][e0]);
+    R::template fetch<4 * LANES>(p.k, &stage[0].k[0][e0]);
     p.state(s);
     p.begin(s);
     // (a step gives the read-out of the token before it: the first one's belongs to no token)
@@ -467,10 +484,10 @@ general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int 
             float o[GROUP];
 #pragma unroll
             for (int i = 0; i < GROUP; ++i) o[i] = p.step(stage[buf], t + i);
-            const int first = c0 + t - 1 + share_tokens(o, p.lane_in_col);
+            const int first = c0 + t - 1 + R::share_tokens(o, p.lane_in_col);
             // (with fewer tokens than lanes, the lanes that hold the same token store the same sum)
 #pragma unroll
-            for (int i = 0; i < KEPT; ++i)
+            for (int i = 0; i < R::KEPT; ++i)
                 if (stores && first + i >= 0) o_row[(first + i) * ld_out] = o[i];
         }
 #pragma unroll 1
@@ -496,6 +513,32 @@ general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int 
                     make_ulonglong2(s[c][2 * i], s[c][2 * i + 1]);
 }
 
+template <typename T, bool VEC, int CPT, typename... Args>
+static int launch_rule(int n_rows, int H, int V, cudaStream_t stream, Args... args) {
+    constexpr int SMEM = Rule<CPT>::SMEM, COLS = Rule<CPT>::COLS;
+    const auto kernel = general_delta_kernel<T, VEC, CPT>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e != cudaSuccess) return (int)e;
+    return (int)sllm_launch_pdl(kernel, dim3((V + COLS - 1) / COLS, H, n_rows), dim3(THREADS), SMEM, stream,
+                                args...);
+}
+
+// Two columns a thread while the launch has at most one CTA an SM even so: 32 heads of 64 x 64, a row of 2,048
+// tokens 300 us with four, 238 with two; 100 tokens 18 and 15; beyond, the SMs' throughput counts (64 heads, a
+// row of 2,400: 353 and 404).
+template <typename T, bool VEC>
+static int launch(const T* rkv, int64_t ld, int r0, int k0, int v0, const float* wa, int64_t ldwa, float* state,
+                  const int* row_start, const int* row_slot, float* out, int n_rows, int H, int V, float unit_eps,
+                  int n_sm, cudaStream_t stream) {
+    constexpr int MOST = EPL == 4 ? 4 : 16 / EPL, FEW = EPL == 4 ? 2 : MOST;
+    const int64_t ctas = (int64_t)((V + Rule<FEW>::COLS - 1) / Rule<FEW>::COLS) * H * n_rows;
+    if (FEW != MOST && ctas <= n_sm)
+        return launch_rule<T, VEC, FEW>(n_rows, H, V, stream, rkv, ld, r0, k0, v0, wa, ldwa, state, row_start,
+                                        row_slot, out, H, V, unit_eps);
+    return launch_rule<T, VEC, MOST>(n_rows, H, V, stream, rkv, ld, r0, k0, v0, wa, ldwa, state, row_start,
+                                     row_slot, out, H, V, unit_eps);
+}
+
 }  // namespace sllm
 
 using namespace sllm;
@@ -510,20 +553,17 @@ SLLM_EXPORT int sllm_general_delta(const void* rkv, int64_t ld, int r0, int k0, 
                                    cudaStream_t stream) {
     if (n_rows <= 0) return 0;
     if (H <= 0 || V <= 0 || H > 65535 || n_rows > 65535) return (int)cudaErrorInvalidValue;
-    dim3 grid((V + COLS - 1) / COLS, H, n_rows);
     // four elements per load where every operand's rows start on multiples of four elements
     const bool vec = D % 4 == 0 && ld % 4 == 0 && r0 % 4 == 0 && k0 % 4 == 0 && ldwa % 4 == 0 &&
                      !(((uintptr_t)rkv | (uintptr_t)wa) & 15);
     typedef __nv_bfloat16 bf16;
+    int dev = 0, n_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return (int)cudaErrorInvalidDevice;
 #define SLLM_GD_LAUNCH(T, VEC)                                                                  \
-    do {                                                                                        \
-        const cudaError_t e = cudaFuncSetAttribute(                                             \
-            general_delta_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);   \
-        if (e != cudaSuccess) return (int)e;                                                    \
-        return (int)sllm_launch_pdl(general_delta_kernel<T, VEC>, grid, dim3(THREADS), SMEM,    \
-                                    stream, (const T*)rkv, ld, r0, k0, v0, wa, ldwa, state,     \
-                                    row_start, row_slot, out, H, V, unit_eps);                  \
-    } while (0)
+    return launch<T, VEC>((const T*)rkv, ld, r0, k0, v0, wa, ldwa, state, row_start, row_slot,  \
+                          out, n_rows, H, V, unit_eps, n_sm, stream)
     if (dtype == 0) {
         if (vec) SLLM_GD_LAUNCH(float, true);
         SLLM_GD_LAUNCH(float, false);
