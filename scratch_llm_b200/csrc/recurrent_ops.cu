@@ -7,7 +7,8 @@
 //           A request's last K - 1 inputs are carried in its state slot, state[slot, s, c] with
 //           s = K - 2 the most recent, so that a row may bring any number of tokens per step.
 //   update: the state after the row's tokens (a launch of its own: the convolution of a row's
-//           first tokens reads the old state while its last tokens would overwrite it).
+//           first tokens reads the old state while its last tokens would overwrite it; rows of one
+//           token each do both in one pass).
 //   read-out: out[t, h, :] = o[t, h, :] / sqrt(mean(o[t, h, :]^2) + eps) * gain * silu(gate[t, h, :]),
 //           optionally with o divided first by max(|den[t, h]|, floor[t, h]) + 1e-6; or, with the
 //           gate ahead of the norm, y = o * silu(gate), each of several equal parts of y over
@@ -242,6 +243,65 @@ __global__ void conv_state_update_kernel(const T* __restrict__ x, int64_t ldx, i
         st[(int64_t)s * C + c] = src < K - 1 ? st[(int64_t)src * C + c]
                                              : x[(int64_t)(t0 + src - (K - 1)) * ldx + c];
     }
+}
+
+// Steps whose rows bring one token each (decoding): the convolution and the carried inputs after it in
+// one pass, a thread has W consecutive channels of a token and is the only one that reads or writes them.  The
+// arithmetic and its order are conv_silu_kernel's.  What such a step takes is its launches: 48 rows of 8,192
+// channels took 5.0 + 4.8 us as two, and eight steps of a layer of that size 856 us, 803 so.
+// TAPS: K, or 0 for any.  taps: [C, K], or its transpose where W > 1 (W = 8: 16-byte accesses, bfloat16).
+template <typename T, int W, int TAPS>
+__global__ void __launch_bounds__(128)
+conv_step_kernel(const T* __restrict__ x, int64_t ldx, const float* __restrict__ taps,
+                 const float* __restrict__ bias, int k_taps, T* state,
+                 const int* __restrict__ token_row, const int* __restrict__ row_slot,
+                 T* __restrict__ out, int C) {
+    struct alignas(W * sizeof(T)) Piece { T e[W]; };
+    pdl_wait();
+    pdl_trigger();
+    const int K = TAPS ? TAPS : k_taps;
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * W;
+    const int64_t n = blockIdx.y;
+    if (c >= C) return;
+    const int r = token_row[n];
+    Piece result;
+    if (r < 0) {
+#pragma unroll
+        for (int w = 0; w < W; ++w) result.e[w] = from_float<T>(0.f);
+        *reinterpret_cast<Piece*>(out + n * C + c) = result;
+        return;
+    }
+    T* st = state + (int64_t)row_slot[r] * (K - 1) * C + c;
+    const Piece now = *reinterpret_cast<const Piece*>(x + n * ldx + c);
+    float acc[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) acc[w] = bias ? bias[c + w] : 0.f;
+    auto add = [&](const Piece& in, int j) {
+#pragma unroll
+        for (int w = 0; w < W; ++w)
+            acc[w] = fmaf(W > 1 ? taps[(int64_t)j * C + c + w] : taps[(int64_t)c * K + j], to_float(in.e[w]), acc[w]);
+    };
+    if (TAPS > 1) {
+        Piece past[TAPS > 1 ? TAPS - 1 : 1];
+#pragma unroll
+        for (int j = 0; j < TAPS - 1; ++j) past[j] = *reinterpret_cast<const Piece*>(st + (int64_t)j * C);
+#pragma unroll
+        for (int j = 0; j < TAPS - 1; ++j) {
+            add(past[j], j);
+            *reinterpret_cast<Piece*>(st + (int64_t)j * C) = j < TAPS - 2 ? past[j + 1 < TAPS - 1 ? j + 1 : 0] : now;
+        }
+    } else {
+        for (int j = 0; j < K - 1; ++j) {
+            const Piece in = *reinterpret_cast<const Piece*>(st + (int64_t)j * C);
+            add(in, j);
+            if (j > 0) *reinterpret_cast<Piece*>(st + (int64_t)(j - 1) * C) = in;
+        }
+        if (K > 1) *reinterpret_cast<Piece*>(st + (int64_t)(K - 2) * C) = now;
+    }
+    add(now, K - 1);
+#pragma unroll
+    for (int w = 0; w < W; ++w) result.e[w] = from_float<T>(acc[w] * sigmoid_of<T>(acc[w]));
+    *reinterpret_cast<Piece*>(out + n * C + c) = result;
 }
 
 // grid (tokens, ceil(H / 4)); one warp per (token, head), or with WIDE (long heads) grid (tokens,
@@ -879,6 +939,30 @@ SLLM_EXPORT int sllm_conv_silu(const void* x, int64_t ldx, const float* taps,
         return (int)cudaErrorInvalidValue;
     SLLM_LAUNCH_CHECK();
     return 0;
+}
+
+// sllm_conv_silu and sllm_conv_state_update of a step whose rows bring at most one token each.
+SLLM_EXPORT int sllm_conv_step(const void* x, int64_t ldx, const float* taps, const float* taps_t,
+                               const float* bias, int K, void* state, const int* token_row,
+                               const int* row_slot, void* out, int C, int n_tokens, int dtype,
+                               cudaStream_t stream) {
+    if (n_tokens <= 0) return 0;
+    if (C <= 0 || K < 1 || K > CONV_MAX_TAPS || ldx < C || n_tokens > 65535 || dtype < 0 || dtype > 1)
+        return (int)cudaErrorInvalidValue;
+    typedef __nv_bfloat16 bf16;
+    if (dtype == 1 && taps_t != nullptr && C % 8 == 0 && ldx % 8 == 0 &&
+        !(((uintptr_t)x | (uintptr_t)state | (uintptr_t)out | (uintptr_t)taps_t) & 15)) {
+        const auto kernel = K == 4 ? conv_step_kernel<bf16, 8, 4> : conv_step_kernel<bf16, 8, 0>;
+        return (int)sllm_launch_pdl(kernel, dim3((C / 8 + 127) / 128, n_tokens), dim3(128), 0, stream,
+                                    (const bf16*)x, ldx, taps_t, bias, K, (bf16*)state, token_row, row_slot,
+                                    (bf16*)out, C);
+    }
+    const dim3 grid((C + 127) / 128, n_tokens);
+    if (dtype == 1)
+        return (int)sllm_launch_pdl(conv_step_kernel<bf16, 1, 0>, grid, dim3(128), 0, stream, (const bf16*)x, ldx,
+                                    taps, bias, K, (bf16*)state, token_row, row_slot, (bf16*)out, C);
+    return (int)sllm_launch_pdl(conv_step_kernel<float, 1, 0>, grid, dim3(128), 0, stream, (const float*)x, ldx,
+                                taps, bias, K, (float*)state, token_row, row_slot, (float*)out, C);
 }
 
 SLLM_EXPORT int sllm_conv_state_update(const void* x, int64_t ldx, int K, void* state,

@@ -1146,12 +1146,13 @@ def qk_norm_kv_write(x: torch.Tensor, positions: torch.Tensor, token_row: torch.
 def conv_silu(x: torch.Tensor, taps: torch.Tensor, state: torch.Tensor | None,
               token_row: torch.Tensor, row_start: torch.Tensor, row_slot: torch.Tensor,
               out: torch.Tensor, taps_t: torch.Tensor | None = None,
-              bias: torch.Tensor | None = None) -> torch.Tensor:
+              bias: torch.Tensor | None = None, update: bool = False) -> torch.Tensor:
     """Short causal convolution over time and silu on the first C columns of ``x`` [N, >= C]:
     ``taps`` float32 [C, K] (the last tap is the current token's), ``state`` [slots, K - 1, C]
     the inputs carried from earlier steps (None when K is 1), ``out`` [N, C].  ``taps_t``: the
     taps' transpose [K, C] (contiguous), which lets bfloat16 rows of whole 16 bytes take the
-    kernel with 16-byte accesses.  ``bias`` (float32 [C]) is added before silu."""
+    kernel with 16-byte accesses.  ``bias`` (float32 [C]) is added before silu.  ``update``: no row
+    brings more than one token, and :func:`conv_state_update` is done in the same pass."""
     _need(x, None, "x", contiguous=False)
     _need(taps, torch.float32, "taps")
     if bias is not None:
@@ -1174,6 +1175,12 @@ def conv_silu(x: torch.Tensor, taps: torch.Tensor, state: torch.Tensor | None,
         _need(taps_t, torch.float32, "taps_t")
         if taps_t.shape != (k, c):
             raise KernelError("taps_t must be the transpose of taps")
+    if update:
+        _check(_core("sllm_recurrent_ops").sllm_conv_step(
+            _ptr(x), c_int64(x.stride(0)), _ptr(taps), _ptr(taps_t), _ptr(bias), c_int(k),
+            _ptr(state if k > 1 else None), _ptr(token_row), _ptr(row_slot), _ptr(out), c_int(c),
+            c_int(x.shape[0]), c_int(_code(x.dtype)), _stream()), "conv_silu")
+        return out
     _check(_core("sllm_recurrent_ops").sllm_conv_silu(
         _ptr(x), c_int64(x.stride(0)), _ptr(taps), _ptr(taps_t), _ptr(bias), c_int(k),
         _ptr(state if k > 1 else None),

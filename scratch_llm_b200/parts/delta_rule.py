@@ -153,9 +153,10 @@ class GatedDeltaRule(Mixer):
         proj = self.proj(x)                                   # [N, C + H V]
         ab = self.ab(x, out_dtype=torch.float32)              # [N, 2 H]: gates in 32-bit
         act = torch.empty((n, C), dtype=proj.dtype, device=proj.device)
+        single = write and batch.n_multi == 0                 # (rows of one token: one pass)
         ops.conv_silu(proj, self.taps, carried, batch.token_row, batch.row_start, batch.row_slot,
-                      act, self.taps_t)
-        if write:
+                      act, self.taps_t, update=single)
+        if write and not single:
             ops.conv_state_update(proj, K, carried, batch.row_start, batch.row_slot, batch.n_rows)
         if not write:
             raise NotImplementedError("a run that only reads another run's recurrent state")

@@ -115,9 +115,10 @@ class StateSpace(Mixer):
         dt = self.dt(x, out_dtype=torch.float32)                   # [N, H]
         act = torch.empty((n, C), dtype=proj.dtype, device=proj.device)
         ops.conv_silu(proj, self.taps, carried, batch.token_row, batch.row_start, batch.row_slot,
-                      act, self.taps_t, bias=self.conv_bias)
-        ops.conv_state_update(proj, self.conv_taps, carried, batch.row_start, batch.row_slot,
-                              batch.n_rows)
+                      act, self.taps_t, bias=self.conv_bias, update=batch.n_multi == 0)
+        if batch.n_multi:
+            ops.conv_state_update(proj, self.conv_taps, carried, batch.row_start, batch.row_slot,
+                                  batch.n_rows)
         gates = torch.empty((2, n, H), dtype=torch.float32, device=proj.device)
         ops.ssd_gates(dt, self.dt_bias, self.a_log, gates[0], gates[1])
         # (padding tokens belong to no row: their read-out stays zero)

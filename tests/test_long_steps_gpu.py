@@ -1,4 +1,4 @@
-"""Kernels for long steps at the edges of their tiles, edges of the nucleus."""
+"""Kernels for long steps at the edges of their tiles, edges of the nucleus, steps of single tokens in one pass."""
 
 import pytest
 import torch
@@ -119,3 +119,25 @@ def test_nucleus_of_flat_and_steep_rows(V):
         slack = 1e-5 + float(edge)               # (32-bit sums; a value on the edge)
         above, upto = float(p[p > edge * (1 + 1e-5)].sum()), float(p[p >= edge * (1 - 1e-5)].sum())
         assert above <= float(tops[r]) + slack and upto >= float(tops[r]) - slack
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("C,taps", [(1032, 4), (7, 4), (24, 2), (16, 1), (128, 6)])
+def test_convolution_and_carried_inputs_in_one_pass(dtype, C, taps):
+    """Rows of one token (one of them padding, one row without tokens): the bits of the two passes."""
+    from scratch_llm_b200.kernels import ops
+    g = torch.Generator().manual_seed(C + taps)
+    x = torch.randn(5, C + 8, generator=g).to(dtype).to(DEV)
+    w, bias = torch.randn(C, taps, generator=g).to(DEV), torch.randn(C, generator=g).to(DEV)
+    state = torch.randn(6, max(taps - 1, 1), C, generator=g).to(dtype).to(DEV)
+    token_row, row_start, row_slot = _i32([0, 2, 3, 4, -1]), _i32([0, 1, 1, 2, 3, 4]), _i32([3, 2, 0, 5, 1])
+    outs = []
+    for update in (False, True):
+        st = state.clone()
+        out = torch.full((5, C), float("nan"), dtype=dtype, device=DEV)
+        ops.conv_silu(x, w, st if taps > 1 else None, token_row, row_start, row_slot, out, w.t().contiguous(),
+                      bias, update=update)
+        if not update:
+            ops.conv_state_update(x, taps, st, row_start, row_slot, 5)
+        outs.append((out, st))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
