@@ -514,13 +514,16 @@ general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int 
 }
 
 template <typename T, bool VEC, int CPT, typename... Args>
-static int launch_rule(int n_rows, int H, int V, cudaStream_t stream, Args... args) {
+static int launch_rule(int n_rows, int H, int V, bool beside, cudaStream_t stream, Args... args) {
     constexpr int SMEM = Rule<CPT>::SMEM, COLS = Rule<CPT>::COLS;
     const auto kernel = general_delta_kernel<T, VEC, CPT>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return (int)e;
-    return (int)sllm_launch_pdl(kernel, dim3((V + COLS - 1) / COLS, H, n_rows), dim3(THREADS), SMEM, stream,
-                                args...);
+    const dim3 grid((V + COLS - 1) / COLS, H, n_rows);
+    if (beside) return (int)sllm_launch_pdl(kernel, grid, dim3(THREADS), SMEM, stream, args...);
+    kernel<<<grid, THREADS, SMEM, stream>>>(args...);
+    SLLM_LAUNCH_CHECK();
+    return 0;
 }
 
 // Two columns a thread while the launch has at most one CTA an SM even so: 32 heads of 64 x 64, a row of 2,048
@@ -529,13 +532,13 @@ static int launch_rule(int n_rows, int H, int V, cudaStream_t stream, Args... ar
 template <typename T, bool VEC>
 static int launch(const T* rkv, int64_t ld, int r0, int k0, int v0, const float* wa, int64_t ldwa, float* state,
                   const int* row_start, const int* row_slot, float* out, int n_rows, int H, int V, float unit_eps,
-                  int n_sm, cudaStream_t stream) {
+                  int n_sm, bool beside, cudaStream_t stream) {
     constexpr int MOST = EPL == 4 ? 4 : 16 / EPL, FEW = EPL == 4 ? 2 : MOST;
     const int64_t ctas = (int64_t)((V + Rule<FEW>::COLS - 1) / Rule<FEW>::COLS) * H * n_rows;
     if (FEW != MOST && ctas <= n_sm)
-        return launch_rule<T, VEC, FEW>(n_rows, H, V, stream, rkv, ld, r0, k0, v0, wa, ldwa, state, row_start,
+        return launch_rule<T, VEC, FEW>(n_rows, H, V, beside, stream, rkv, ld, r0, k0, v0, wa, ldwa, state, row_start,
                                         row_slot, out, H, V, unit_eps);
-    return launch_rule<T, VEC, MOST>(n_rows, H, V, stream, rkv, ld, r0, k0, v0, wa, ldwa, state, row_start,
+    return launch_rule<T, VEC, MOST>(n_rows, H, V, beside, stream, rkv, ld, r0, k0, v0, wa, ldwa, state, row_start,
                                      row_slot, out, H, V, unit_eps);
 }
 
@@ -545,11 +548,13 @@ using namespace sllm;
 
 SLLM_EXPORT int sllm_general_delta_padded_dim() { return DP; }
 
-// dtype of rkv: 0 = float32, 1 = bfloat16.
+// dtype of rkv: 0 = float32, 1 = bfloat16.  n_tokens: of all rows.  Steps of single tokens start beside the kernel
+// before them; longer rows do not: their CTAs would take the places that come free first, two on some SMs, and
+// the launch goes by the slowest (a layer of 32 heads of 64 x 64 and 2,048 tokens: 483 us, 387 so).
 SLLM_EXPORT int sllm_general_delta(const void* rkv, int64_t ld, int r0, int k0, int v0,
                                    const float* wa, int64_t ldwa, float* state,
                                    const int* row_start, const int* row_slot, float* out,
-                                   int n_rows, int H, int V, float unit_eps, int dtype,
+                                   int n_rows, int n_tokens, int H, int V, float unit_eps, int dtype,
                                    cudaStream_t stream) {
     if (n_rows <= 0) return 0;
     if (H <= 0 || V <= 0 || H > 65535 || n_rows > 65535) return (int)cudaErrorInvalidValue;
@@ -557,13 +562,14 @@ SLLM_EXPORT int sllm_general_delta(const void* rkv, int64_t ld, int r0, int k0, 
     const bool vec = D % 4 == 0 && ld % 4 == 0 && r0 % 4 == 0 && k0 % 4 == 0 && ldwa % 4 == 0 &&
                      !(((uintptr_t)rkv | (uintptr_t)wa) & 15);
     typedef __nv_bfloat16 bf16;
+    const bool beside = n_tokens <= n_rows;
     int dev = 0, n_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return (int)cudaErrorInvalidDevice;
 #define SLLM_GD_LAUNCH(T, VEC)                                                                  \
     return launch<T, VEC>((const T*)rkv, ld, r0, k0, v0, wa, ldwa, state, row_start, row_slot,  \
-                          out, n_rows, H, V, unit_eps, n_sm, stream)
+                          out, n_rows, H, V, unit_eps, n_sm, beside, stream)
     if (dtype == 0) {
         if (vec) SLLM_GD_LAUNCH(float, true);
         SLLM_GD_LAUNCH(float, false);

@@ -1292,7 +1292,7 @@ def general_delta(rkv: torch.Tensor, cols: tuple[int, int, int], wa: torch.Tenso
     _check(_load(*general_delta_library(key_dim)).sllm_general_delta(
         _ptr(rkv), c_int64(rkv.stride(0)), c_int(r0), c_int(k0), c_int(v0), _ptr(wa),
         c_int64(wa.stride(0)), _ptr(state), _ptr(row_start), _ptr(row_slot), _ptr(out),
-        c_int(n_rows), c_int(n_heads), c_int(value_dim), c_float(unit_eps),
+        c_int(n_rows), c_int(n), c_int(n_heads), c_int(value_dim), c_float(unit_eps),
         c_int(_code(rkv.dtype)), _stream()), "general_delta")
     return out
 
