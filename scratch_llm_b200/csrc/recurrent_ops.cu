@@ -454,8 +454,20 @@ __device__ __forceinline__ void lowrank_tile(LowrankTile& s, float (&acc)[8][8],
         }
     }
 }
-__device__ __forceinline__ int lowrank_token(int i) { return threadIdx.x / 16 * 4 + i % 4 + i / 4 * 32; }
-__device__ __forceinline__ int lowrank_col(int half) { return threadIdx.x % 16 * 4 + half * 64; }
+// The sums move to where the weights stood, [LR_TOKENS][LR_COLS], so that what follows them is a loop over
+// quads: unrolled over a thread's 64 sums its code no longer fits the instruction caches.
+__device__ __forceinline__ void lowrank_sums(LowrankTile& s, const float (&acc)[8][8]) {
+    static_assert(LR_TOKENS == LR_STEP, "the sums of a tile take the weights' place");
+    const int tx = threadIdx.x % 16 * 4, ty = threadIdx.x / 16 * 4;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+            *reinterpret_cast<float4*>(&s.w[ty + i % 4 + i / 4 * 32][tx + 64 * half]) =
+                *reinterpret_cast<const float4*>(acc[i] + 4 * half);
+    __syncthreads();
+}
 
 // Decays and removal rates of a delta-rule mixer whose decay comes through a low-rank pair of
 // matrices.  pre: float32 [N, ldp] holds the removal rates' inputs in columns [0, C) and the
@@ -516,10 +528,10 @@ lowrank_decay_kernel(const float* __restrict__ pre, int64_t ldp, const float* __
 }
 
 // The same for long steps (C % 4 == 0, every operand on a 16-byte boundary).  C 2,048, R 64, us with 8 tokens a
-// CTA and so: 512 tokens 16.9 / 18.1, 2,048 43.8 / 29.1, 3,001 64 / 52; C 4,096, R 128, 4,096 tokens 265 / 184.
-// The exponentials and divisions of the two outputs take as long as the products.
+// CTA and so: 256 tokens 12.5 / 16.9, 512 16.8 / 17.0, 1,024 25.2 / 20.9, 2,048 43.5 / 28.6, 3,001 64 / 52; C 4,096,
+// R 128, 4,096 tokens 265 / 195.  The exponentials and divisions of the two outputs take as long as the products.
 // grid (ceil(C / LR_COLS), ceil(N / LR_TOKENS)).
-constexpr int LR_MIN_TOKENS = 1024;
+constexpr int LR_MIN_TOKENS = 512;
 __global__ void __launch_bounds__(LR_THREADS, 4)
 lowrank_decay_tile_kernel(const float* __restrict__ pre, int64_t ldp, const float* __restrict__ w2t,
                           const float* __restrict__ w0, const float* __restrict__ a_bias,
@@ -532,30 +544,26 @@ lowrank_decay_tile_kernel(const float* __restrict__ pre, int64_t ldp, const floa
     const float* rows = pre + n0 * ldp;
     float acc[8][8];
     lowrank_tile(s, acc, rows + C, ldp, w2t, R, C, c0, nt, vec, true);
+    lowrank_sums(s, acc);
+    const int c = c0 + threadIdx.x % 32 * 4;
+    if (c >= C) return;
+    const float4 b0 = *reinterpret_cast<const float4*>(w0 + c), ab = *reinterpret_cast<const float4*>(a_bias + c);
+#pragma unroll 2
+    for (int t = threadIdx.x / 32; t < nt; t += LR_THREADS / 32) {
+        const float4 x = *reinterpret_cast<const float4*>(&s.w[t][c - c0]);
+        float p[4];
+        if (vec) {
+            *reinterpret_cast<float4*>(p) = *reinterpret_cast<const float4*>(rows + t * ldp + c);
+        } else {
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const int c = c0 + lowrank_col(half);
-        if (c >= C) continue;
-        const float4 b0 = *reinterpret_cast<const float4*>(w0 + c), ab = *reinterpret_cast<const float4*>(a_bias + c);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int t = lowrank_token(i);
-            if (t >= nt) continue;
-            const float* x = acc[i] + 4 * half;
-            float p[4];
-            if (vec) {
-                *reinterpret_cast<float4*>(p) = *reinterpret_cast<const float4*>(rows + t * ldp + c);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) p[k] = rows[t * ldp + c + k];
-            }
-            float* o = out + (int64_t)(n0 + t) * 2 * C + c;
-            *reinterpret_cast<float4*>(o) =
-                make_float4(decay_of(x[0] + b0.x, decay_scale), decay_of(x[1] + b0.y, decay_scale),
-                            decay_of(x[2] + b0.z, decay_scale), decay_of(x[3] + b0.w, decay_scale));
-            *reinterpret_cast<float4*>(o + C) =
-                make_float4(rate_of(p[0] + ab.x), rate_of(p[1] + ab.y), rate_of(p[2] + ab.z), rate_of(p[3] + ab.w));
+            for (int k = 0; k < 4; ++k) p[k] = rows[t * ldp + c + k];
         }
+        float* o = out + (int64_t)(n0 + t) * 2 * C + c;
+        *reinterpret_cast<float4*>(o) =
+            make_float4(decay_of(x.x + b0.x, decay_scale), decay_of(x.y + b0.y, decay_scale),
+                        decay_of(x.z + b0.z, decay_scale), decay_of(x.w + b0.w, decay_scale));
+        *reinterpret_cast<float4*>(o + C) =
+            make_float4(rate_of(p[0] + ab.x), rate_of(p[1] + ab.y), rate_of(p[2] + ab.z), rate_of(p[3] + ab.w));
     }
 }
 
@@ -580,6 +588,53 @@ struct ExpandJob {
     float rate; int tanh_in;
     void* out; int out_bf16; int C; int R;
 };
+
+// What follows the product; rate: exp(rate_log) of mode 1.
+__device__ __forceinline__ float expanded(float z, int mode, float rate) {
+    if (mode == 1) return -rate * (z > 20.f ? z : log1pf(expf(z)));
+    if (mode == 2) return fmaxf(rate * (fminf(z, 0.f) - log1pf(expf(-fabsf(z)))), LOG_DECAY_FLOOR);
+    if (mode == 3) return fmaxf(-expf(z), LOG_DECAY_FLOOR);
+    return z;
+}
+
+// Long steps (C % 4 == 0, weights and outputs on 16-byte boundaries), in the tiles of the decays above.  Two
+// products of C 2,048, R 64, us with 16 tokens a CTA and so: 256 tokens 18.5 / 18.3, 512 25.6 / 21.7, 1,024 40.0 /
+// 26.1, 2,048 65.2 / 50.5, 3,001 89 / 68 (84 with what follows the products unrolled over a thread's 64 sums).
+constexpr int LR_MIN_EXPANDED = 256;
+// grid (blocks of LR_COLS channels of both jobs, ceil(N / LR_TOKENS)).
+__global__ void __launch_bounds__(LR_THREADS, 4)
+lowrank_expand_tile_kernel(const float* __restrict__ pre, int64_t ldp, const ExpandJob j0,
+                           const ExpandJob j1, int blocks0, int N, bool vec) {
+    __shared__ LowrankTile s;
+    const bool second = (int)blockIdx.x >= blocks0;
+    const ExpandJob& j = second ? j1 : j0;
+    const int n0 = blockIdx.y * LR_TOKENS, nt = min(LR_TOKENS, N - n0);
+    const int c0 = ((int)blockIdx.x - (second ? blocks0 : 0)) * LR_COLS, C = j.C;
+    lowrank_weights(s, j.w2t, j.R, C, 0, c0);
+    pdl_wait();
+    pdl_trigger();
+    float acc[8][8];
+    lowrank_tile(s, acc, pre + n0 * ldp + j.col0, ldp, j.w2t, j.R, C, c0, nt, vec && j.col0 % 4 == 0, j.tanh_in);
+    lowrank_sums(s, acc);
+    const int c = c0 + threadIdx.x % 32 * 4;
+    if (c >= C) return;
+    float b0[4], rate[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        b0[k] = j.bias ? j.bias[c + k] : 0.f;
+        rate[k] = j.mode == 1 ? expf(j.rate_log[(c + k) / j.per_rate]) : j.rate;
+    }
+#pragma unroll 2
+    for (int t = threadIdx.x / 32; t < nt; t += LR_THREADS / 32) {
+        float z[4];
+        *reinterpret_cast<float4*>(z) = *reinterpret_cast<const float4*>(&s.w[t][c - c0]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) z[k] = expanded(z[k] + b0[k], j.mode, rate[k]);
+        const int64_t at = (int64_t)(n0 + t) * C + c;
+        if (j.out_bf16) store_few<4>(reinterpret_cast<__nv_bfloat16*>(j.out) + at, z);
+        else store_few<4>(reinterpret_cast<float*>(j.out) + at, z);
+    }
+}
 
 // A CTA has TOKENS tokens and CH channels a thread (2: C even); a thread's next AHEAD rows of
 // weights are in flight while it works on the ones before, the first ones already before the kernel
@@ -642,19 +697,14 @@ lowrank_expand_kernel(const float* __restrict__ pre, int64_t ldp, const ExpandJo
 #pragma unroll
     for (int h = 0; h < CH; ++h) {
         b0[h] = j.bias ? j.bias[c + h] : 0.f;
-        rate[h] = j.mode == 1 ? expf(j.rate_log[(c + h) / j.per_rate]) : 0.f;
+        rate[h] = j.mode == 1 ? expf(j.rate_log[(c + h) / j.per_rate]) : j.rate;
     }
 #pragma unroll
     for (int t = 0; t < TOKENS; ++t) {
         if (t >= nt) break;
 #pragma unroll
         for (int h = 0; h < CH; ++h) {
-            float z = acc[t][h] + b0[h];
-            if (j.mode == 1) z = -rate[h] * (z > 20.f ? z : log1pf(expf(z)));
-            else if (j.mode == 2)
-                z = fmaxf(j.rate * (fminf(z, 0.f) - log1pf(expf(-fabsf(z)))), LOG_DECAY_FLOOR);
-            else if (j.mode == 3) z = fmaxf(-expf(z), LOG_DECAY_FLOOR);
-            acc[t][h] = z;
+            acc[t][h] = expanded(acc[t][h] + b0[h], j.mode, rate[h]);
         }
         const int64_t at = (int64_t)(n0 + t) * C + c;
         if (j.out_bf16) {
@@ -1077,7 +1127,18 @@ SLLM_EXPORT int sllm_lowrank_expand(const float* pre, int64_t ldp, int n_jobs, c
         max_r = R[i] > max_r ? R[i] : max_r;
         max_c = C[i] > max_c ? C[i] : max_c;
     }
-    // steps of few tokens: narrow CTAs, so that the channels spread over more SMs; long steps: more
+    bool tiled = n_tokens >= LR_MIN_EXPANDED;
+    for (int i = 0; i < n_jobs; ++i)
+        tiled = tiled && C[i] % 4 == 0 && !(((uintptr_t)w2t[i] | (uintptr_t)out[i]) & 15);
+    if (tiled && (n_tokens + LR_TOKENS - 1) / LR_TOKENS <= 65535) {
+        const int blocks0 = (j[0].C + LR_COLS - 1) / LR_COLS;
+        const int blocks1 = n_jobs > 1 ? (j[1].C + LR_COLS - 1) / LR_COLS : 0;
+        return (int)sllm_launch_pdl(lowrank_expand_tile_kernel,
+                                    dim3(blocks0 + blocks1, (n_tokens + LR_TOKENS - 1) / LR_TOKENS), dim3(LR_THREADS),
+                                    0, stream, pre, ldp, j[0], j[1], blocks0, n_tokens,
+                                    ldp % 4 == 0 && !((uintptr_t)pre & 15));
+    }
+    // steps of few tokens: narrow CTAs, so that the channels spread over more SMs; long steps of other sizes: more
     // tokens a CTA and two channels a thread, so that the weights are read less often
     bool wide = n_tokens >= 512;
     for (int i = 0; i < n_jobs; ++i)

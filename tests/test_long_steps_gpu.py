@@ -69,26 +69,34 @@ def test_32bit_product_widths_of_tiles(m, n, k):
     assert torch.equal(got, ops.gemm_simt(odd, w, torch.empty(m, n, device=DEV)))
 
 
-@pytest.mark.parametrize("n,c,r,ld", [(1024, 128, 64, 0), (1025, 132, 5, 0), (1087, 4, 130, 0), (1030, 260, 64, 1)])
-def test_decays_of_a_low_rank_pair(n, c, r, ld):
+@pytest.mark.parametrize("n,c,r,ld", [(512, 128, 64, 0), (577, 132, 5, 0), (575, 4, 130, 0), (530, 260, 64, 1),
+                                       (257, 256, 33, 0)])
+def test_second_products_of_low_rank_pairs(n, c, r, ld):
     """One chain of multiply-adds over the rank per output: a token's bits are those of a step of few tokens.
     ``ld``: hidden values that allow no reads of 16 bytes."""
     from scratch_llm_b200.kernels import ops
     g = torch.Generator().manual_seed(n + c + r)
     pre = torch.randn(n, c + r + ld, generator=g).to(DEV)[:, :c + r]
     w2t = (torch.randn(r, c, generator=g) * r ** -0.5).to(DEV)
-    w0, ab = torch.randn(c, generator=g).to(DEV), torch.randn(c, generator=g).to(DEV)
+    w0, ab, rate = (torch.randn(c, generator=g).to(DEV) for _ in range(3))
 
-    def decays(pre):
-        return ops.lowrank_decay(pre, w2t, w0, ab, 0.6, torch.empty(len(pre), 2 * c, device=DEV))
+    def outputs(pre):
+        m = len(pre)
+        wa, log, gate = (torch.empty(m, w, device=DEV) for w in (2 * c, c, c))
+        ops.lowrank_decay(pre, w2t, w0, ab, 0.6, wa)
+        ops.lowrank_expand(pre, c, w2t, log, bias=w0, rate_log=rate, per_rate=1, also=(c, w2t, gate))
+        half = ops.lowrank_expand(pre, c, w2t, torch.empty(m, c, device=DEV, dtype=torch.bfloat16), tanh_in=True)
+        return wa, log, gate, half
 
-    got = decays(pre)
-    assert torch.equal(got, torch.cat([decays(pre[t:t + 200]) for t in range(0, n, 200)]))
-    x = pre.double()
-    want = torch.cat([torch.exp(-0.6 * torch.sigmoid(torch.tanh(x[:, c:]) @ w2t.double() + w0)),
-                      torch.sigmoid(x[:, :c] + ab)], 1)
-    # 32-bit sums of r products: r / 2 roundings of the largest partial sum at most
-    assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -24 * max(8, r / 2)
+    got = outputs(pre)
+    for parts in zip(got, *(outputs(pre[t:t + 100]) for t in range(0, n, 100))):
+        assert torch.equal(parts[0], torch.cat(parts[1:]))
+    x, w = pre.double(), w2t.double()
+    z = x[:, c:] @ w
+    want = torch.cat([torch.exp(-0.6 * torch.sigmoid(torch.tanh(x[:, c:]) @ w + w0)), torch.sigmoid(x[:, :c] + ab)], 1)
+    want = want, -rate.double().exp() * torch.nn.functional.softplus(z + w0), z
+    for a, b in zip(got, want):     # 32-bit sums of r products: r / 2 roundings of the largest partial sum at most
+        assert ((a.double() - b).norm() / b.norm()).item() < 2 ** -24 * max(8, r / 2)
 
 
 @pytest.mark.parametrize("V", [8192, 8200, 50001, 190001])
