@@ -24,7 +24,7 @@
 //
 // Why: a row's tokens in order are a chain of 128 pieces of 16 tokens for 2,048 tokens, 5.9 us each
 // whatever the GPU's width.  In chunks the chain has 32 links of two small products.  2,048 tokens, 16
-// heads of 128 x 128, bfloat16: one decay per head 733 -> 186 us, per channel 666 -> 277 us.  One by one, per
+// heads of 128 x 128, bfloat16: one decay per head 733 -> 186 us, per channel 666 -> 260 us.  One by one, per
 // head: 56, 89 and 46 us.
 #pragma once
 
@@ -167,6 +167,73 @@ __device__ __forceinline__ void substitute(Two (&acc)[TC / 2], const float* At) 
     }
 }
 
+// Forward substitution of one column of (I + A)^{-1} b, At[s][t] = -A_ts, a block of BT tokens at a time: what
+// the blocks before it do to a block, then the block itself.  Per entry one chain over s in ascending order.
+// The loops over blocks and over the tokens before one stay loops: as straight code over all 64 tokens (1,600
+// instructions, and twice 1,700 for the pairs of tokens inside the blocks) instruction fetches were what the kernel
+// of decays per channel waited for most (2.45 of 6 cycles an instruction, 0.32 now; 247 -> 227 us at 3,001 tokens,
+// four rows, 16 heads).  The kernel with one decay per head, two CTAs an SM and no other long code, keeps
+// `substitute`: 186 us for 2,048 tokens, 188 so.  The same bits.
+// X: this thread's place for solved entries, rows PREP_THREADS apart.  fetch(t): b_t as it lies in memory; it is asked
+// for a block ahead.  right(t, raw): b_t.  store(t0, acc): the solved entries t0 .. t0 + BT - 1.
+template <typename Fetch, typename Right, typename Store>
+__device__ __forceinline__ void solve_column(const float* At, float* X, const Fetch& fetch, const Right& right,
+                                             const Store& store) {
+    float raw[BT];
+#pragma unroll
+    for (int t = 0; t < BT; ++t) raw[t] = fetch(t);
+#pragma unroll 1
+    for (int t0 = 0; t0 < TC; t0 += BT) {
+        Two acc[BT / 2];
+#pragma unroll
+        for (int t = 0; t < BT; t += 2) acc[t / 2] = two(right(t0 + t, raw[t]), right(t0 + t + 1, raw[t + 1]));
+        if (t0 + BT < TC) {
+#pragma unroll
+            for (int t = 0; t < BT; ++t) raw[t] = fetch(t0 + BT + t);
+        }
+        const float* a = At + t0;
+#pragma unroll 4
+        for (int s = 0; s < t0; ++s) {
+            const float us = X[s * PREP_THREADS];
+            const Two u = two(us, us);
+#pragma unroll
+            for (int t4 = 0; t4 < BT / 4; ++t4) {
+                const Four v = load22(a + s * LDT + 4 * t4);
+                acc[2 * t4] = fma2(v.a, u, acc[2 * t4]);
+                acc[2 * t4 + 1] = fma2(v.b, u, acc[2 * t4 + 1]);
+            }
+        }
+        a += t0 * LDT;
+#pragma unroll
+        for (int s = 0; s < BT - 1; ++s) {
+            const float us = s & 1 ? second(acc[s / 2]) : first(acc[s / 2]);
+            const Two u = two(us, us);
+            // the pair that holds s itself: only its second entry may come after s
+            if (!(s & 1)) acc[s / 2] = two(us, fmaf(a[s * LDT + s + 1], us, second(acc[s / 2])));
+            const int p0 = s / 2 + 1;        // pairs from here on lie after s
+            if ((p0 & 1) && p0 < BT / 2) {
+                const Two v = {*reinterpret_cast<const unsigned long long*>(a + s * LDT + 2 * p0)};
+                acc[p0] = fma2(v, u, acc[p0]);
+            }
+#pragma unroll
+            for (int t4 = (p0 + 1) / 2; t4 < BT / 4; ++t4) {
+                const Four v = load22(a + s * LDT + 4 * t4);
+                acc[2 * t4] = fma2(v.a, u, acc[2 * t4]);
+                acc[2 * t4 + 1] = fma2(v.b, u, acc[2 * t4 + 1]);
+            }
+        }
+        if (t0 + BT < TC) {
+#pragma unroll
+            for (int t = 0; t < BT; t += 2) {
+                X[(t0 + t) * PREP_THREADS] = first(acc[t / 2]);
+                X[(t0 + t + 1) * PREP_THREADS] = second(acc[t / 2]);
+            }
+        }
+        store(t0, acc);
+    }
+}
+constexpr int SOLVED = (TC - BT) * PREP_THREADS;     // floats of shared memory for the solved entries
+
 // Where the pass finds W_td and y~_td (its threads' operands of mma.m16n8k16, four elements each):
 // W as [d / 16][t / 8][lane][4], y~ as [d / 16][t / 16][d % 16 / 8][lane][4].
 __device__ __forceinline__ int w_place(int t, int d) {
@@ -189,6 +256,22 @@ __device__ __forceinline__ void store_column(const Two (&acc)[TC / 2], float* W,
         for (int t = 0; t < TC; t += 4)
             *reinterpret_cast<float4*>(X0 + t) = make_float4(first(acc[t / 2]), second(acc[t / 2]),
                                                              first(acc[t / 2 + 1]), second(acc[t / 2 + 1]));
+    }
+}
+
+// Solved entries t0 .. t0 + BT - 1 of a column of W (d >= 0), or of X0.
+__device__ __forceinline__ void store_column(const Two (&acc)[BT / 2], int t0, float* W, int d, float* X0) {
+    if (d >= 0) {
+#pragma unroll
+        for (int t = 0; t < BT; t += 2) {
+            W[w_place(t0 + t, d)] = first(acc[t / 2]);
+            W[w_place(t0 + t + 1, d)] = second(acc[t / 2]);
+        }
+    } else {
+#pragma unroll
+        for (int t = 0; t < BT; t += 4)
+            *reinterpret_cast<float4*>(X0 + t0 + t) = make_float4(first(acc[t / 2]), second(acc[t / 2]),
+                                                                  first(acc[t / 2 + 1]), second(acc[t / 2 + 1]));
     }
 }
 
@@ -482,15 +565,17 @@ __device__ __forceinline__ void prep_head(const PrepArgs& a, const Scratch& z, c
 }
 
 template <int D> constexpr size_t prep_channels_smem() {
-    return (size_t)(3 * TC * (D + 4) + TC * LDT + 15 * D) * 4;
+    return (size_t)(3 * TC * (D + 4) + TC * LDT + 15 * D + SOLVED) * 4;
 }
 
-// The pairs of tokens inside a block: x_t with every y_s, s < t (OWN: s <= t), decayed from s to t.  D / 4 lanes
+// The pairs of tokens inside a block: x_t with every y_s, s < t (own: s <= t), decayed from s to t.  D / 4 lanes
 // share the channels; a lane keeps its channels of the y's in registers and fades them token by token, so
 // that no exponential is needed, and the lanes' sums are exchanged per t.  `fade`: the tokens' decays.
-// entry(t, s, dot) takes the result.
-template <int D, bool OWN, typename Entry>
-__device__ __forceinline__ void block_pairs(const float* x, const float* y, const float* fade, const Entry& entry) {
+// The result, times -factor[t] if there are factors, goes to to[t * to_t + s * to_s]; zero for other s.  (One body for
+// both tables: it is 1,700 instructions long.)
+template <int D>
+__device__ __forceinline__ void block_pairs(const float* x, const float* y, const float* fade, bool own_too,
+                                            const float* factor, float* to, int to_t, int to_s) {
     constexpr int LD = D + 4, LANES = D / 4;
     const int e = threadIdx.x % LANES * 4, lane = threadIdx.x & 31;
     const Two zero = two(0.f, 0.f);
@@ -509,9 +594,10 @@ __device__ __forceinline__ void block_pairs(const float* x, const float* y, cons
 #pragma unroll
         for (int s = 0; s < BT; ++s) {
             v[s] = 0.f;
-            if (s < t || (OWN && s == t)) {
+            if (s <= t) {
                 const Two d = fma2(xv.b, ys[s][1], fma2(xv.a, ys[s][0], zero));
                 v[s] = first(d) + second(d);
+                if (s == t && !own_too) v[s] = 0.f;
             }
         }
         int n = BT;
@@ -530,21 +616,22 @@ __device__ __forceinline__ void block_pairs(const float* x, const float* y, cons
                 v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
             }
         }
+        const float by = factor ? -factor[t] : 1.f;
         if (LANES == 8) {
-            entry(t, (lane & 7) * 2, v[0]);
-            entry(t, (lane & 7) * 2 + 1, v[1]);
+            to[t * to_t + (lane & 7) * 2 * to_s] = by * v[0];
+            to[t * to_t + ((lane & 7) * 2 + 1) * to_s] = by * v[1];
         } else if (LANES == 16) {
-            entry(t, lane & 15, v[0]);
+            to[t * to_t + (lane & 15) * to_s] = by * v[0];
         } else if (!(lane & 1)) {
-            entry(t, lane >> 1, v[0]);
+            to[t * to_t + (lane >> 1) * to_s] = by * v[0];
         }
     }
 }
 
 // A decay per key channel.  Arrays in shared memory change what they hold: R = q, then q e^{l}; U = k, then
 // k e^{l}; L = the decays, then k e^{border - l} (l: sums of logarithms from the block's border on).  One
-// CTA an SM: the 254 registers of the substitution's column allow no second, nor do 127 KB at D = 128.  245 us at
-// 3,001 tokens in four rows and 16 heads of 128 x 128 (960 CTAs, 6.5 rounds).
+// CTA an SM: its shared memory allows no second.  227 us at 3,001 tokens in four rows and 16 heads of 128 x 128
+// (960 CTAs, 6.5 rounds): latencies of eight warps (0.34 instructions a cycle and scheduler).
 template <int D, typename T>
 __device__ __forceinline__ void prep_channels(const PrepArgs& a, const Scratch& z, const Group& group) {
     constexpr int LD = D + 4;
@@ -591,12 +678,9 @@ __device__ __forceinline__ void prep_channels(const PrepArgs& a, const Scratch& 
     for (int unit = tid / (D / 4); unit < 2 * NB; unit += PREP_THREADS / (D / 4)) {
         const int r0 = BT * (unit % NB);
         const float *u = U + r0 * LD, *fade = L + r0 * LD;
-        if (unit >= NB)
-            block_pairs<D, true>(R + r0 * LD, u, fade, [&](int t, int s, float d) { M[(r0 + t) * TC + r0 + s] = d; });
-        else
-            block_pairs<D, false>(u, u, fade, [&](int t, int s, float d) {
-                At[(r0 + s) * LDT + r0 + t] = -beta[r0 + t] * d;
-            });
+        const bool with_q = unit >= NB;
+        block_pairs<D>(with_q ? R + r0 * LD : u, u, fade, with_q, with_q ? nullptr : beta + r0,
+                       with_q ? M + r0 * TC + r0 : At + r0 * LDT + r0, with_q ? TC : 1, with_q ? 1 : LDT);
     }
     __syncthreads();
     for (int i = tid; i < NB * D; i += PREP_THREADS) {       // decays into the operands
@@ -656,21 +740,20 @@ __device__ __forceinline__ void prep_channels(const PrepArgs& a, const Scratch& 
         const float gy = post[ty / BT * D + d];
         store4(z.Y + at * TC * D + 4 * i, make_float4(y[0] * gy, y[LD] * gy, y[8 * LD] * gy, y[9 * LD] * gy));
     }
+    float* solved = mids + 3 * D;
     for (int at_col = tid; at_col < (D + a.V + 31) / 32 * 32; at_col += PREP_THREADS) {    // whole warps
         const int col = min(at_col, D + a.V - 1);
-        Two acc[TC / 2];
-        if (col < D) {
-#pragma unroll
-            for (int t = 0; t < TC; t += 2) {
-                const float f = pre[t / BT * D + col];
-                acc[t / 2] = two(beta[t] * f * U[t * LD + col], beta[t + 1] * f * U[(t + 1) * LD + col]);
-            }
-        } else {
-            load_column(acc, x + a.v0 + (int64_t)head * a.V + (col - D), a.ld, nt, beta);
-        }
-        substitute(acc, At);
-        if (at_col < D + a.V)
-            store_column(acc, z.W + at * TC * D, col < D ? col : -1, z.X + (at * a.V + (col - D)) * TC);
+        const bool is_w = col < D;
+        const T* v = x + a.v0 + (int64_t)head * a.V + max(col - D, 0);
+        float* X0 = z.X + (at * a.V + (col - D)) * TC;
+        solve_column(At, solved + tid,
+                     [&](int t) { return is_w ? U[t * LD + col] : to_float(v[min(t, nt - 1) * a.ld]); },
+                     [&](int t, float raw) {
+                         return is_w ? beta[t] * pre[t / BT * D + col] * raw : t < nt ? beta[t] * raw : 0.f;
+                     },
+                     [&](int t0, const Two (&acc)[BT / 2]) {
+                         if (at_col < D + a.V) store_column(acc, t0, z.W + at * TC * D, is_w ? col : -1, X0);
+                     });
     }
 }
 
