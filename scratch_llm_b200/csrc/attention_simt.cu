@@ -33,7 +33,8 @@ constexpr bool PAIRS = HD % 64 == 0; // a lane's dims are pairs of neighbours
 // Queries of a warp: a read of a key or a value in shared memory serves all of them, and a tile of keys
 // that a CTA fetches serves WARPS times as many.  Eight for long portions, where registers and shared
 // memory hold them; one for rows of a few tokens, whose other queries would be worked on for nothing.
-// 777 tokens, 32 heads of 64: 317 us with four queries a warp and a read per operand, 213 with eight.
+// 777 tokens, 32 heads of 64: 317 us with four queries a warp and a read per operand, 213 with eight, 178 with the
+// blocks of the most keys first over all heads (heads of 128: 313 and 249).
 constexpr int LONG_QUERIES = HD <= 128 ? 8 : 4;
 
 constexpr size_t smem_floats(int rpw) {
@@ -286,9 +287,10 @@ attn_simt_kernel(const T* __restrict__ q, const T* __restrict__ pages, const int
     extern __shared__ __align__(16) float smem[];
     __shared__ long long key_base[BKV];  // element offset of each key's K row, -1 if absent
     constexpr int BQ = WARPS * MOST;
-    const int r = blockIdx.y, h = blockIdx.z;
+    const int r = blockIdx.y, h = blockIdx.x % args.H;
     const int t0 = row_start[r], n_new = row_start[r + 1] - t0;
-    const int q0 = (gridDim.x - 1 - blockIdx.x) * BQ;    // the queries with the most keys first
+    // the queries with the most keys first, of all heads
+    const int q0 = (gridDim.x - 1 - blockIdx.x) / args.H * BQ;
     if (q0 >= n_new) return;
     const int nq = min(BQ, n_new - q0);
     const int* table = block_table + (int64_t)r * args.table_stride;
@@ -311,7 +313,7 @@ static int launch(const void* q, const void* pages, const int* block_table, cons
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     constexpr int BQ = WARPS * MOST;
-    attn_simt_kernel<T, MOST><<<dim3((max_new + BQ - 1) / BQ, n_rows, args.H), THREADS, smem, stream>>>(
+    attn_simt_kernel<T, MOST><<<dim3(args.H * ((max_new + BQ - 1) / BQ), n_rows), THREADS, smem, stream>>>(
         (const T*)q, (const T*)pages, block_table, row_start, row_pos0, (T*)out, slopes, sinks, args);
     SLLM_LAUNCH_CHECK();
     return 0;
