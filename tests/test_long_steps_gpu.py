@@ -149,3 +149,52 @@ def test_convolution_and_carried_inputs_in_one_pass(dtype, C, taps):
             ops.conv_state_update(x, taps, st, row_start, row_slot, 5)
         outs.append((out, st))
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("hd", [64, 16, 80, 112])
+@pytest.mark.parametrize("H,G", [(4, 1), (6, 3), (3, 3)])
+@pytest.mark.parametrize("more", [{}, dict(window=37), dict(chunk=48), dict(softcap=5.0), dict(slopes=1, sinks=1)])
+def test_attention_simt_tiles(hd, H, G, more):
+    """Long 32-bit portions: four, two and one heads of a kv head to a block, each option: a token's bits are those
+    it has alone (a kernel of its own)."""
+    from scratch_llm_b200.kernels import ops
+    ops.prepare_jobs([ops.attention_library(hd)], verbose=False)
+    page, before, n = 16, 21, 95
+    gen = torch.Generator().manual_seed(hd + H)
+    pages = torch.randn(-(-(before + n) // page), 2, G, page, hd, generator=gen).to(DEV)
+    q = torch.randn(n, H * hd, generator=gen).to(DEV)
+    table = torch.arange(len(pages), dtype=torch.int32, device=DEV).view(1, -1)
+    kw = {k: torch.randn(H, generator=gen).to(DEV) if k in ("slopes", "sinks") else v for k, v in more.items()}
+    window = kw.pop("window", None)
+
+    def attend(first, count):
+        out = torch.empty(count, H * hd, device=DEV)
+        ops.attention_simt(q[first:first + count], pages, table, page, _i32([0, count]), _i32([before + first]),
+                           out, 1, count, H, G, hd, hd ** -0.5, window, **kw)
+        return out
+
+    assert torch.equal(attend(0, n), torch.cat([attend(t, 1) for t in range(n)]))
+
+
+@pytest.mark.parametrize("hd", [64, 48])
+@pytest.mark.parametrize("window", [None, 37])
+def test_attention_simt_rows_in_two_launches(hd, window):
+    """Rows of all lengths in a launch for long ones (tiles, and the other kernel for rows of up to 16 tokens)."""
+    from scratch_llm_b200.kernels import ops
+    ops.prepare_jobs([ops.attention_library(hd)], verbose=False)
+    H, G, page = 8, 2, 16
+    rows = [(70, 1), (0, 40), (5, 4), (31, 16), (0, 0), (64, 17), (90, 5), (3, 33)]      # (cached, new)
+    gen = torch.Generator().manual_seed(hd)
+    need = [-(-(b + n) // page) for b, n in rows]
+    pages = torch.randn(sum(need), 2, G, page, hd, generator=gen).to(DEV)
+    first = [sum(x for _, x in rows[:r]) for r in range(len(rows) + 1)]
+    q = torch.randn(first[-1], H * hd, generator=gen).to(DEV)
+    table = torch.full((len(rows), max(need)), -1, dtype=torch.int32)
+    for r, k in enumerate(need):
+        table[r, :k] = torch.arange(sum(need[:r]), sum(need[:r]) + k)
+    outs = []
+    for most in (40, 600):
+        outs.append(torch.full_like(q, float("nan")))
+        ops.attention_simt(q, pages, table.to(DEV), page, _i32(first), _i32([b for b, _ in rows]), outs[-1], len(rows),
+                           most, H, G, hd, hd ** -0.5, window)
+    assert torch.equal(outs[0], outs[1])
