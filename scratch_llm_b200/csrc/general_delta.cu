@@ -90,6 +90,14 @@ __device__ __forceinline__ void loaders_sync() {
 __device__ __forceinline__ float4 load4(const float* p) {
     return *reinterpret_cast<const float4*>(p);
 }
+// Dot products are formed with the key itself and not with the unit key, so a large key would overflow them where
+// the rule does not.  A chunk with a key of LARGE or more is therefore changed once it is staged (`shrink`).  The
+// question costs decode steps 0 to 2 % (heads of 16: 64 single tokens 18.0 / 18.5 us) and long rows nothing.
+constexpr float LARGE = 1024.f;
+__device__ __forceinline__ bool large(float x) { return fabsf(x) >= LARGE; }
+__device__ __forceinline__ bool large(const float4& x) {
+    return large(fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
+}
 // Four elements as they lie in memory, and as numbers.
 template <typename T> struct Four;
 template <> struct Four<float> { typedef float4 Raw; };
@@ -109,6 +117,7 @@ struct alignas(16) Staged {
     float r[CHUNK][DP], w[CHUNK][DP], nak[CHUNK][DP];   // nak: -a * k
     float v[CHUNK][COLS];
     float2 ic[CHUNK];           // i_t = 1 / (|k_t|^2 + eps), and i_t (k_t . nak_{t-1})
+    float by[CHUNK];            // (of `shrink` alone)
 };
 static constexpr int SMEM = 2 * (int)sizeof(Staged);
 
@@ -174,13 +183,58 @@ static __device__ __forceinline__ void request_chunk(Request<T, VEC>& q, int lt,
     }
 }
 
+// 1 / (|k_t|^2 + eps) and the product with the neighbour's row p of nak (or null), by a warp.
+static __device__ __forceinline__ void token_sums(Staged& st, int lane, int t, const float* p, float eps) {
+    float ss = 0.f, c = 0.f;
+    for (int e = lane; e < DP; e += 32) {
+        const float k = st.k[t][e];
+        ss = fmaf(k, k, ss);
+        if (p) c = fmaf(k, p[e], c);
+    }
+    ss = warp_sum(ss);
+    c = warp_sum(c);
+    const float inv = 1.0f / (ss + eps);
+    if (lane == 0) st.ic[t] = make_float2(inv, inv * c);
+}
+
+// The large keys of a staged chunk of n tokens, by the loader warps: each is divided by a power of two that brings its
+// largest element below 4, and its token's values multiplied by it.  k v, a k d and k . s / (|k|^2 + eps) stay what
+// they were, eps being divided by the square.  (A token's key is the same wherever it is staged: large or not by itself.)
+static __device__ __noinline__ void shrink(Staged& st, int lt, const float* before, int n, bool more, float unit_eps) {
+    const int lane = lt & 31;
+    for (int t = lt >> 5; t < n + more; t += LOADERS / 32) {       // a warp per key; the last: st.k[CHUNK]
+        unsigned most = 0u;
+        for (int e = lane; e < DP; e += 32) most = max(most, __float_as_uint(fabsf(st.k[t][e])));
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (lane == 0 && t < n) st.by[t] = 1.f;
+        if (most < __float_as_uint(LARGE)) continue;
+        const unsigned x = min(most >> 23, 254u);                  // (exponents from 2^2 on: 129)
+        const float by = __uint_as_float((255u - x) << 23), grow = __uint_as_float((x - 1u) << 23);
+        for (int e = lane; e < DP; e += 32) {
+            st.k[t][e] *= by;
+            if (t < n) st.nak[t][e] *= by;
+        }
+        if (t < n) {
+            for (int c = lane; c < COLS; c += 32) st.v[t][c] *= grow;
+            if (lane == 0) st.by[t] = by;
+        }
+    }
+    loaders_sync();
+    for (int t = lt >> 5; t < n; t += LOADERS / 32) {
+        const float by = st.by[t];
+        if (by != 1.f || (t > 0 && st.by[t - 1] != 1.f))
+            token_sums(st, lane, t, t == 0 ? before : st.nak[t - 1], unit_eps * by * by);
+    }
+}
+
 // The loader warps bring the chunk [tok0, tok0 + n), which they have requested, into `st`, and
 // request what is left of the `left` tokens after it.  `before`: the row of nak of the token before
-// tok0, or null.
+// tok0, or null.  Whether this thread has met a large key.
 template <typename T, bool VEC>
-static __device__ __forceinline__ void stage_chunk(Staged& st, Request<T, VEC>& q, int lt,
+static __device__ __forceinline__ bool stage_chunk(Staged& st, Request<T, VEC>& q, int lt,
                                             const Operands<T>& x, const float* before,
                                             int64_t tok0, int n, int left) {
+    bool met = false;
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
         const int i = lt + j * LOADERS, t = i / COLS, c = i - t * COLS;
@@ -189,15 +243,18 @@ static __device__ __forceinline__ void stage_chunk(Staged& st, Request<T, VEC>& 
     if (VEC) {
 #pragma unroll
         for (int j = 0; j < APT; ++j)
-            if ((lt + j * LOADERS) * 4 < DP)
-                *reinterpret_cast<float4*>(&st.k[CHUNK][(lt + j * LOADERS) * 4]) =
-                    numbers(q.k_after[j]);
+            if ((lt + j * LOADERS) * 4 < DP) {
+                const float4 k = numbers(q.k_after[j]);
+                met = met || large(k);
+                *reinterpret_cast<float4*>(&st.k[CHUNK][(lt + j * LOADERS) * 4]) = k;
+            }
 #pragma unroll
         for (int j = 0; j < QPT; ++j) {
             const int i = lt + j * LOADERS;
             const int t = i / (DP / 4), e = (i - t * (DP / 4)) * 4;
             if (i < QUADS && t < n) {
                 const float4 k = numbers(q.k[j]), a = q.a[j];
+                met = met || large(k);
                 *reinterpret_cast<float4*>(&st.r[t][e]) = numbers(q.r[j]);
                 *reinterpret_cast<float4*>(&st.k[t][e]) = k;
                 *reinterpret_cast<float4*>(&st.w[t][e]) = q.w[j];
@@ -217,10 +274,13 @@ static __device__ __forceinline__ void stage_chunk(Staged& st, Request<T, VEC>& 
                 a = x.wa[tok * x.ldwa + x.HD + x.head * D + e];
             }
             st.r[t][e] = r; st.k[t][e] = k; st.w[t][e] = w; st.nak[t][e] = -a * k;
+            met = met || large(k);
         }
-        for (int e = lt; e < DP; e += LOADERS)
-            st.k[CHUNK][e] = left > 0 && e < D
-                ? to_float(x.rkv[(tok0 + n) * x.ld + x.k0 + x.head * D + e]) : 0.f;
+        for (int e = lt; e < DP; e += LOADERS) {
+            const float k = left > 0 && e < D ? to_float(x.rkv[(tok0 + n) * x.ld + x.k0 + x.head * D + e]) : 0.f;
+            st.k[CHUNK][e] = k;
+            met = met || large(k);
+        }
     }
     loaders_sync();
     if (VEC && FUSED) {
@@ -254,21 +314,11 @@ static __device__ __forceinline__ void stage_chunk(Staged& st, Request<T, VEC>& 
             if (i < QUADS && t < n && e == 0) st.ic[t] = make_float2(inv, inv * c[j]);
         }
     } else {
-        for (int t = lt >> 5; t < n; t += LOADERS / 32) {   // a warp per token
-            const float* p = t == 0 ? before : st.nak[t - 1];
-            float ss = 0.f, c = 0.f;
-            for (int e = lt & 31; e < DP; e += 32) {
-                const float k = st.k[t][e];
-                ss = fmaf(k, k, ss);
-                if (p) c = fmaf(k, p[e], c);
-            }
-            ss = warp_sum(ss);
-            c = warp_sum(c);
-            const float inv = 1.0f / (ss + x.unit_eps);
-            if ((lt & 31) == 0) st.ic[t] = make_float2(inv, inv * c);
-        }
+        for (int t = lt >> 5; t < n; t += LOADERS / 32)     // a warp per token
+            token_sums(st, lt & 31, t, t == 0 ? before : st.nak[t - 1], x.unit_eps);
     }
     if (left > 0) request_chunk<T, VEC>(q, lt, x, tok0 + n, min(CHUNK, left), left > CHUNK);
+    return met;
 }
 
 static constexpr int SHARE = LANES / CPT;          // lanes that go on with the same column
@@ -443,9 +493,14 @@ general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int 
         typename R::template Request<T, VEC> q;
         R::template request_chunk<T, VEC>(q, lt, x, t0, min(CHUNK, n_new), n_new > CHUNK);
         for (int c0 = 0, buf = 0; c0 < n_new; c0 += CHUNK, buf ^= 1) {
-            R::template stage_chunk<T, VEC>(stage[buf], q, lt, x, c0 ? stage[buf ^ 1].nak[CHUNK - 1] : nullptr,
-                                (int64_t)t0 + c0, min(CHUNK, n_new - c0), n_new - c0 - CHUNK);
-            __syncthreads();    // chunk c is staged, chunk c - 1 is done with
+            const float* before = c0 ? stage[buf ^ 1].nak[CHUNK - 1] : nullptr;
+            const int n = min(CHUNK, n_new - c0), left = n_new - c0 - CHUNK;
+            const bool met = R::template stage_chunk<T, VEC>(stage[buf], q, lt, x, before, (int64_t)t0 + c0, n, left);
+            // chunk c is staged, chunk c - 1 is done with (the compute warps wait again while large keys are changed)
+            if (__syncthreads_or(met)) {
+                R::shrink(stage[buf], lt, before, n, left > 0, unit_eps);
+                __syncthreads();
+            }
         }
         return;
     }
@@ -471,7 +526,7 @@ general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int 
     const bool stores = o_col < V;
     float* o_row = out + t0 * ld_out + (int64_t)head * V + o_col;    // of token 0
     f2 s[CPT][2 * UNITS];
-    __syncthreads();            // the first chunk is staged
+    if (__syncthreads_or(false)) __syncthreads();       // the first chunk is staged
     R::template fetch<4 * LANES>(p.k, &stage[0].k[0][e0]);
     p.state(s);
     p.begin(s);
@@ -497,7 +552,7 @@ general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int 
             for (int sh = SHARE >> 1; sh > 0; sh >>= 1) o += __shfl_xor_sync(0xffffffffu, o, sh);
             if (stores && c0 + t > 0) o_row[(c0 + t - 1) * ld_out] = o;
         }
-        if (c0 + CHUNK < n_new) __syncthreads();
+        if (c0 + CHUNK < n_new && __syncthreads_or(false)) __syncthreads();
     }
     p.state(s);
     float o = p.begin(s);

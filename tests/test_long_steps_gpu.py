@@ -198,3 +198,37 @@ def test_attention_simt_rows_in_two_launches(hd, window):
         ops.attention_simt(q, pages, table.to(DEV), page, _i32(first), _i32([b for b, _ in rows]), outs[-1], len(rows),
                            most, H, G, hd, hd ** -0.5, window)
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("D", [64, 128, 16, 33, 200])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("size", [5e2, 1e10, 1e17, 1e25])
+def test_general_delta_large_keys(D, dtype, size):
+    """Keys whose products with each other or with the state leave the range of 32 bits, though neither the state
+    nor the read-outs do, beside ordinary ones, a small one and one of zeros."""
+    from scratch_llm_b200.kernels import ops
+    ops.prepare_jobs([ops.general_delta_library(D)], verbose=False)
+    H, V, lens = 2, 8, [1, 5, 40]
+    g = torch.Generator().manual_seed(D)
+    n, DP = sum(lens), ops.general_delta_padded_dim(D)
+    k = torch.randn(n, H * D, generator=g) * size
+    k[::3] /= size
+    k[20], k[31] = 1e-3, 0.0
+    r, v = torch.randn(n, H * D, generator=g), torch.randn(n, H * V, generator=g) * 1e8
+    rkv = torch.cat([r, k, v], 1).to(dtype).to(DEV)
+    wa = torch.cat([torch.rand(n, H * D, generator=g) * 0.45 + 0.55, torch.rand(n, H * D, generator=g)], 1).to(DEV)
+    state, out = torch.zeros(3, H, V, DP, device=DEV), torch.empty(n, H * V, device=DEV)
+    starts = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    ops.general_delta(rkv, (0, H * D, 2 * H * D), wa, state, _i32(starts), _i32([0, 1, 2]), out, 3, H, D, V, 1e-6)
+    r, k, v = rkv.double().split([H * D, H * D, H * V], 1)
+    r, k, v, (w, a) = r.view(n, H, D), k.view(n, H, D), v.view(n, H, V), wa.double().view(n, 2, H, D).unbind(1)
+    u = k / (k.square().sum(-1, keepdim=True) + 1e-6).sqrt()
+    want = torch.empty(n, H, V, device=DEV, dtype=torch.float64)
+    for i in range(len(lens)):
+        S = torch.zeros(H, V, D, dtype=torch.float64, device=DEV)
+        for t in range(starts[i], starts[i + 1]):
+            S = S * w[t][:, None] - (S @ u[t][..., None]) * (a[t] * u[t])[:, None] + v[t][..., None] * k[t][:, None]
+            want[t] = (S @ r[t][..., None])[..., 0]
+        # (a few tokens' roundings, each a few of 2^-24)
+        assert ((state[i, ..., :D].double() - S).norm() / S.norm()).item() < 1e-6
+    assert ((out.double() - want.flatten(1)).norm() / want.norm()).item() < 1e-6
