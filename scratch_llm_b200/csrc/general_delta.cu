@@ -54,7 +54,6 @@ constexpr int DP = padded(D);                 // padded key size
 static_assert(DP <= 512, "key sizes up to 512");
 constexpr int EPL = DP <= 128 ? 4 : DP / 32;  // elements of a column per lane
 constexpr int LANES = DP / EPL;
-constexpr int COMPUTE = 128, LOADERS = 128, THREADS = COMPUTE + LOADERS;
 constexpr int UNITS = EPL / 4;                // float4 units per lane
 // tokens per chunk: two buffers of four vectors of DP floats per token, within 64 KB
 constexpr int CHUNK = DP <= 128 ? 16 : 2048 / DP;
@@ -83,10 +82,6 @@ __device__ __forceinline__ float pair_sum(f2 a) {
     return x + y;
 }
 
-__device__ __forceinline__ void loaders_sync() {
-    asm volatile("bar.sync 1, %0;\n" ::"n"(LOADERS) : "memory");
-}
-
 __device__ __forceinline__ float4 load4(const float* p) {
     return *reinterpret_cast<const float4*>(p);
 }
@@ -109,9 +104,17 @@ __device__ __forceinline__ float4 numbers(const uint2& r) {
 }
 
 // The rule for threads with slices of CPT columns: 4, or 2 where that still leaves the launch within one CTA an
-// SM (half of each token's work a warp, twice the CTAs).
-template <int CPT> struct Rule {
+// SM (half of each token's work a warp, twice the CTAs); WARPS compute warps: 4, or one where many CTAs with heads
+// of few columns have to share an SM.
+template <int CPT, int WARPS> struct Rule {
+static constexpr int COMPUTE = 32 * WARPS;
+static constexpr int QUADS = CHUNK * DP / 4;         // units of 4 elements in a chunk
+static constexpr int LOADERS = WARPS > 1 ? 128 : QUADS / 4 < 32 ? 32 : QUADS / 4;
+static constexpr int THREADS = COMPUTE + LOADERS;
 static constexpr int COLS = COMPUTE / LANES * CPT;   // columns of S per CTA
+static __device__ __forceinline__ void loaders_sync() {
+    asm volatile("bar.sync 1, %0;\n" ::"n"(LOADERS) : "memory");
+}
 struct alignas(16) Staged {
     float k[CHUNK + 1][DP];     // (the last: the first key of the chunk that follows)
     float r[CHUNK][DP], w[CHUNK][DP], nak[CHUNK][DP];   // nak: -a * k
@@ -121,7 +124,6 @@ struct alignas(16) Staged {
 };
 static constexpr int SMEM = 2 * (int)sizeof(Staged);
 
-static constexpr int QUADS = CHUNK * DP / 4;                       // units of 4 elements in a chunk
 static constexpr int QPT = (QUADS + LOADERS - 1) / LOADERS;        // of which a loader thread takes
 static constexpr int VPT = (CHUNK * COLS + LOADERS - 1) / LOADERS; // values that a loader thread takes
 static constexpr int APT = (DP / 4 + LOADERS - 1) / LOADERS;       // units of the key after the chunk
@@ -468,8 +470,9 @@ static __device__ __forceinline__ int share_tokens(float (&o)[GROUP], int lane_i
 
 // rkv: [N, ld] with the heads' r at column r0, k at k0, v at v0 (each heads x D or heads x V);
 // wa: float32 [N, ldwa] with the decays at column 0 and the removal rates at column H * D.
-template <typename T, bool VEC, int CPT>
-__global__ void __launch_bounds__(THREADS, DP <= 128 ? 2 : 1)
+// (two CTAs an SM at every key size: 4 heads of 300 x 300, 64 single tokens 311 us with one, 159 so)
+template <typename T, bool VEC, int CPT, int WARPS>
+__global__ void __launch_bounds__(Rule<CPT, WARPS>::THREADS, WARPS > 1 ? 2 : 512 / Rule<CPT, WARPS>::THREADS)
 general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int v0,
                      const float* __restrict__ wa, int64_t ldwa, float* __restrict__ state,
                      const int* __restrict__ row_start, const int* __restrict__ row_slot,
@@ -477,7 +480,7 @@ general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int 
     pdl_wait();
     pdl_trigger();
     extern __shared__ __align__(16) uint8_t smem[];
-    typedef Rule<CPT> R;
+    typedef Rule<CPT, WARPS> R;
     typedef typename R::Staged Staged;
     constexpr int SHARE = R::SHARE, GROUP = R::GROUP;
     Staged* stage = reinterpret_cast<Staged*>(smem);
@@ -485,10 +488,10 @@ general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int 
     const int t0 = row_start[row], n_new = row_start[row + 1] - t0;
     if (n_new <= 0) return;
     const int tid = threadIdx.x;
-    const bool loader = tid >= COMPUTE;
+    const bool loader = tid >= R::COMPUTE;
     const int col0 = blockIdx.x * R::COLS;
     if (loader) {
-        const int lt = tid - COMPUTE;
+        const int lt = tid - R::COMPUTE;
         const typename R::template Operands<T> x{rkv, wa, ld, ldwa, r0, k0, v0, H * D, head, V, col0, unit_eps};
         typename R::template Request<T, VEC> q;
         R::template request_chunk<T, VEC>(q, lt, x, t0, min(CHUNK, n_new), n_new > CHUNK);
@@ -568,10 +571,10 @@ general_delta_kernel(const T* __restrict__ rkv, int64_t ld, int r0, int k0, int 
                     make_ulonglong2(s[c][2 * i], s[c][2 * i + 1]);
 }
 
-template <typename T, bool VEC, int CPT, typename... Args>
+template <typename T, bool VEC, int CPT, int WARPS, typename... Args>
 static int launch_rule(int n_rows, int H, int V, bool beside, cudaStream_t stream, Args... args) {
-    constexpr int SMEM = Rule<CPT>::SMEM, COLS = Rule<CPT>::COLS;
-    const auto kernel = general_delta_kernel<T, VEC, CPT>;
+    constexpr int SMEM = Rule<CPT, WARPS>::SMEM, COLS = Rule<CPT, WARPS>::COLS, THREADS = Rule<CPT, WARPS>::THREADS;
+    const auto kernel = general_delta_kernel<T, VEC, CPT, WARPS>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return (int)e;
     const dim3 grid((V + COLS - 1) / COLS, H, n_rows);
@@ -582,19 +585,27 @@ static int launch_rule(int n_rows, int H, int V, bool beside, cudaStream_t strea
 }
 
 // Two columns a thread while the launch has at most one CTA an SM even so: 32 heads of 64 x 64, a row of 2,048
-// tokens 300 us with four, 238 with two; 100 tokens 18 and 15; beyond, the SMs' throughput counts (64 heads, a
+// tokens 300 us with four, 231 with two; 100 tokens 18 and 15; beyond, the SMs' throughput counts (64 heads, a
 // row of 2,400: 353 and 404).
+// One compute warp and few loaders (64 threads at key size 16) where an SM gets more than the two CTAs of 256
+// threads that it holds, and the head's columns leave most of such a CTA idle.  us with 256 threads and so: 256 single
+// tokens, 32 heads of 16 x 16 67.6 / 21.2, of 9 x 9 69.7 / 21.0, 16 of 32 x 32 27.8 / 18.9, 16 of 64 x 5 28.6 / 14.1; 48 rows
+// of 8 tokens, 32 heads of 16 x 16 21.8 / 10.2.  (8 heads of 16 x 100, which take four such CTAs: 19.2 / 21.2.)
 template <typename T, bool VEC>
 static int launch(const T* rkv, int64_t ld, int r0, int k0, int v0, const float* wa, int64_t ldwa, float* state,
                   const int* row_start, const int* row_slot, float* out, int n_rows, int H, int V, float unit_eps,
                   int n_sm, bool beside, cudaStream_t stream) {
     constexpr int MOST = EPL == 4 ? 4 : 16 / EPL, FEW = EPL == 4 ? 2 : MOST;
-    const int64_t ctas = (int64_t)((V + Rule<FEW>::COLS - 1) / Rule<FEW>::COLS) * H * n_rows;
-    if (FEW != MOST && ctas <= n_sm)
-        return launch_rule<T, VEC, FEW>(n_rows, H, V, beside, stream, rkv, ld, r0, k0, v0, wa, ldwa, state, row_start,
-                                        row_slot, out, H, V, unit_eps);
-    return launch_rule<T, VEC, MOST>(n_rows, H, V, beside, stream, rkv, ld, r0, k0, v0, wa, ldwa, state, row_start,
-                                     row_slot, out, H, V, unit_eps);
+    const auto ctas = [&](int cols) { return (int64_t)((V + cols - 1) / cols) * H * n_rows; };
+#define SLLM_GD_RULE(CPT, WARPS)                                                                                \
+    return launch_rule<T, VEC, CPT, WARPS>(n_rows, H, V, beside, stream, rkv, ld, r0, k0, v0, wa, ldwa, state,  \
+                                           row_start, row_slot, out, H, V, unit_eps)
+    if (FEW != MOST && ctas(Rule<FEW, 4>::COLS) <= n_sm) SLLM_GD_RULE(FEW, 4);
+    if constexpr (DP <= 64) {
+        if (V <= 2 * Rule<MOST, 1>::COLS && ctas(Rule<MOST, 4>::COLS) > 2 * n_sm) SLLM_GD_RULE(MOST, 1);
+    }
+    SLLM_GD_RULE(MOST, 4);
+#undef SLLM_GD_RULE
 }
 
 }  // namespace sllm

@@ -232,3 +232,42 @@ def test_general_delta_large_keys(D, dtype, size):
         # (a few tokens' roundings, each a few of 2^-24)
         assert ((state[i, ..., :D].double() - S).norm() / S.norm()).item() < 1e-6
     assert ((out.double() - want.flatten(1)).norm() / want.norm()).item() < 1e-6
+
+
+@pytest.mark.parametrize("D,V", [(64, 64), (64, 20), (64, 12), (128, 33), (16, 16), (16, 70), (9, 9), (24, 30), (33, 5),
+                                 (200, 9), (300, 3)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_general_delta_in_large_launches(D, V, dtype):
+    """More CTAs than the SMs hold (four columns a thread, one compute warp where heads have few columns): against 64
+    bits, and the bits of a row with three of the heads in a launch of its own (two columns a thread)."""
+    from scratch_llm_b200.kernels import ops
+    ops.prepare_jobs([ops.general_delta_library(D)], verbose=False)
+    lens = [1, 3, 4, 15, 16, 17, 0, 32, 33, 70]
+    H = 2 * torch.cuda.get_device_properties(0).multi_processor_count // len(lens) + 1
+    g = torch.Generator().manual_seed(D + V)
+    n, DP, few = sum(lens), ops.general_delta_padded_dim(D), 3
+    rkv = torch.randn(n, 2 * H * D + H * V, generator=g).to(dtype).to(DEV)
+    wa = torch.cat([torch.rand(n, H * D, generator=g) * 0.45 + 0.55, torch.rand(n, H * D, generator=g)], 1).to(DEV)
+    first = torch.zeros(len(lens), H, V, DP, device=DEV)
+    first[..., :D] = torch.randn(len(lens), H, V, D, generator=g).to(DEV)
+    cols, starts = (0, H * D, 2 * H * D), [sum(lens[:i]) for i in range(len(lens) + 1)]
+    state, out = first.clone(), torch.empty(n, H * V, device=DEV)
+    ops.general_delta(rkv, cols, wa, state, _i32(starts), _i32(list(range(len(lens)))), out, len(lens), H, D, V, 1e-6)
+
+    r, k, v = rkv.double().split([H * D, H * D, H * V], 1)
+    r, k, v, (w, a) = r.view(n, H, D), k.view(n, H, D), v.view(n, H, V), wa.double().view(n, 2, H, D).unbind(1)
+    u = k / (k.square().sum(-1, keepdim=True) + 1e-6).sqrt()
+    want, S_all = torch.empty(n, H, V, device=DEV, dtype=torch.float64), first.double().clone()
+    for i, m in enumerate(lens):
+        at, S = slice(starts[i], starts[i] + m), first[i, ..., :D].double()
+        for t in range(starts[i], starts[i] + m):
+            S = S * w[t][:, None] - (S @ u[t][..., None]) * (a[t] * u[t])[:, None] + v[t][..., None] * k[t][:, None]
+            want[t] = (S @ r[t][..., None])[..., 0]
+        S_all[i, ..., :D] = S
+        alone, o = first[i:i + 1, :few].contiguous(), torch.empty(m, few * V, device=DEV)
+        part = wa[at].view(m, 2, H, D)[:, :, :few].flatten(1).contiguous()
+        ops.general_delta(rkv[at].clone(), cols, part, alone, _i32([0, m]), _i32([0]), o, 1, few, D, V, 1e-6)
+        assert torch.equal(o, out[at, :few * V]) and torch.equal(alone[0], state[i, :few])
+    # decays of at least 0.55: a few tokens' roundings, each a few of 2^-24
+    for got, ref in ((out, want.flatten(1)), (state, S_all)):
+        assert ((got.double() - ref).norm() / ref.norm()).item() < 1e-6
