@@ -230,8 +230,7 @@ static __device__ __noinline__ void shrink(Staged& st, int lt, const float* befo
 }
 
 // The loader warps bring the chunk [tok0, tok0 + n), which they have requested, into `st` (`left` tokens come after
-// it).  `before`: the row of nak of the token before
-// tok0, or null.  Whether this thread has met a large key.
+// it).  `before`: the row of nak of the token before tok0, or null.  Returns whether this thread has met a large key.
 template <typename T, bool VEC>
 static __device__ __forceinline__ bool stage_chunk(Staged& st, Request<T, VEC>& q, int lt,
                                             const Operands<T>& x, const float* before,
@@ -595,18 +594,25 @@ static int launch_rule(int n_rows, int H, int V, bool beside, cudaStream_t strea
 // threads that it holds, and the head's columns leave most of such a CTA idle.  us with 256 threads and so: 256 single
 // tokens, 32 heads of 16 x 16 67.6 / 21.2, of 9 x 9 69.7 / 21.0, 16 of 32 x 32 27.8 / 18.9, 16 of 64 x 5 28.6 / 14.1; 48 rows
 // of 8 tokens, 32 heads of 16 x 16 21.8 / 10.2.  (8 heads of 16 x 100, which take four such CTAs: 19.2 / 21.2.)
+// `beside`: begun beside the kernel before it, a launch's CTAs take the places that come free first, two on some SMs,
+// and long rows of a launch that does not fill the SMs go by the slowest.  us of decays, rule and read-out in
+// turn, ordinary / beside: 32 heads of 64 x 64, 2,048 tokens 299 / 391, 300 52 / 67, 64 20.9 / 23.6, 8 13.0 / 12.7, 2
+// 10.0 / 9.8; 48 single tokens and one of 64 44.4 / 43.8; 48 rows of 8 50.2 / 49.9; more CTAs than the SMs hold:
+// 16 heads of 128 x 128, four rows of 1,024 660 / 635, eight of 300 396 / 392.  So: launches that fill the SMs, and those
+// of a chunk a row at most on average.
 template <typename T, bool VEC>
 static int launch(const T* rkv, int64_t ld, int r0, int k0, int v0, const float* wa, int64_t ldwa, float* state,
                   const int* row_start, const int* row_slot, float* out, int n_rows, int H, int V, float unit_eps,
-                  int n_sm, bool beside, cudaStream_t stream) {
+                  int n_sm, int n_tokens, cudaStream_t stream) {
     constexpr int MOST = EPL == 4 ? 4 : 16 / EPL, FEW = EPL == 4 ? 2 : MOST;
     const auto ctas = [&](int cols) { return (int64_t)((V + cols - 1) / cols) * H * n_rows; };
+    const bool many = ctas(Rule<MOST, 4>::COLS) > 2 * n_sm, beside = many || n_tokens <= CHUNK * (int64_t)n_rows;
 #define SLLM_GD_RULE(CPT, WARPS)                                                                                \
     return launch_rule<T, VEC, CPT, WARPS>(n_rows, H, V, beside, stream, rkv, ld, r0, k0, v0, wa, ldwa, state,  \
                                            row_start, row_slot, out, H, V, unit_eps)
     if (FEW != MOST && ctas(Rule<FEW, 4>::COLS) <= n_sm) SLLM_GD_RULE(FEW, 4);
     if constexpr (DP <= 64) {
-        if (V <= 2 * Rule<MOST, 1>::COLS && ctas(Rule<MOST, 4>::COLS) > 2 * n_sm) SLLM_GD_RULE(MOST, 1);
+        if (many && V <= 2 * Rule<MOST, 1>::COLS) SLLM_GD_RULE(MOST, 1);
     }
     SLLM_GD_RULE(MOST, 4);
 #undef SLLM_GD_RULE
@@ -618,9 +624,7 @@ using namespace sllm;
 
 SLLM_EXPORT int sllm_general_delta_padded_dim() { return DP; }
 
-// dtype of rkv: 0 = float32, 1 = bfloat16.  n_tokens: of all rows.  Steps of single tokens start beside the kernel
-// before them; longer rows do not: their CTAs would take the places that come free first, two on some SMs, and
-// the launch goes by the slowest (a layer of 32 heads of 64 x 64 and 2,048 tokens: 483 us, 387 so).
+// dtype of rkv: 0 = float32, 1 = bfloat16.  n_tokens: of all rows.
 SLLM_EXPORT int sllm_general_delta(const void* rkv, int64_t ld, int r0, int k0, int v0,
                                    const float* wa, int64_t ldwa, float* state,
                                    const int* row_start, const int* row_slot, float* out,
@@ -632,14 +636,13 @@ SLLM_EXPORT int sllm_general_delta(const void* rkv, int64_t ld, int r0, int k0, 
     const bool vec = D % 4 == 0 && ld % 4 == 0 && r0 % 4 == 0 && k0 % 4 == 0 && ldwa % 4 == 0 &&
                      !(((uintptr_t)rkv | (uintptr_t)wa) & 15);
     typedef __nv_bfloat16 bf16;
-    const bool beside = n_tokens <= n_rows;
     int dev = 0, n_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return (int)cudaErrorInvalidDevice;
 #define SLLM_GD_LAUNCH(T, VEC)                                                                  \
     return launch<T, VEC>((const T*)rkv, ld, r0, k0, v0, wa, ldwa, state, row_start, row_slot,  \
-                          out, n_rows, H, V, unit_eps, n_sm, beside, stream)
+                          out, n_rows, H, V, unit_eps, n_sm, n_tokens, stream)
     if (dtype == 0) {
         if (vec) SLLM_GD_LAUNCH(float, true);
         SLLM_GD_LAUNCH(float, false);
