@@ -527,9 +527,12 @@ lowrank_decay_kernel(const float* __restrict__ pre, int64_t ldp, const float* __
     }
 }
 
-// The same for long steps (C % 4 == 0, every operand on a 16-byte boundary).  C 2,048, R 64, us with 8 tokens a
-// CTA and so: 256 tokens 12.5 / 16.9, 512 16.8 / 17.0, 1,024 25.2 / 20.9, 2,048 43.5 / 28.6, 3,001 64 / 52; C 4,096,
-// R 128, 4,096 tokens 265 / 195.  The exponentials and divisions of the two outputs take as long as the products.
+// The same for long steps (C % 4 == 0, every operand on a 16-byte boundary).  us with 8 tokens a CTA and so, C x
+// tokens: R 64, 2,048 x 512 14.8 / 17.0, 1,024 23.1 / 20.6, 2,048 40.8 / 28.3, 3,001 59 / 51; R 128, 4,096 x 4,096 265 / 197
+// (186 with what follows the products unrolled).  The exponentials and divisions of the two outputs take as long as
+// the products.  A CTA takes 14 us at R 32, 17 at 64, 24 at 128 however many there are, so what counts is how
+// many: by 64 x 128 outputs a CTA, 128 CTAs lose (1,024 x 1,024, R 64: 14.8 / 16.9), 192 about match (1,024 x
+// 1,536: 19.9 / 20.5; R 128 31.8 / 31.2), 256 gain (1,024 x 2,048: 22.9 / 20.6), at R 32 from 384 on (256: 16.1 / 16.8).
 // grid (ceil(C / LR_COLS), ceil(N / LR_TOKENS)).
 constexpr int LR_MIN_TOKENS = 512;
 __global__ void __launch_bounds__(LR_THREADS, 4)
@@ -598,8 +601,13 @@ __device__ __forceinline__ float expanded(float z, int mode, float rate) {
 }
 
 // Long steps (C % 4 == 0, weights and outputs on 16-byte boundaries), in the tiles of the decays above.  Two
-// products of C 2,048, R 64, us with 16 tokens a CTA and so: 256 tokens 18.5 / 18.3, 512 25.6 / 21.7, 1,024 40.0 /
-// 26.1, 2,048 65.2 / 50.5, 3,001 89 / 68 (84 with what follows the products unrolled over a thread's 64 sums).
+// products, one with a softplus, of C 2,048, R 64, us with 8 or (from 512 tokens on) 16 tokens a CTA and so: 256
+// tokens 15.2 / 15.6, 512 24.4 / 18.8, 1,024 39.1 / 25.6, 2,048 64.4 / 50.5, 3,001 88 / 68 (84 with what follows the products
+// unrolled over a thread's 64 sums).  Here too the number of CTAs decides, of both products together: 64 lose
+// (1,024 x 256, R 64: 8.2 / 15.5), 128 match (1,024 x 512: 15.6 / 15.6), 192 gain (1,024 x 768: 22.5 / 18.6); at R 128 96 gain
+// (1,024 x 384: 23.1 / 22.7), as they do without a decay, whose tiles take 11 us instead of 15 (2,048 x 384, R 64:
+// 11.7 / 11.1; 64 of them, 2,048 x 256: 7.4 / 11.0).  From 512 tokens on the other kernel, with 16 tokens a CTA, takes 12
+// us itself at R 64 and more: plain products gain with any number of CTAs (256 x 512: 11.9 / 10.9), the others from 128 on.
 constexpr int LR_MIN_EXPANDED = 256;
 // grid (blocks of LR_COLS channels of both jobs, ceil(N / LR_TOKENS)).
 __global__ void __launch_bounds__(LR_THREADS, 4)
@@ -943,6 +951,14 @@ __global__ void silu_columns_kernel(T* __restrict__ x, int64_t ldx, int C, int64
     }
 }
 
+static int sm_count() {
+    int dev = 0, n_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    return n_sm;
+}
+
 }  // namespace sllm
 
 using namespace sllm;
@@ -1088,7 +1104,9 @@ SLLM_EXPORT int sllm_lowrank_decay(const float* pre, int64_t ldp, const float* w
     if (n_tokens >= LR_MIN_TOKENS && C % 4 == 0 &&
         !(((uintptr_t)w2t | (uintptr_t)w0 | (uintptr_t)a_bias | (uintptr_t)out) & 15)) {
         const dim3 tiles((C + LR_COLS - 1) / LR_COLS, (n_tokens + LR_TOKENS - 1) / LR_TOKENS);
-        if (tiles.y <= 65535)
+        const int n_sm = sm_count();
+        if (n_sm <= 0) return (int)cudaErrorInvalidDevice;
+        if (tiles.y <= 65535 && 4 * (int64_t)tiles.x * tiles.y >= (R < 64 ? 8 : R < 128 ? 6 : 5) * n_sm)
             return (int)sllm_launch_pdl(lowrank_decay_tile_kernel, tiles, dim3(LR_THREADS), 0, stream, pre, ldp,
                                         w2t, w0, a_bias, decay_scale, out, n_tokens, C, R,
                                         ldp % 4 == 0 && !((uintptr_t)pre & 15));
@@ -1127,16 +1145,23 @@ SLLM_EXPORT int sllm_lowrank_expand(const float* pre, int64_t ldp, int n_jobs, c
         max_r = R[i] > max_r ? R[i] : max_r;
         max_c = C[i] > max_c ? C[i] : max_c;
     }
-    bool tiled = n_tokens >= LR_MIN_EXPANDED;
-    for (int i = 0; i < n_jobs; ++i)
+    bool tiled = n_tokens >= LR_MIN_EXPANDED, plain = true;
+    for (int i = 0; i < n_jobs; ++i) {
         tiled = tiled && C[i] % 4 == 0 && !(((uintptr_t)w2t[i] | (uintptr_t)out[i]) & 15);
-    if (tiled && (n_tokens + LR_TOKENS - 1) / LR_TOKENS <= 65535) {
+        plain = plain && mode[i] == 0;
+    }
+    const int token_blocks = (n_tokens + LR_TOKENS - 1) / LR_TOKENS;
+    if (tiled && token_blocks <= 65535) {
         const int blocks0 = (j[0].C + LR_COLS - 1) / LR_COLS;
         const int blocks1 = n_jobs > 1 ? (j[1].C + LR_COLS - 1) / LR_COLS : 0;
-        return (int)sllm_launch_pdl(lowrank_expand_tile_kernel,
-                                    dim3(blocks0 + blocks1, (n_tokens + LR_TOKENS - 1) / LR_TOKENS), dim3(LR_THREADS),
-                                    0, stream, pre, ldp, j[0], j[1], blocks0, n_tokens,
-                                    ldp % 4 == 0 && !((uintptr_t)pre & 15));
+        const int n_sm = sm_count();
+        if (n_sm <= 0) return (int)cudaErrorInvalidDevice;
+        const bool slow = n_tokens >= 512 && max_r >= 64;      // (the other kernel is, see above)
+        if ((int64_t)(blocks0 + blocks1) * token_blocks >=
+                (plain || max_r >= 128 ? n_sm / 2 : slow ? n_sm * 3 / 4 : n_sm) || (plain && slow))
+            return (int)sllm_launch_pdl(lowrank_expand_tile_kernel, dim3(blocks0 + blocks1, token_blocks),
+                                        dim3(LR_THREADS), 0, stream, pre, ldp, j[0], j[1], blocks0, n_tokens,
+                                        ldp % 4 == 0 && !((uintptr_t)pre & 15));
     }
     // steps of few tokens: narrow CTAs, so that the channels spread over more SMs; long steps of other sizes: more
     // tokens a CTA and two channels a thread, so that the weights are read less often

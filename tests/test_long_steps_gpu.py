@@ -70,10 +70,12 @@ def test_32bit_product_widths_of_tiles(m, n, k):
 
 
 @pytest.mark.parametrize("n,c,r,ld", [(512, 128, 64, 0), (577, 132, 5, 0), (575, 4, 130, 0), (530, 260, 64, 1),
-                                       (257, 256, 33, 0)])
+                                       (257, 256, 33, 0), (2113, 900, 64, 1), (2401, 1000, 5, 0), (1900, 1028, 130, 0),
+                                       (545, 3076, 64, 0), (300, 4100, 33, 0)])
 def test_second_products_of_low_rank_pairs(n, c, r, ld):
     """One chain of multiply-adds over the rank per output: a token's bits are those of a step of few tokens.
-    ``ld``: hidden values that allow no reads of 16 bytes."""
+    ``ld``: hidden values that allow no reads of 16 bytes.  (Launches of few CTAs keep the kernels of short steps: of the
+    sizes up to 577 tokens and 260 channels all but the plain products, at ranks from 64 on; the others take the tiles.)"""
     from scratch_llm_b200.kernels import ops
     g = torch.Generator().manual_seed(n + c + r)
     pre = torch.randn(n, c + r + ld, generator=g).to(DEV)[:, :c + r]
