@@ -7,17 +7,17 @@
 // and N are, so a token's result does not depend on what else is in the batch.
 //
 // Three kernels.  32-bit operands whose rows allow 16-byte requests, by size:
-//   gemm_f32_wide_kernel   tiles of 64 x 64, 64 x 48 or 64 x 32, where those give every SM two
+//   gemm_f32_wide_kernel   tiles of 64 x 64, 64 x 48 or 64 x 32, where `wide_columns` finds them faster
 //   gemm_f32_kernel        smaller tiles behind a ring of cp.async stages: few tokens are bound by the chain
 //                          of steps over k, whose loads the ring keeps ahead of.  Tiles of 32 x 32, and of
 //                          16 x 16 up to 16 tokens.
 // gemm_simt_kernel: every other type and layout (one step of loads, then its arithmetic).
-// us (all on gemm_simt_kernel / with the wide kernel's rows a lane / now), K = 2,048:
-//   1 token    N 3,072: 116 / 25 / 25         16,384: 213 / 70 / 70          128,256: 1,161 / 419 / 419
-//   64         134 / 62 / 62                  236 / 184 / 184                1,369 / 1,235 / 1,235
-//   256        214 / 137 / 124                701 / 560 / -                  5,258 / 4,300 / -
-//   777        497 / 365 / 257                2,194 / 1,598 / -
-//   2,048      1,067 / 820 / -                5,337 / 3,788 / 3,050 (45 TF/s)
+// us (all on gemm_simt_kernel / with a row a lane in the wide kernel / now), K = 2,048:
+//   1 token    N 3,072: 116 / 25 / 25         16,384: 213 / 70 / 71          128,256: 1,161 / 419 / 419
+//   64         134 / 62 / 62                  236 / 184 / 173                1,369 / 973 / 827
+//   256        214 / 137 / 124                701 / 560 / 469                5,258 / 3,751 / 2,996
+//   777        497 / 366 / 258                2,194 / 1,594 / 1,258          - / 11,730 / 9,383
+//   2,048      1,067 / 811 / 600              5,337 / 3,767 / 3,020          - / 28,897 / 22,874 (47 TF/s)
 // What bounds the wide kernel now is shared memory: a read of 16 bytes a lane takes four cycles of it
 // whether or not lanes ask for the same, 16 per 64 multiply-adds a lane, as many as the four schedulers have.
 #include "common.cuh"
@@ -276,9 +276,36 @@ static int launch_f32(const float* X, const float* W, float* Y, int M, int N, in
     return 0;
 }
 
+// Columns of the wide kernel's tiles for M > 16 rows of X by N of W, or 0 where the ring's tiles of 32 x 32 take less, by
+// what the SM with the most tiles takes (in units of 0.138 us at K = 2,048).  The ring: rounds of two tiles an SM (65
+// tokens by 6,144, 576 tiles: 95 us, 122 in wide tiles 48 columns across; by 8,192, 768: 135 and, 32 across, 151; 256 by
+// 3,072, 768: 136 and, 48 across, 123).  Wide tiles: rounds of six (twelve warps, three a scheduler); one or two
+// tiles take half a full round, three or four 0.73 of it, latencies being hidden less.  A narrow tile reads more of shared
+// memory per multiply-add (777 tokens by 3,072: 320 us 64 across, 257 so).  Where no other row of tiles reads the
+// weights again, weights beyond what the L2 is sure to hold come late, which the ring's loads stay further ahead of (33
+// tokens by 12,288: 135 us, 158 in wide tiles; K = 256: 20.4 and 18.2).  Measured over 17 to 2,048 tokens by 512 to 65,536.
+static int wide_columns(int M, int N, int K, int n_sm) {
+    static const int tail[6] = {0, 15, 15, 22, 22, 30};
+    const auto per_sm = [&](int rows, int cols) {
+        return ((int64_t)((M + rows - 1) / rows) * ((N + cols - 1) / cols) + n_sm - 1) / n_sm;
+    };
+    int best = 0;
+    int64_t least = (per_sm(32, 32) + 1) / 2 * (K < 512 ? 345 : 327);      // (its ring fills and empties)
+    for (int tn = 8; tn >= 4; tn -= 2) {
+        const int64_t tiles = per_sm(WIDE, 8 * tn);
+        int64_t cost = (tiles / 6 * 30 + tail[tiles % 6]) * (tn == 8 ? 80 : tn == 6 ? 62 : 48);
+        if (M <= WIDE && (int64_t)N * K >= 1 << 24) cost += cost / 5;
+        if (cost < least) { best = 8 * tn; least = cost; }
+    }
+    return best;
+}
+
 }  // namespace sllm
 
 using namespace sllm;
+
+// The columns of the wide kernel's tiles, 0: another kernel.
+SLLM_EXPORT int sllm_gemm_simt_columns(int M, int N, int K, int n_sm) { return M > 16 ? wide_columns(M, N, K, n_sm) : 0; }
 
 // in_dtype / out_dtype: 0 = float32, 1 = bfloat16.  Supported: (0,0), (1,1), (1,0).
 SLLM_EXPORT int sllm_gemm_simt(const void* X, const void* W, void* Y, int M, int N, int K,
@@ -295,29 +322,12 @@ SLLM_EXPORT int sllm_gemm_simt(const void* X, const void* W, void* Y, int M, int
         if (cudaGetDevice(&dev) != cudaSuccess ||
             cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             return (int)cudaErrorInvalidDevice;
-        // Few tiles even of the narrowest width (of the widest, where half of a tile's rows stay empty): the
-        // ring's small tiles (128 tokens by 3,072: 93 us, 103 with tiles 32 wide; 256 tokens: 137 and, 48
-        // wide, 124).
-        const int narrow = M <= 32 ? 64 : 32;
-        if ((int64_t)((M + 63) / 64) * ((N + narrow - 1) / narrow) < 2 * n_sm)
-            return launch_f32<32, 32, 4, 4, 32, 4>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
-        // The tiles' width by what the SM with the most tiles takes: rounds of six tiles (twelve warps, three a
-        // scheduler); one or two tiles take half a full round, three or four 0.73 of it, latencies being
-        // hidden less.  A narrow tile reads more of shared memory per multiply-add.  Measured over sizes of 33
-        // to 2,048 tokens by 2,048 to 128,256, this is within 3 % of the best width (the widest always: 777
-        // tokens by 3,072 320 us, 257 so).
-        static const int tail[6] = {0, 15, 15, 22, 22, 30};
-        int best = 0;
-        int64_t cost = 0;
-        for (int tn = 8; tn >= 4; tn -= 2) {
-            const int64_t tiles = (int64_t)((M + 63) / 64) * ((N + 8 * tn - 1) / (8 * tn));
-            const int64_t per_sm = (tiles + n_sm - 1) / n_sm;
-            const int64_t now = (per_sm / 6 * 30 + tail[per_sm % 6]) * (tn == 8 ? 80 : tn == 6 ? 62 : 48);
-            if (!best || now < cost) { best = tn; cost = now; }
+        switch (wide_columns(M, N, K, n_sm)) {
+        case 64: return launch_wide<8>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
+        case 48: return launch_wide<6>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
+        case 32: return launch_wide<4>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
         }
-        if (best == 8) return launch_wide<8>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
-        if (best == 6) return launch_wide<6>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
-        return launch_wide<4>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
+        return launch_f32<32, 32, 4, 4, 32, 4>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
     }
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return (int)cudaErrorInvalidValue;

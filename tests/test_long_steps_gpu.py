@@ -69,6 +69,22 @@ def test_32bit_product_widths_of_tiles(m, n, k):
     assert torch.equal(got, ops.gemm_simt(odd, w, torch.empty(m, n, device=DEV)))
 
 
+@pytest.mark.parametrize("columns,m,n,k", [(64, 513, 6144, 52), (64, 777, 16390, 36), (64, 2050, 5120, 20),
+                                            (48, 777, 3070, 52), (48, 129, 4100, 36), (48, 50, 12290, 20),
+                                            (32, 129, 6144, 52), (32, 1030, 1020, 36), (32, 33, 16390, 20),
+                                            (0, 65, 6144, 52), (0, 33, 3072, 36), (0, 257, 2046, 20)])
+def test_32bit_product_over_several_steps(columns, m, n, k):
+    """Each width of the wide tiles, and the ring, over more than one step of 16 and a remainder, with rows and columns
+    that end inside a tile: the bits of the plainest kernel.  (The rule depends on the SMs: sizes for 148 of them.)"""
+    from scratch_llm_b200.kernels import ops
+    assert columns == ops._core("sllm_gemm_simt").sllm_gemm_simt_columns(m, n, k, 148)
+    g = torch.Generator().manual_seed(m + n)
+    x, w = torch.randn(m, k, generator=g).to(DEV), torch.randn(n, k, generator=g).to(DEV)
+    odd = torch.empty(m, k + 1, device=DEV)[:, :k].copy_(x)
+    got = ops.gemm_simt(x, w, torch.full((m, n), float("nan"), device=DEV))
+    assert torch.equal(got, ops.gemm_simt(odd, w, torch.empty(m, n, device=DEV)))
+
+
 @pytest.mark.parametrize("n,c,r,ld", [(512, 128, 64, 0), (577, 132, 5, 0), (575, 4, 130, 0), (530, 260, 64, 1),
                                        (257, 256, 33, 0), (2113, 900, 64, 1), (2401, 1000, 5, 0), (1900, 1028, 130, 0),
                                        (545, 3076, 64, 0), (300, 4100, 33, 0)])
