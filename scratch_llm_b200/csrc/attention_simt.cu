@@ -517,14 +517,16 @@ template <typename T, int MOST>
 __global__ void __launch_bounds__(THREADS, HD <= 64 ? 5 : HD <= 128 ? 4 : 1)
 attn_simt_kernel(const T* __restrict__ q, const T* __restrict__ pages, const int* __restrict__ block_table,
                  const int* __restrict__ row_start, const int* __restrict__ row_pos0, T* __restrict__ out,
-                 const float* __restrict__ slopes, const float* __restrict__ sinks, const Args args, int max_new) {
+                 const float* __restrict__ slopes, const float* __restrict__ sinks, const Args args, int max_new,
+                 int first_block) {
     extern __shared__ __align__(16) float smem[];
     __shared__ long long key_base[BKV];  // element offset of each key's K row, -1 if absent
     constexpr int BQ = WARPS * MOST;
-    const int r = blockIdx.y, h = blockIdx.x % args.H;
+    // (the head as it comes from the grid: as a remainder it took a register, and eight queries a warp spilled: 3-5 %)
+    const int r = blockIdx.z, h = blockIdx.x;
     const int t0 = row_start[r], n_new = row_start[r + 1] - t0;
     // the queries with the most keys first, of all heads
-    const int q0 = (gridDim.x - 1 - blockIdx.x) / args.H * BQ;
+    const int q0 = (first_block + gridDim.y - 1 - blockIdx.y) * BQ;
     if (q0 >= n_new || n_new > max_new) return;          // (longer rows: attn_simt_tile_kernel)
     const int nq = min(BQ, n_new - q0);
     const int* table = block_table + (int64_t)r * args.table_stride;
@@ -546,10 +548,14 @@ static int launch(const void* q, const void* pages, const int* block_table, cons
     const cudaError_t e = cudaFuncSetAttribute(attn_simt_kernel<T, MOST>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    constexpr int BQ = WARPS * MOST;
-    attn_simt_kernel<T, MOST><<<dim3(args.H * ((max_new + BQ - 1) / BQ), n_rows), THREADS, smem, stream>>>(
-        (const T*)q, (const T*)pages, block_table, row_start, row_pos0, (T*)out, slopes, sinks, args, max_new);
-    SLLM_LAUNCH_CHECK();
+    constexpr int BQ = WARPS * MOST, AT_ONCE = 65535;
+    for (int end = (max_new + BQ - 1) / BQ; end > 0; end -= AT_ONCE) {
+        const int blocks = end < AT_ONCE ? end : AT_ONCE;
+        attn_simt_kernel<T, MOST><<<dim3(args.H, blocks, n_rows), THREADS, smem, stream>>>(
+            (const T*)q, (const T*)pages, block_table, row_start, row_pos0, (T*)out, slopes, sinks, args, max_new,
+            end - blocks);
+        SLLM_LAUNCH_CHECK();
+    }
     return 0;
 }
 
@@ -571,7 +577,7 @@ SLLM_EXPORT int sllm_attn_simt_head_dim() { return HD; }
 // pages: [n_pages, planes, G, page_size, HD]; planes = 2: keys, then values; planes = 1: one
 // vector per token that is its key and, by its leading entries, its value.  block_table: [n_rows, table_stride], -1 = no page.
 // row_start: [n_rows + 1] token offsets; row_pos0: [n_rows] position of each row's first token.
-// max_new: the largest number of new tokens of any row.  window: 0 = all keys.
+// n_tokens: of all rows; max_new: the largest number of new tokens of any row.  window: 0 = all keys.
 // slopes (may be null): float [H]; slopes[h] * (query position - key position) is taken off the
 // scaled score of head h.  sinks (may be null): float [H]; exp(sinks[h]) is added to the softmax's
 // denominator of head h, once, with no value behind it.  softcap > 0: the scaled score s becomes
@@ -580,7 +586,7 @@ SLLM_EXPORT int sllm_attn_simt_head_dim() { return HD; }
 SLLM_EXPORT int sllm_attn_simt(const void* q, int64_t q_stride, const void* pages,
                                const int* block_table, int table_stride, int page_size,
                                const int* row_start, const int* row_pos0, void* out,
-                               int64_t out_stride, int n_rows, int max_new, int H, int G,
+                               int64_t out_stride, int n_rows, int n_tokens, int max_new, int H, int G,
                                float scale, int window, const float* slopes, const float* sinks,
                                int planes, float softcap, int chunk, int dtype,
                                cudaStream_t stream) {
@@ -591,11 +597,18 @@ SLLM_EXPORT int sllm_attn_simt(const void* q, int64_t q_stride, const void* page
     const Args args = {q_stride, out_stride, table_stride, page_size, H, G, scale, softcap, window, chunk, planes,
                        ((uintptr_t)pages & 15) == 0};
 #ifdef SLLM_TILED
-    // 32-bit rows whose pages and heads are whole 16-byte words.  Several rows take two launches (the rows of
-    // up to 16 tokens are the other kernel's), which short ones do not earn.
-    if (dtype == 0 && args.vec && (n_rows == 1 ? max_new > 8 * WARPS : max_new >= 512)) {
-        const int gs = H / G, heads = gs % 4 == 0 ? 4 : gs % 2 == 0 ? 2 : 1;
-        const bool alone = n_rows == 1;
+    // 32-bit rows whose pages and heads are whole 16-byte words.  us with attn_simt_kernel and so: a row of 48 tokens
+    // without keys before them, 32 heads of 64 on 8 kv heads 11.8 / 14.7, of 112 13.8 / 19.9; of 64 16.3 / 15.1 and 19.8 / 20.4; of
+    // 48 after 200 44 / 39 and 61 / 56; of 33, 2 heads of 80 on a kv head 13.7 / 11.3.  Several rows take two launches (rows
+    // of up to 16 tokens are the other kernel's), which short ones do not earn; nor do rows of just more than 16 where
+    // every head has a kv head of its own and a block thus 64 tokens (one of 512 and 63 of 17, 8 heads of 64: 185 / 214;
+    // 20 of 30: 289 / 219; 64 of one: 113 / 103).
+    const int gs = H / G, heads = gs % 4 == 0 ? 4 : gs % 2 == 0 ? 2 : 1;
+    const bool alone = n_rows == 1, far = (int64_t)table_stride * page_size >= 256;
+    const int least = far || HD <= 32 || (HD % 64 && HD < 96 && heads < 4) ? 8 * WARPS : HD < 96 ? 12 * WARPS : 16 * WARPS;
+    const bool short_rows = n_tokens > 16 * (int64_t)n_rows && n_tokens < 40 * (int64_t)n_rows;    // on average
+    const bool tiles = alone ? max_new > least : max_new >= 512 && !(heads == 1 && short_rows);
+    if (dtype == 0 && args.vec && tiles) {
         if (!alone) {
             const int e = launch<float, 4>(q, pages, block_table, row_start, row_pos0, out, slopes, sinks, args,
                                            n_rows, 4 * WARPS, stream);

@@ -642,8 +642,8 @@ def attention_simt(q: torch.Tensor, pages: torch.Tensor, block_table: torch.Tens
     _check(lib.sllm_attn_simt(
         _ptr(q), c_int64(q.stride(0)), _ptr(pages), _ptr(block_table),
         c_int(block_table.stride(0)), c_int(page_size), _ptr(row_start), _ptr(row_pos0),
-        _ptr(out), c_int64(out.stride(0)), c_int(n_rows), c_int(max_new), c_int(n_heads),
-        c_int(n_kv_heads), c_float(scale), c_int(window or 0), _ptr(slopes), _ptr(sinks),
+        _ptr(out), c_int64(out.stride(0)), c_int(n_rows), c_int(q.shape[0]), c_int(max_new),
+        c_int(n_heads), c_int(n_kv_heads), c_float(scale), c_int(window or 0), _ptr(slopes), _ptr(sinks),
         c_int(planes), c_float(softcap), c_int(chunk or 0), c_int(_code(q.dtype)), _stream()),
         "attention_simt")
     return out

@@ -289,3 +289,54 @@ def test_general_delta_in_large_launches(D, V, dtype):
     # decays of at least 0.55: a few tokens' roundings, each a few of 2^-24
     for got, ref in ((out, want.flatten(1)), (state, S_all)):
         assert ((got.double() - ref).norm() / ref.norm()).item() < 1e-6
+
+
+@pytest.mark.parametrize("hd", [64, 80, 112, 128])
+@pytest.mark.parametrize("n", [32, 33, 48, 49, 64, 65])
+def test_attention_simt_around_the_tiles_limits(hd, n):
+    """A row's portion with a block table of few keys and of many (which kernel takes it depends on that): the same
+    bits, those of single tokens."""
+    from scratch_llm_b200.kernels import ops
+    ops.prepare_jobs([ops.attention_library(hd)], verbose=False)
+    H, G, page, before = 6, 3, 16, 5
+    gen = torch.Generator().manual_seed(hd + n)
+    need = -(-(before + n) // page)
+    pages, q = torch.randn(need, 2, G, page, hd, generator=gen).to(DEV), torch.randn(n, H * hd, generator=gen).to(DEV)
+    wide = torch.full((1, 40), -1, dtype=torch.int32)
+    wide[0, :need] = torch.arange(need)
+
+    def attend(table, first, count):
+        out = torch.full((count, H * hd), float("nan"), device=DEV)
+        return ops.attention_simt(q[first:first + count], pages, table.to(DEV), page, _i32([0, count]),
+                                  _i32([before + first]), out, 1, count, H, G, hd, hd ** -0.5, None)
+
+    single = torch.cat([attend(wide, t, 1) for t in range(n)])
+    assert torch.equal(attend(wide, 0, n), single)
+    assert torch.equal(attend(wide[:, :need].contiguous(), 0, n), single)
+
+
+@pytest.mark.parametrize("short", [17, 90])
+def test_attention_simt_many_rows_of_own_heads(short):
+    """A long row beside many, each head with a kv head of its own: by the tokens a row on average one launch or two,
+    the same bits."""
+    from scratch_llm_b200.kernels import ops
+    ops.prepare_jobs([ops.attention_library(64)], verbose=False)
+    H, page, hd, rows = 2, 16, 64, [520] + [short] * 30 + [0, 1]
+    gen = torch.Generator().manual_seed(short)
+    need = [-(-n // page) for n in rows]
+    pages = torch.randn(sum(need), 2, H, page, hd, generator=gen).to(DEV)
+    first = [sum(rows[:r]) for r in range(len(rows) + 1)]
+    q = torch.randn(first[-1], H * hd, generator=gen).to(DEV)
+    table = torch.full((len(rows), max(need)), -1, dtype=torch.int32)
+    for r, k in enumerate(need):
+        table[r, :k] = torch.arange(sum(need[:r]), sum(need[:r]) + k)
+    table = table.to(DEV)
+    out = torch.full_like(q, float("nan"))
+    ops.attention_simt(q, pages, table, page, _i32(first), _i32([0] * len(rows)), out, len(rows), 520, H, H, hd, 0.125, None)
+    for r, n in enumerate(rows):
+        if n:
+            at = slice(first[r], first[r + 1])
+            alone = torch.empty(n, H * hd, device=DEV)
+            ops.attention_simt(q[at], pages, table[r:r + 1], page, _i32([0, n]), _i32([0]), alone, 1, n, H, H, hd, 0.125,
+                               None)
+            assert torch.equal(alone, out[at])
