@@ -386,7 +386,8 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t ld, int V, int s
         __syncthreads();
         float thresh = 0.f;  // keep p >= thresh
         if (NUCLEUS && tp < 1.0f) {
-            // f(t) = sum of p_i > t.  lo: f(lo) > tp.  hi: f(hi) <= tp.  p_max = 1 / Z.
+            // f(t) = sum of p_i > t.  lo: f(lo) > tp.  hi: f(hi) <= tp, or the search ends there: the largest
+            // probability is 1 / Z but for the rounding of its logit times inv_t, and may lie above.
             unsigned lo = 0u, hi = __float_as_uint(inv_z);
             if (bounds) {   // the row's histogram: each CTA adds up its share of the buckets and tells all
                 constexpr int SHARE = SC_BUCKETS / SC_RANKS;
@@ -413,7 +414,9 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t ld, int V, int s
                 const int surely = __syncthreads_count((float)above <= (tp - margin) * SC_UNIT);
                 const int maybe = __syncthreads_count((float)above <= (tp + margin) * SC_UNIT);
                 if (surely > 0 && surely < SC_BUCKETS) hi = min(hi, sc_edge(surely - 1));
-                if (maybe < SC_BUCKETS - 1) lo = sc_edge(maybe) - 1u;
+                // (a row that its largest probability fills may have its bucket's edge above 1 / Z: f is above top_p
+                // all the way to hi then, which is where the search from 0 ends too)
+                if (maybe < SC_BUCKETS - 1) lo = min(sc_edge(maybe), hi) - 1u;
             }
             while (hi - lo > 1u) {
                 // two steps of the bisection in one round: the middle, and the middles of the

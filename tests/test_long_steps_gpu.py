@@ -147,6 +147,30 @@ def test_nucleus_of_flat_and_steep_rows(V):
         assert above <= float(tops[r]) + slack and upto >= float(tops[r]) - slack
 
 
+@pytest.mark.parametrize("V", [8192, 50001])
+@pytest.mark.parametrize("more", [0, 1])
+def test_nucleus_of_rows_that_one_value_fills(V, more):
+    """The largest probability's exponential is not exactly 1 at a temperature (the rounding of its logit over it), so
+    it may lie on either side of 1 / Z, and so on either side of an edge of the histogram's buckets.  ``more``: as many
+    equal values again, all kept or none but the first."""
+    from scratch_llm_b200.kernels import ops
+    tops = torch.linspace(8.0, 40.0, 96)
+    temps, rows, top_p = (torch.linspace(0.3, 0.8, 96), torch.full((96, V), -200.0),
+                          torch.tensor([1e-6, 0.3, 0.9]).repeat(32))
+    at = torch.arange(96) * 83 % V
+    rows[torch.arange(96), at] = tops
+    if more:
+        rows[torch.arange(96), (at + V // 2) % V] = tops
+    probs, out = torch.empty(96, V, device=DEV), torch.empty(96, dtype=torch.int32, device=DEV)
+    seed = torch.arange(96, device=DEV)
+    ops.sample(rows.to(DEV), out, temps.to(DEV), top_p.to(DEV), seed, seed, probs_out=probs)
+    # (equal values are kept together)
+    want = torch.zeros(96, V)
+    want[rows == tops[:, None]] = 1.0 / (1 + more)
+    assert torch.equal(probs.cpu(), want)
+    assert (rows[torch.arange(96), out.cpu().long()] == tops).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("C,taps", [(1032, 4), (7, 4), (24, 2), (16, 1), (128, 6)])
 def test_convolution_and_carried_inputs_in_one_pass(dtype, C, taps):
