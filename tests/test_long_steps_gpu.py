@@ -193,6 +193,21 @@ def test_convolution_and_carried_inputs_in_one_pass(dtype, C, taps):
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
 
 
+@pytest.mark.parametrize("taps", [1, 4])
+def test_convolution_step_of_very_many_tokens(taps):
+    """More single tokens than a grid's second dimension holds, which the convolution alone has always taken."""
+    from scratch_llm_b200.kernels import ops
+    n, C, g = 70_000, 8, torch.Generator().manual_seed(taps)
+    x, w = torch.randn(n, C, generator=g).to(DEV), torch.randn(C, taps, generator=g).to(DEV)
+    state = torch.randn(n, max(taps - 1, 1), C, generator=g).to(DEV)
+    rows, starts = torch.arange(n, dtype=torch.int32, device=DEV), torch.arange(n + 1, dtype=torch.int32, device=DEV)
+    carried = state if taps > 1 else None
+    want = ops.conv_silu(x, w, carried, rows, starts, rows, torch.empty_like(x))
+    after = torch.cat([state[:, 1:], x[:, None]], 1)
+    assert torch.equal(ops.conv_silu(x, w, carried, rows, starts, rows, torch.empty_like(x), update=True), want)
+    assert taps == 1 or torch.equal(state, after)
+
+
 @pytest.mark.parametrize("hd", [64, 16, 80, 112])
 @pytest.mark.parametrize("H,G", [(4, 1), (6, 3), (3, 3)])
 @pytest.mark.parametrize("more", [{}, dict(window=37), dict(chunk=48), dict(softcap=5.0), dict(slopes=1, sinks=1)])
