@@ -9,10 +9,11 @@
 //
 // Layout: a column is spread over LANES neighbouring lanes of a warp, each with EPL = 4 of its
 // elements in registers as pairs (the key size D is padded to DP = 16 * 2^i; the padding stays
-// zero), and a thread holds such slices of CPT = 4 neighbouring columns, which the vectors that it
-// reads from shared memory per token serve together.  A CTA has four COMPUTE warps, one per
-// scheduler, which own 128 / LANES * CPT columns of one (row, head), and four LOADER warps; a
-// head's columns are spread over several CTAs.  The row's tokens come in chunks through two
+// zero; keys of more than 128 elements have more of them a lane), and a thread holds such slices of CPT
+// neighbouring columns, four, or two in small launches, which the vectors that it reads from shared memory
+// per token serve together.  A CTA has four COMPUTE warps, one per scheduler, which own
+// 128 / LANES * CPT columns of one (row, head), and four LOADER warps (fewer of both where many heads of few
+// columns share an SM: `launch`); a head's columns are spread over several CTAs.  The row's tokens come in chunks through two
 // buffers: while the compute warps run chunk c, the loader warps, which have requested chunk
 // c + 1 (r, k, w, a of the head, v of the CTA's columns) a chunk earlier, form -a * k, 1 / (|k|^2 +
 // eps) and the products of neighbouring tokens; all warps meet once per chunk.
@@ -27,12 +28,16 @@
 // run: the second half of one sum beside the first half of the next (`Pipe`).
 // Multiply-adds come in pairs (fma.rn.f32x2: the same rate, half the instructions).
 //
-// us before (a column a thread, sixteen elements a lane, five vectors) and now, bfloat16, 64 x 64:
-//   32 heads, a row of 2,048 tokens   592 / 300       64 heads, a row of 2,400       908 / 354
-//   32 heads, four rows of 1,024      485 / 246       64 heads, eight rows of 300    550 / 253
-//   32 heads, 64 single tokens         40 / 29        128 x 128, 16 heads, 2,048     734 / 367
-// It issues 138 instructions per token and scheduler in 300 cycles: latencies.  With two columns a thread
-// (twice the CTAs) the first takes 239, four rows of 1,024 348 and 64 single tokens 48.
+// A token's dot product is thus formed in another order when it is the first of a step: the same bits whatever else
+// is in the step, not however a row is cut into steps.
+//
+// us before (a column a thread, sixteen elements a lane, five vectors) and now (columns a thread), bfloat16, 64 x 64:
+//   32 heads, a row of 2,048 tokens   590 / 233 (2)   64 heads, a row of 2,400       908 / 340 (4)
+//   32 heads, a row of 100             34 / 15 (2)    64 heads, eight rows of 300    547 / 238 (4)
+//   32 heads, four rows of 1,024      481 / 232 (4)   128 x 128, 16 heads, 2,048     758 / 328 (4)
+//   32 heads, 64 single tokens         41 / 29 (4)
+// Latencies: 138 instructions per token and scheduler in 300 cycles with four columns a thread, 92 in 250 with two
+// (twice the CTAs).  With the other number the first takes 300, four rows of 1,024 348 and 64 single tokens 48.
 //
 // state: float32 [slots, H, V, DP] with DP = the padded key size; a fresh slot holds zeros.
 // Compiled once per key size (-DSLLM_HEAD_DIM=D).
@@ -109,7 +114,9 @@ __device__ __forceinline__ float4 numbers(const uint2& r) {
 template <int CPT, int WARPS> struct Rule {
 static constexpr int COMPUTE = 32 * WARPS;
 static constexpr int QUADS = CHUNK * DP / 4;         // units of 4 elements in a chunk
-static constexpr int LOADERS = WARPS > 1 ? 128 : QUADS / 4 < 32 ? 32 : QUADS / 4;
+// (64 loaders for rows that are fetched element by element: 48 single tokens and one row of 64, 32 heads of 9 x 9, 24.6 us,
+// with 32 of them 34.0)
+static constexpr int LOADERS = WARPS > 1 ? 128 : D % 4 || QUADS / 4 > 32 ? 64 : 32;
 static constexpr int THREADS = COMPUTE + LOADERS;
 static constexpr int COLS = COMPUTE / LANES * CPT;   // columns of S per CTA
 static __device__ __forceinline__ void loaders_sync() {
@@ -592,8 +599,10 @@ static int launch_rule(int n_rows, int H, int V, bool beside, cudaStream_t strea
 // row of 2,400: 353 and 404).
 // One compute warp and few loaders (64 threads at key size 16) where an SM gets more than the two CTAs of 256
 // threads that it holds, and the head's columns leave most of such a CTA idle.  us with 256 threads and so: 256 single
-// tokens, 32 heads of 16 x 16 67.6 / 21.2, of 9 x 9 69.7 / 21.0, 16 of 32 x 32 27.8 / 18.9, 16 of 64 x 5 28.6 / 14.1; 48 rows
-// of 8 tokens, 32 heads of 16 x 16 21.8 / 10.2.  (8 heads of 16 x 100, which take four such CTAs: 19.2 / 21.2.)
+// tokens, 32 heads of 16 x 16 67.6 / 21.2, of 9 x 9 69.7 / 22.8, 16 of 32 x 32 27.8 / 18.9, 16 of 64 x 5 28.6 / 14.1; 48 rows
+// of 8 tokens, 32 heads of 16 x 16 21.8 / 10.2.  (8 heads of 16 x 100, which take four such CTAs: 19.2 / 21.2.)  With 16
+// elements a key from more CTAs than SMs on (8 single tokens, 32 heads of 16 x 16 3.9 / 3.7, 8 rows of 64 18.9 / 13.5; of
+// 24 x 24 3.3 / 3.8 and 17.6 / 17.7, of 9 x 9 8 rows of 300 77 / 83).
 // `beside`: begun beside the kernel before it, a launch's CTAs take the places that come free first, two on some SMs,
 // and long rows of a launch that does not fill the SMs go by the slowest.  us of decays, rule and read-out in
 // turn, ordinary / beside: 32 heads of 64 x 64, 2,048 tokens 299 / 391, 300 52 / 67, 64 20.9 / 23.6, 8 13.0 / 12.7, 2
@@ -612,7 +621,8 @@ static int launch(const T* rkv, int64_t ld, int r0, int k0, int v0, const float*
                                            row_start, row_slot, out, H, V, unit_eps)
     if (FEW != MOST && ctas(Rule<FEW, 4>::COLS) <= n_sm) SLLM_GD_RULE(FEW, 4);
     if constexpr (DP <= 64) {
-        if (many && V <= 2 * Rule<MOST, 1>::COLS) SLLM_GD_RULE(MOST, 1);
+        const bool crowded = DP == 16 && D % 4 == 0 ? ctas(Rule<MOST, 4>::COLS) > n_sm : many;
+        if (crowded && V <= 2 * Rule<MOST, 1>::COLS) SLLM_GD_RULE(MOST, 1);
     }
     SLLM_GD_RULE(MOST, 4);
 #undef SLLM_GD_RULE
