@@ -1264,7 +1264,7 @@ def lowrank_decay(pre: torch.Tensor, w2t: torch.Tensor, w0: torch.Tensor, a_bias
 
 
 def general_delta_padded_dim(key_dim: int) -> int:
-    """The key size as the generalized delta rule's state stores it (padded to whole lanes)."""
+    """The key size as the generalized delta rule's state stores it (padded to 16 * 2^i)."""
     return int(_load(*general_delta_library(key_dim)).sllm_general_delta_padded_dim())
 
 

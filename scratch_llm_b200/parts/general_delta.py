@@ -55,12 +55,12 @@ class GeneralDelta(Mixer):
         self.w2t = self.w0 = self.a_bias = self.gain = None
 
     def state_spec(self) -> StateSpec:
-        # the key size as the kernel stores it: whole lanes of 16 elements (no device is needed
-        # to know it, so that a cache can be planned on the host)
-        lanes = 1
-        while lanes * 16 < self.key_dim:
-            lanes *= 2
-        return StateSpec((self.n_heads, self.value_dim, lanes * 16), torch.float32)
+        # the key size as the kernel stores it: padded to 16 * 2^i (no device is needed to know it, so
+        # that a cache can be planned on the host)
+        padded = 16
+        while padded < self.key_dim:
+            padded *= 2
+        return StateSpec((self.n_heads, self.value_dim, padded), torch.float32)
 
     def kernel_jobs(self, dtype: torch.dtype):
         return [ops.core_job("sllm_recurrent_ops"), ops.general_delta_library(self.key_dim)]
